@@ -122,7 +122,6 @@ static bool is_sky_kernel(const void *k) {
 template <typename T, int L, int SIGN, int NA, class Pro, class Epi>
 static int launch_col_L(dim3 grid, const Pro &pro, const Epi &epi_in, const cx<T> *tw, cudaStream_t st) {
      size_t smem = pass_smem_bytes<T, L, NA>();
-     if constexpr (is_staged<Pro>::value) smem = pro.smem;
      Epi epi = epi_in;
      if constexpr (has_tables<Epi>::value) {
           // the epilogue's tables go after everything else
@@ -215,7 +214,8 @@ struct DevBuf {
 template <typename T>
 struct FFTTables {
      int N = 0, N1 = 0, N2 = 0;
-     DevBuf line1, line2, hi, lo, base, step;
+     DevBuf line1, line2, hi, lo;
+     DevBuf base, step, ltw1, ltw2;   // split-form passes (build_split)
      int build(int n) {
           N = n;
           int l = ilog2i(n);
@@ -235,18 +235,32 @@ struct FFTTables {
           CUCHK(cudaMemcpy(lo.p, o.data(), 1024 * sizeof(cx<T>), cudaMemcpyHostToDevice));
           return TDF_OK;
      }
-     // per-thread base twiddles of the column-pass epilogue (StoreFourstepG):
-     // base[t*N2 + n2] = W^(n2*t), t < N1/8, and step[n2] = W^(n2*N1/8)
-     int build_base() {
+     // tables of the split-form passes (tdf_split.cuh): the columns' base
+     // twiddles base[n2*N1/8 + t] = W^(n2*t), t < N1/8, and step[n2] =
+     // W^(n2*N1/8); the pass twiddles of the two line lengths
+     int build_split() {
           const int R = N1 / 8;
           std::vector<cx<T>> b((size_t)R * N2), st(N2);
-          for (int t = 0; t < R; t++)
-               for (int n2 = 0; n2 < N2; n2++) b[(size_t)t * N2 + n2] = tw((long)n2 * t, N);
+          for (int n2 = 0; n2 < N2; n2++)
+               for (int t = 0; t < R; t++) b[(size_t)n2 * R + t] = tw((long)n2 * t, N);
           for (int n2 = 0; n2 < N2; n2++) st[n2] = tw((long)n2 * R, N);
-          TRY(base.alloc(b.size() * sizeof(cx<T>)));
-          TRY(step.alloc(st.size() * sizeof(cx<T>)));
-          CUCHK(cudaMemcpy(base.p, b.data(), b.size() * sizeof(cx<T>), cudaMemcpyHostToDevice));
-          CUCHK(cudaMemcpy(step.p, st.data(), st.size() * sizeof(cx<T>), cudaMemcpyHostToDevice));
+          TRY(put(base, b));
+          TRY(put(step, st));
+          TRY(put(ltw1, pass_twiddles(N1)));
+          return put(ltw2, pass_twiddles(N2));
+     }
+     static std::vector<cx<T>> pass_twiddles(int L) {
+          std::vector<cx<T>> v;
+          for (int NS = 8; NS < L; NS *= 8) {
+               const int R = pass_radix(L, NS);
+               for (int k = 0; k < pass_powers(R); k++)
+                    for (int j = 0; j < NS; j++) v.push_back(tw((long)j << k, (long)NS * R));
+          }
+          return v;
+     }
+     static int put(DevBuf &b, const std::vector<cx<T>> &v) {
+          TRY(b.alloc(v.size() * sizeof(cx<T>)));
+          CUCHK(cudaMemcpy(b.p, v.data(), v.size() * sizeof(cx<T>), cudaMemcpyHostToDevice));
           return TDF_OK;
      }
      static cx<T> tw(long m, long n) {
@@ -264,7 +278,9 @@ struct FFTTables {
           CUCHK(cudaMemcpy(b.p, v.data(), L * sizeof(cx<T>), cudaMemcpyHostToDevice));
           return TDF_OK;
      }
-     void release() { line1.release(); line2.release(); hi.release(); lo.release(); base.release(); step.release(); }
+     void release() {
+          for (DevBuf *b : {&line1, &line2, &hi, &lo, &base, &step, &ltw1, &ltw2}) b->release();
+     }
      const cx<T> *l1() const { return line1.as<cx<T>>(); }
      const cx<T> *l2() const { return line2.as<cx<T>>(); }
      const cx<T> *h() const { return hi.as<cx<T>>(); }
@@ -302,6 +318,7 @@ struct SegData {
 
 struct tdf_engine {
      int dev = 0, form = TDF_FORM_SPLIT;
+     int sms = 148;     // SMs of the device
      cudaStream_t own = nullptr, stream = nullptr;
      // The sky stage of the next batch runs on sky_stream, created at the
      // lowest stream priority while the engine's own stream and the lanes
@@ -325,9 +342,10 @@ struct tdf_engine {
      std::vector<double> lines;
      int N = 0, nfft = 0, nfftf = 0, Ninterp = 0, nifo = 0, Nal = 0, n2N = 0;
      int nF = 0, nblk_mu = 0;
+     int CL = 0;        // split form: entries of an operand column (ceil(N/N2), up to a multiple of 32)
      int Bs = 8;        // sky points per batch
-     int Tc = 16;       // templates per chunk (intermediate spectra sized for L2)
-     int TcMax = 32;    // buffers are sized for chunks up to this size
+     int Tc = 96;       // templates per chunk
+     int TcMax = 96;    // buffers are sized for chunks up to this size
      int Gt = 64;       // templates per resolve group at most (whole chunks; TDF_GROUP_TEMPLATES)
      static constexpr int kGtMax = 128;   // buffers are sized for groups up to this size
      int64_t launches = 0;
@@ -336,14 +354,9 @@ struct tdf_engine {
      // inputs
      DevBuf pco, gco;
      // sky stage
-     DevBuf skyp[2], B0, B1, B2, shftf, partial, aabb[2];
+     DevBuf skyp[2], B0, B1, B2, shft, partial, aabb[2];
      // operands
      DevBuf xab[2], s2[2], xa64[2], xb64[2], t1[2];   // per batch slot
-     // TMA staging of the split-form operands in the column pass
-     bool staged = false;
-     CUtensorMap tm_x[2], tm_s[2];   // xab[k], s2[k]
-     int stg_groups = 0, stg_stages = 0;
-     unsigned stg_bar_off = 0, stg_smem = 0;
      // spindown stage: consecutive resolve groups alternate between lanes,
      // each with its own stream and buffers, so that one lane's kernel tails
      // and trigger resolution overlap the other lane's passes
@@ -419,7 +432,7 @@ struct tdf_engine {
      uint64_t graph_tick = 0;
      bool use_graphs = true;   // TDF_GRAPHS=0 launches every kernel from the host
      bool graph_prio = true;   // TDF_GRAPH_PRIORITY=0 leaves captured kernel nodes at their default priority
-     bool row_bulk = true;     // row passes fetch their rows by bulk copies (TDF_ROW_BULK=0: per thread)
+     bool row_bulk = true;     // FP64 form: row passes fetch their rows by bulk copies (TDF_ROW_BULK=0: per thread)
      // split form, N1 = N2: TDF_FUSED_PASSES=1 runs the column and row
      // passes of a chunk as one ordered launch of persistent CTAs
      // (k_spinpass), a template's rows fuse_lag templates behind its
@@ -541,91 +554,6 @@ static int upload_inputs(tdf_engine *e, const tdf_segment *s) {
      return TDF_OK;
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// against libcuda); null when the driver does not provide it
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-     static std::once_flag once;
-     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-     std::call_once(once, [] {
-          void *p = nullptr;
-          cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-          if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-              q == cudaDriverEntryPointSuccess)
-               fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-     });
-     return fn;
-}
-
-template <int L>
-static void col_geometry(size_t *smem, int *blocks) {
-     *smem = pass_smem_bytes<float, L, 2>();
-     *blocks = pass_min_blocks<float, L>();
-}
-
-// Sizes the TMA ring of the split-form column pass (DemodSplitStaged) and
-// encodes the operand tensor maps of both batch slots.  The ring takes as
-// many row groups as fit in the shared memory a CTA may use at the pass's
-// occupancy (228 KB per SM, 1 KB reserved per CTA).  Used with
-// TDF_STAGED_OPERANDS=1; by default the column pass loads its operands per
-// thread (DemodSplit), which measured as fast with the operands L2-resident.
-static int staged_setup(tdf_engine *e) {
-     e->staged = false;
-     if (e->form != TDF_FORM_SPLIT) return TDF_OK;
-     const char *env = getenv("TDF_STAGED_OPERANDS");
-     if (!env || env[0] != '1') return TDF_OK;
-     const int L = e->t_f32.N1, N2 = e->t_f32.N2, R = L / 8, nifo = e->nifo;
-     if (e->Nal % N2 != 0) return TDF_OK;
-     size_t pass_smem = 0;
-     int blocks = 1;
-     switch (L) {
-     case 64: col_geometry<64>(&pass_smem, &blocks); break;
-     case 128: col_geometry<128>(&pass_smem, &blocks); break;
-     case 256: col_geometry<256>(&pass_smem, &blocks); break;
-     case 512: col_geometry<512>(&pass_smem, &blocks); break;
-     case 1024: col_geometry<1024>(&pass_smem, &blocks); break;
-     default: return TDF_OK;
-     }
-     const size_t tw = (size_t)L * sizeof(float2);
-     const size_t lines = pass_smem - tw;
-     const size_t slot = (size_t)nifo * R * LINES * (sizeof(float4) + sizeof(float));
-     const size_t bars = 8 * sizeof(uint64_t);
-     const int rows = (e->N + N2 - 1) / N2;
-     const int groups = std::min(8, (rows + R - 1) / R);
-     // less the epilogue's twiddle tables (StoreFourstep), which follow the ring
-     const size_t tables = sizeof(float2) * ((size_t)L * N2 / 1024 + 1024) + 16;
-     const size_t budget = std::min<size_t>(227 * 1024, 233472 / blocks - 1024) - tables;
-     if (budget < tw + bars + slot) return TDF_OK;
-     const int stages = (int)std::min<size_t>((size_t)groups, (budget - tw - bars) / slot);
-     const size_t area = std::max(lines, (size_t)stages * slot);
-     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-     if (!encode) return TDF_OK;
-     for (int k = 0; k < 2; k++) {
-          // interleaved operands: sample i, detector d at word (slot*Nal + i)*nifo + d
-          const cuuint64_t rowsx = (cuuint64_t)(e->Nal / N2);
-          const cuuint64_t dx[3] = {(cuuint64_t)4 * nifo * N2, rowsx, (cuuint64_t)e->Bs};
-          const cuuint64_t sx[2] = {(cuuint64_t)nifo * N2 * 16, (cuuint64_t)e->Nal * nifo * 16};
-          const cuuint32_t bx[3] = {(cuuint32_t)(4 * nifo * LINES), (cuuint32_t)R, 1};
-          const cuuint64_t ds[3] = {(cuuint64_t)nifo * N2, rowsx, (cuuint64_t)e->Bs};
-          const cuuint64_t ss[2] = {(cuuint64_t)nifo * N2 * 4, (cuuint64_t)e->Nal * nifo * 4};
-          const cuuint32_t bs[3] = {(cuuint32_t)(nifo * LINES), (cuuint32_t)R, 1};
-          const cuuint32_t one[3] = {1, 1, 1};
-          CUresult r = encode(&e->tm_x[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, e->xab[k].p, dx, sx, bx, one,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-          if (r != CUDA_SUCCESS) return set_error(TDF_ERR_CUDA, "cuTensorMapEncodeTiled (operands xab): %d", (int)r);
-          r = encode(&e->tm_s[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, e->s2[k].p, ds, ss, bs, one,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-          if (r != CUDA_SUCCESS) return set_error(TDF_ERR_CUDA, "cuTensorMapEncodeTiled (operands s2): %d", (int)r);
-     }
-     e->stg_groups = groups;
-     e->stg_stages = stages;
-     e->stg_bar_off = (unsigned)(tw + area);
-     e->stg_smem = (unsigned)(tw + area + bars);
-     e->staged = true;
-     return TDF_OK;
-}
-
 // device inputs of one resident segment (xDat rows padded to Nal with zeros)
 static int seg_alloc(const tdf_engine *e, SegData &d) {
      const int nifo = e->nifo;
@@ -661,14 +589,22 @@ static int engine_alloc(tdf_engine *e) {
      TRY(e->B0.alloc(Q * 2 * ws * sizeof(double2)));
      TRY(e->B1.alloc(Q * 2 * ws * sizeof(double2)));
      TRY(e->B2.alloc(Q * 2 * ws * sizeof(double2)));
-     TRY(e->shftf.alloc(Q * e->Nal * sizeof(double)));
+     TRY(e->shft.alloc(Q * e->Nal * sizeof(double)));
      TRY(e->partial.alloc(Q * (e->nfft / 256) * 2 * sizeof(double)));
      for (int k = 0; k < 2; k++) TRY(e->aabb[k].alloc(Bs * sizeof(AaBb)));
      const size_t ops = Q * e->Nal;
      if (e->form == TDF_FORM_SPLIT) {
+          TRY(e->t_f32.build(e->nfftf));
+          TRY(e->t_f32.build_split());
+          const int N2 = e->t_f32.N2;
+          e->CL = ((e->N + N2 - 1) / N2 + 31) / 32 * 32;
+          const size_t cols = Q * N2 * (size_t)e->CL;
           for (int k = 0; k < 2; k++) {
-               TRY(e->xab[k].alloc(ops * sizeof(float4)));
-               TRY(e->s2[k].alloc(ops * sizeof(float)));
+               TRY(e->xab[k].alloc(cols * sizeof(float4)));
+               TRY(e->s2[k].alloc(cols * sizeof(float)));
+               // entries past the last sample are never written and stay zero
+               CUCHK(cudaMemset(e->xab[k].p, 0, e->xab[k].bytes));
+               CUCHK(cudaMemset(e->s2[k].p, 0, e->s2[k].bytes));
           }
      } else {
           for (int k = 0; k < 2; k++) {
@@ -689,8 +625,8 @@ static int engine_alloc(tdf_engine *e) {
           TRY(L.tcnt.alloc((G + 1) * sizeof(unsigned)));
           CUCHK(cudaMemset(L.tcnt.p, 0, L.tcnt.bytes));
           TRY(L.cand.alloc(e->cand_cap * sizeof(uint4)));
-          // edge ring: 2 floats per (template, row CTA, k2) = nfftf bytes per template
-          if (e->form == TDF_FORM_SPLIT) TRY(L.Ebuf.alloc(G * (size_t)e->nfftf));
+          // edge ring: 2 floats per (template, row CTA, k2)
+          if (e->form == TDF_FORM_SPLIT) TRY(L.Ebuf.alloc(G * (size_t)e->nfftf / RUN * 2 * sizeof(float)));
           TRY(L.ctl.alloc((2 + (size_t)Tc) * sizeof(unsigned)));
           CUCHK(cudaMemset(L.ctl.p, 0, L.ctl.bytes));
      }
@@ -708,12 +644,7 @@ static int engine_alloc(tdf_engine *e) {
      CUCHK(cudaMallocHost((void **)&e->h_cnt, 4 * sizeof(unsigned long long)));
      TRY(e->t_nfft.build(e->nfft));
      TRY(e->t_ninterp.build(e->Ninterp));
-     if (e->form == TDF_FORM_SPLIT) {
-          TRY(e->t_f32.build(e->nfftf));
-          TRY(e->t_f32.build_base());
-     }
-     else TRY(e->t_f64.build(e->nfftf));
-     TRY(staged_setup(e));
+     if (e->form == TDF_FORM_FP64) TRY(e->t_f64.build(e->nfftf));
      return TDF_OK;
 }
 
@@ -730,7 +661,7 @@ static void engine_free(tdf_engine *e) {
      graphs_clear(e);
      for (SegData &d : e->sdv) d.release();
      DevBuf *bufs[] = {&e->pco, &e->gco, &e->plan_sky, &e->plan_tp, &e->plan_pts, &e->skyp[0],
-                       &e->skyp[1], &e->B0, &e->B1, &e->B2, &e->shftf, &e->partial, &e->aabb[0], &e->aabb[1],
+                       &e->skyp[1], &e->B0, &e->B1, &e->B2, &e->shft, &e->partial, &e->aabb[0], &e->aabb[1],
                        &e->xab[0], &e->xab[1], &e->s2[0], &e->s2[1], &e->xa64[0], &e->xa64[1], &e->xb64[0],
                        &e->xb64[1], &e->t1[0], &e->t1[1], &e->tparam, &e->trig[0], &e->trig[1],
                        &e->counters[0], &e->counters[1], &e->linesd};
@@ -885,8 +816,8 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
      k_sky_prep<<<dim3(nblk, Q), 256, 0, st>>>(
           e->S().xdat.as<float>(), e->S().detssb.as<double>(), e->S().cosm.as<double>(), e->S().sinm.as<double>(),
           dsky, e->S().detp.as<DetParam>(), nifo, e->N, e->nfft, e->Nal, e->S().seg.oms,
-          e->B0.as<double2>(), ws, e->shftf.as<double>(), split ? e->s2[sl].as<float>() : nullptr,
-          split ? nullptr : e->t1[sl].as<double>(), e->partial.as<double>());
+          e->B0.as<double2>(), ws, e->shft.as<double>(), split ? nullptr : e->t1[sl].as<double>(),
+          e->partial.as<double>());
      CUCHK(cudaGetLastError());
      k_sky_sums<<<npts, 256, 0, st>>>(e->partial.as<double>(), nblk, e->S().detp.as<DetParam>(), nifo,
                                        e->aabb[sl].as<AaBb>());
@@ -923,10 +854,17 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
           k_spline_bwd<<<g, SPL_T, 0, st>>>(e->B1.as<double2>(), e->B2.as<double2>(), ws, e->gco.as<double>(), e->n2N);
           CUCHK(cudaGetLastError());
      }
-     k_splint<<<dim3((e->N + 255) / 256, Q), 256, 0, st>>>(
-          e->B0.as<double2>(), e->B2.as<double2>(), ws, e->shftf.as<double>(), e->Nal, e->N, e->n2N,
-          e->S().seg.interpftpad, e->S().detp.as<DetParam>(), nifo, split ? e->xab[sl].as<float4>() : nullptr,
-          split ? nullptr : e->xa64[sl].as<double2>(), split ? nullptr : e->xb64[sl].as<double2>());
+     const SplintIn in{e->B0.as<double2>(), e->B2.as<double2>(), ws, e->shft.as<double>(), dsky,
+                       e->S().detssb.as<double>(), e->S().detp.as<DetParam>(), e->Nal, e->N, e->n2N,
+                       e->S().seg.interpftpad, nifo};
+     if (split) {
+          const int N2 = e->t_f32.N2;
+          k_splint_split<<<dim3(N2 / 32, ((e->N + N2 - 1) / N2 + 7) / 8, Q), 256, 0, st>>>(
+               in, N2, e->CL, e->xab[sl].as<float4>(), e->s2[sl].as<float>());
+     } else {
+          k_splint<<<dim3((e->N + 255) / 256, Q), 256, 0, st>>>(in, e->xa64[sl].as<double2>(),
+                                                                e->xb64[sl].as<double2>());
+     }
      CUCHK(cudaGetLastError());
      e->launches += 3;
      CUCHK(cudaEventRecord(e->sky_done[sl], st));
@@ -942,74 +880,90 @@ static cudaStream_t lane_stream(const tdf_engine *e, int l) { return l == 0 ? e-
 // at most Gt templates (one chunk when a chunk is larger)
 static int group_templates(const tdf_engine *e) { return std::max(1, e->Gt / e->Tc) * e->Tc; }
 
-// Split-form spindown passes with the four-step geometry fixed at compile
-// time for the transform lengths of the benchmark sizes (nfftf 2^15 .. 2^18,
-// two detectors); every other case takes the same policies with the
-// geometry read at run time.
-template <int L, int N2C>
-static int launch_split_col_c(dim3 grid, const DemodSplitIL &p, const StoreFourstepG<0> &g, const float2 *tw,
-                              cudaStream_t st) {
-     DemodSplitILT<N2C, 2> pro{p.xab, p.s2, p.tp, p.N, p.N2, p.Nal, p.nifo};
-     StoreFourstepG<N2C> epi{g.y, g.w0, g.ws, g.N2, g.N};
-     return launch_col_L<float, L, -1, 2>(grid, pro, epi, tw, st);
+// Launches of the split-form passes: the line length, N1 = N2 or 2 N2 and the
+// detector count (1..3; more: read at run time) are compile-time constants.
+template <int L, int N2, int NIFO, int T>
+static int launch_split_col_t(const SplitCol &a, cudaStream_t st) {
+     auto kern = k_split_col<L, N2, NIFO, T>;
+     const size_t smem = split_col_lines<L>() * T * SplitLine<L, false>::BYTES;
+     TRY(set_smem(kern, smem));
+     kern<<<dim3(N2 / split_col_lines<L>(), (a.nt + T - 1) / T), split_col_threads<L>(), smem, st>>>(a);
+     CUCHK(cudaGetLastError());
+     return TDF_OK;
 }
 
-static int launch_split_col(int nifo, int N1, int N2, dim3 grid, const DemodSplitIL &pro, const StoreFourstepG<0> &epi,
-                            const float2 *tw, cudaStream_t st) {
-     if (nifo == 2) {
-          if (N1 == 512 && N2 == 512) return launch_split_col_c<512, 512>(grid, pro, epi, tw, st);
-          if (N1 == 512 && N2 == 256) return launch_split_col_c<512, 256>(grid, pro, epi, tw, st);
-          if (N1 == 256 && N2 == 256) return launch_split_col_c<256, 256>(grid, pro, epi, tw, st);
-          if (N1 == 256 && N2 == 128) return launch_split_col_c<256, 128>(grid, pro, epi, tw, st);
+// Two templates per thread when that still gives every SM its two CTAs; the
+// operands are then read once for both.  At 2^18 points (48 templates, two
+// detectors) 1.41 against 1.59 us per template; below that grid size the
+// halved CTA count costs more: 2^14 points, 16 templates, 0.59 against 0.56.
+template <int L, int N2, int NIFO>
+static int launch_split_col_c(int sms, const SplitCol &a, cudaStream_t st) {
+     if constexpr (NIFO > 0)
+          if ((a.nt / 2) * (N2 / split_col_lines<L>()) >= 2 * sms) return launch_split_col_t<L, N2, NIFO, 2>(a, st);
+     return launch_split_col_t<L, N2, NIFO, 1>(a, st);
+}
+
+template <int L, int N2>
+static int launch_split_col_n(int sms, const SplitCol &a, cudaStream_t st) {
+     switch (a.nifo) {
+     case 1: return launch_split_col_c<L, N2, 1>(sms, a, st);
+     case 2: return launch_split_col_c<L, N2, 2>(sms, a, st);
+     case 3: return launch_split_col_c<L, N2, 3>(sms, a, st);
      }
-     return launch_col<float, -1, 2>(N1, grid, pro, epi, tw, st);
+     return launch_split_col_c<L, N2, 0>(sms, a, st);
 }
 
-template <int L, int N1C, bool HALF>
-static int launch_split_row_c(dim3 grid, const RowsYBulk<float> &src, const StoreFstatT<0, false> &f,
-                              const float2 *tw, cudaStream_t st) {
-     StoreFstatT<N1C, HALF> epi{f.F, f.tp, f.ab, f.nF, f.fr0, f.fr1, f.N1, f.thr, f.cand, f.cand_cnt, f.cand_cap, f.boff,
-                                f.E, f.scand};
-     return launch_row_L<float, L, -1, 2>(grid, src, epi, tw, st);
+static int launch_split_col(int N1, int N2, int sms, const SplitCol &a, cudaStream_t st) {
+     const bool square = N1 == N2;   // else N1 = 2 N2
+     switch (N1) {
+     case 64: return launch_split_col_n<64, 64>(sms, a, st);
+     case 128: return square ? launch_split_col_n<128, 128>(sms, a, st) : launch_split_col_n<128, 64>(sms, a, st);
+     case 256: return square ? launch_split_col_n<256, 256>(sms, a, st) : launch_split_col_n<256, 128>(sms, a, st);
+     case 512: return square ? launch_split_col_n<512, 512>(sms, a, st) : launch_split_col_n<512, 256>(sms, a, st);
+     case 1024: return square ? launch_split_col_n<1024, 1024>(sms, a, st) : launch_split_col_n<1024, 512>(sms, a, st);
+     }
+     return set_error(TDF_ERR_UNSUPPORTED, "column FFT length %d", N1);
 }
 
-template <int L, int N1C>
-static int launch_split_row_h(bool half, dim3 grid, const RowsYBulk<float> &src, const StoreFstatT<0, false> &f,
-                              const float2 *tw, cudaStream_t st) {
-     return half ? launch_split_row_c<L, N1C, true>(grid, src, f, tw, st)
-                 : launch_split_row_c<L, N1C, false>(grid, src, f, tw, st);
+template <int L, int N1, bool HALF>
+static int launch_split_row_c(int sms, const SplitRow &a, cudaStream_t st) {
+     auto kern = k_split_row<L, N1, HALF>;
+     const size_t smem = split_row_smem<L>();
+     TRY(set_smem(kern, smem));
+     kern<<<std::min(sms, a.nt * (N1 / RUN)), 512, smem, st>>>(a);
+     CUCHK(cudaGetLastError());
+     return TDF_OK;
 }
 
 // the row pass keeps only bins <= fr1; with fr1 < nfftf/2 = N1*N2/2 every
 // kept output has k2 < N2/2
-static int launch_split_row(int N1, int N2, int fr1, dim3 grid, const RowsYBulk<float> &src,
-                            const StoreFstatT<0, false> &epi, const float2 *tw, cudaStream_t st) {
-     const bool half = (int64_t)fr1 < (int64_t)N1 * N2 / 2;
-     if (N2 == 512 && N1 == 512) return launch_split_row_h<512, 512>(half, grid, src, epi, tw, st);
-     if (N2 == 256 && N1 == 512) return launch_split_row_h<256, 512>(half, grid, src, epi, tw, st);
-     if (N2 == 256 && N1 == 256) return launch_split_row_h<256, 256>(half, grid, src, epi, tw, st);
-     if (N2 == 128 && N1 == 256) return launch_split_row_h<128, 256>(half, grid, src, epi, tw, st);
-     return launch_row<float, -1, 2>(N2, grid, src, epi, tw, st);
+template <int L, int N1>
+static int launch_split_row_h(int sms, const SplitRow &a, cudaStream_t st) {
+     return (int64_t)a.fr1 < (int64_t)N1 * L / 2 ? launch_split_row_c<L, N1, true>(sms, a, st)
+                                                 : launch_split_row_c<L, N1, false>(sms, a, st);
+}
+
+static int launch_split_row(int N1, int N2, int sms, const SplitRow &a, cudaStream_t st) {
+     const bool square = N1 == N2;
+     switch (N2) {
+     case 64: return square ? launch_split_row_h<64, 64>(sms, a, st) : launch_split_row_h<64, 128>(sms, a, st);
+     case 128: return square ? launch_split_row_h<128, 128>(sms, a, st) : launch_split_row_h<128, 256>(sms, a, st);
+     case 256: return square ? launch_split_row_h<256, 256>(sms, a, st) : launch_split_row_h<256, 512>(sms, a, st);
+     case 512: return square ? launch_split_row_h<512, 512>(sms, a, st) : launch_split_row_h<512, 1024>(sms, a, st);
+     case 1024: return launch_split_row_h<1024, 1024>(sms, a, st);
+     }
+     return set_error(TDF_ERR_UNSUPPORTED, "row FFT length %d", N2);
 }
 
 // The two split-form passes of nt templates as one ordered launch of
 // persistent CTAs (k_spinpass), for N1 = N2 = L (nfftf 2^16, 2^18) and two
 // detectors; ctl (2 + nt words) is zeroed first, on the same stream.
 template <int L, bool HALF>
-static int launch_spin_c(int nt, int lag, const DemodSplitIL &p, const StoreFourstepG<0> &g, const RowsYBulk<float> &s,
-                         const StoreFstatT<0, false> &f, const float2 *tw, unsigned *ctl, unsigned *err,
+static int launch_spin_c(int nt, int lag, const SplitCol &col, const SplitRow &row, unsigned *ctl, unsigned *err,
                          cudaStream_t st) {
-     DemodSplitILT<L, 2> pro{p.xab, p.s2, p.tp, p.N, p.N2, p.Nal, p.nifo};
-     StoreFourstepG<L> epic{g.y, g.w0, g.ws, g.N2, g.N};
-     StoreFstatT<L, HALF> epir{f.F, f.tp, f.ab, f.nF, f.fr0, f.fr1, f.N1, f.thr, f.cand, f.cand_cnt, f.cand_cap, f.boff,
-                               f.E, f.scand};
-     RowsYBulk<float> src = s;
-     size_t smem = pass_smem_bytes<float, L, 2>();
-     smem = (smem + 15) / 16 * 16;
-     src.bar_off = (unsigned)smem;
-     smem += 16;
-     SpinOrder o{ctl, err, nt, L / LINES, L / LINES, std::max(1, std::min(lag, nt)), 1 << 20};
-     auto kern = k_spinpass<L, DemodSplitILT<L, 2>, StoreFourstepG<L>, RowsYBulk<float>, StoreFstatT<L, HALF>>;
+     const size_t smem = std::max(RUN / 2 * SplitLine<L, false>::BYTES, SplitLine<L, true>::BYTES);
+     SpinOrder o{ctl, err, nt, L / RUN, L / RUN, std::max(1, std::min(lag, nt)), 1 << 20};
+     auto kern = k_spinpass<L, HALF>;
      TRY(set_smem(kern, smem));
      // as many CTAs as are resident at once (queried once per device and variant)
      static std::mutex mu;
@@ -1023,7 +977,7 @@ static int launch_spin_c(int nt, int lag, const DemodSplitIL &p, const StoreFour
                nres = resident[dev];
           } else {
                int per_sm = 0, nsm = 0;
-               CUCHK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, pass_threads<L>(), smem));
+               CUCHK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, split_row_threads<L>(), smem));
                CUCHK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
                nres = std::max(1, per_sm) * std::max(1, nsm);
                if (dev < 64) resident[dev] = nres;
@@ -1031,14 +985,14 @@ static int launch_spin_c(int nt, int lag, const DemodSplitIL &p, const StoreFour
      }
      const unsigned items = (unsigned)nt * (unsigned)(o.C + o.R);
      CUCHK(cudaMemsetAsync(ctl, 0, (2 + (size_t)nt) * sizeof(unsigned), st));
-     kern<<<std::min(items, (unsigned)nres), pass_threads<L>(), smem, st>>>(pro, epic, src, epir, tw, o);
+     kern<<<std::min(items, (unsigned)nres), split_row_threads<L>(), smem, st>>>(col, row, o);
      CUCHK(cudaGetLastError());
      return TDF_OK;
 }
 
 // whether the chunk passes of this engine run as one ordered launch
 static bool spin_fused(const tdf_engine *e, int N1, int N2) {
-     return e->fused && !e->staged && e->row_bulk && e->nifo == 2 && N1 == N2 && (N1 == 512 || N1 == 256);
+     return e->fused && e->nifo == 2 && N1 == N2 && (N1 == 512 || N1 == 256);
 }
 
 template <typename T>
@@ -1053,87 +1007,47 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
      const TmplParam *ctp = dtp + boff;
      const unsigned G = (unsigned)group_templates(e);
      unsigned *tcnt = Ln.tcnt.as<unsigned>();
+     unsigned *errw = reinterpret_cast<unsigned *>(e->counters[e->cur].as<unsigned long long>() + 1);
+     const bool blocks = e->opts.blocks_avg && e->nblk_mu > 0;
      size_t tev = e->timing ? timing_begin(e, st) : (size_t)-1;
      if constexpr (std::is_same<T, float>::value) {
+          const SplitCol col{e->xab[e->cur].as<float4>(), e->s2[e->cur].as<float>(), ctp, Ln.Ybuf.as<float4>(),
+                             t.base.template as<float2>(), t.step.template as<float2>(), t.ltw1.template as<float2>(),
+                             e->N, e->CL, (e->N + t.N2 - 1) / t.N2, e->nifo, nt};
+          SplitRow row{Ln.Ybuf.as<float4>(), t.ltw2.template as<float2>(), Ln.Fbuf.as<float>() + (size_t)boff * e->nF,
+                       ctp, e->aabb[e->cur].as<AaBb>(), e->nF, e->opts.fr[0], e->opts.fr[1], e->opts.thr,
+                       blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff, nullptr, nullptr, nt, errw};
+          if (e->sparse_now) {
+               row.cand = nullptr;
+               row.E = Ln.Ebuf.as<float>();
+               row.scand = Ln.cand.as<uint4>();
+          }
           if (spin_fused(e, t.N1, t.N2)) {
-               StoreFourstepG<0> epi{Ln.Ybuf.as<float2>(), t.base.template as<float2>(), t.step.template as<float2>(),
-                                     t.N2, e->nfftf};
-               DemodSplitIL pro{e->xab[e->cur].as<float4>(), e->s2[e->cur].as<float>(), ctp, e->N, t.N2, e->Nal,
-                                e->nifo};
-               unsigned *errw = reinterpret_cast<unsigned *>(e->counters[e->cur].as<unsigned long long>() + 1);
-               const bool blocks = e->opts.blocks_avg && e->nblk_mu > 0;
-               StoreFstatT<0, false> epi2{Ln.Fbuf.as<float>() + (size_t)boff * e->nF, ctp, e->aabb[e->cur].as<AaBb>(),
-                                          e->nF, e->opts.fr[0], e->opts.fr[1], t.N1, e->opts.thr,
-                                          blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff};
-               if (e->sparse_now) {
-                    epi2.cand = nullptr;
-                    epi2.E = Ln.Ebuf.as<float>();
-                    epi2.scand = Ln.cand.as<uint4>();
-               }
-               RowsYBulk<float> src{Ln.Ybuf.as<float2>(), e->nfftf, t.N2, errw};
                const bool half = (int64_t)e->opts.fr[1] < (int64_t)t.N1 * t.N2 / 2;
                unsigned *ctl = Ln.ctl.as<unsigned>();
-               const float2 *tw = t.l1();   // N1 = N2: the row pass's line table is the same
                int rc;
                if (t.N1 == 512)
-                    rc = half ? launch_spin_c<512, true>(nt, e->fuse_lag, pro, epi, src, epi2, tw, ctl, errw, st)
-                              : launch_spin_c<512, false>(nt, e->fuse_lag, pro, epi, src, epi2, tw, ctl, errw, st);
+                    rc = half ? launch_spin_c<512, true>(nt, e->fuse_lag, col, row, ctl, errw, st)
+                              : launch_spin_c<512, false>(nt, e->fuse_lag, col, row, ctl, errw, st);
                else
-                    rc = half ? launch_spin_c<256, true>(nt, e->fuse_lag, pro, epi, src, epi2, tw, ctl, errw, st)
-                              : launch_spin_c<256, false>(nt, e->fuse_lag, pro, epi, src, epi2, tw, ctl, errw, st);
+                    rc = half ? launch_spin_c<256, true>(nt, e->fuse_lag, col, row, ctl, errw, st)
+                              : launch_spin_c<256, false>(nt, e->fuse_lag, col, row, ctl, errw, st);
                TRY(rc);
                if (e->timing) timing_end(e, tev, KT_COL, nt, st);
                e->launches += 1;   // the memset before it is not a kernel
                return TDF_OK;
           }
-          StoreFourstepG<0> epi{Ln.Ybuf.as<float2>(), t.base.template as<float2>(), t.step.template as<float2>(), t.N2,
-                                e->nfftf};
-          if (e->staged) {
-               DemodSplitStaged pro;
-               pro.mx = e->tm_x[e->cur];
-               pro.ms = e->tm_s[e->cur];
-               pro.tp = ctp;
-               pro.err = reinterpret_cast<unsigned *>(e->counters[e->cur].as<unsigned long long>() + 1);
-               pro.N = e->N;
-               pro.N2 = t.N2;
-               pro.nifo = e->nifo;
-               pro.groups = e->stg_groups;
-               pro.stages = e->stg_stages;
-               pro.bar_off = e->stg_bar_off;
-               pro.smem = e->stg_smem;
-               TRY((launch_col<T, -1, 2>(t.N1, dim3(t.N2 / LINES, nt), pro, epi, t.l1(), st)));
-          } else {
-               DemodSplitIL pro{e->xab[e->cur].as<float4>(), e->s2[e->cur].as<float>(), ctp, e->N, t.N2, e->Nal,
-                                e->nifo};
-               TRY(launch_split_col(e->nifo, t.N1, t.N2, dim3(t.N2 / LINES, nt), pro, epi, t.l1(), st));
-          }
+          TRY(launch_split_col(t.N1, t.N2, e->sms, col, st));
+          if (e->timing) timing_end(e, tev, KT_COL, nt, st);
+          tev = e->timing ? timing_begin(e, st) : (size_t)-1;
+          TRY(launch_split_row(t.N1, t.N2, e->sms, row, st));
      } else {
           StoreFourstep<T, -1, 2> epi{Ln.Ybuf.as<cx<T>>(), t.h(), t.o(), t.N2, e->nfftf};
           DemodFP64 pro{e->xa64[e->cur].as<double2>(), e->xb64[e->cur].as<double2>(), e->t1[e->cur].as<double>(), ctp,
                         e->N, t.N2, e->Nal, e->nifo};
           TRY((launch_col<T, -1, 2>(t.N1, dim3(t.N2 / LINES, nt), pro, epi, t.l1(), st)));
-     }
-     if (e->timing) timing_end(e, tev, KT_COL, nt, st);
-     const bool blocks = e->opts.blocks_avg && e->nblk_mu > 0;
-     tev = e->timing ? timing_begin(e, st) : (size_t)-1;
-     unsigned *errw = reinterpret_cast<unsigned *>(e->counters[e->cur].as<unsigned long long>() + 1);
-     if constexpr (std::is_same<T, float>::value) {
-          StoreFstatT<0, false> epi2{Ln.Fbuf.as<float>() + (size_t)boff * e->nF, ctp, e->aabb[e->cur].as<AaBb>(), e->nF,
-                                     e->opts.fr[0], e->opts.fr[1], t.N1, e->opts.thr,
-                                     blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff};
-          if (e->sparse_now) {
-               epi2.cand = nullptr;
-               epi2.E = Ln.Ebuf.as<float>();
-               epi2.scand = Ln.cand.as<uint4>();
-          }
-          if (e->row_bulk) {
-               RowsYBulk<float> src{Ln.Ybuf.as<float2>(), e->nfftf, t.N2, errw};
-               TRY(launch_split_row(t.N1, t.N2, e->opts.fr[1], dim3(t.N1 / LINES, nt), src, epi2, t.l2(), st));
-          } else {
-               RowsY<float, 2> src{Ln.Ybuf.as<float2>(), e->nfftf, t.N2};
-               TRY((launch_row<float, -1, 2>(t.N2, dim3(t.N1 / LINES, nt), src, epi2, t.l2(), st)));
-          }
-     } else {
+          if (e->timing) timing_end(e, tev, KT_COL, nt, st);
+          tev = e->timing ? timing_begin(e, st) : (size_t)-1;
           StoreFstat<T> epi2{Ln.Fbuf.as<T>() + (size_t)boff * e->nF, ctp, e->aabb[e->cur].as<AaBb>(), e->nF,
                              e->opts.fr[0], e->opts.fr[1], t.N1, e->opts.thr,
                              blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff};
@@ -1245,6 +1159,7 @@ static int set_graph_priorities(const tdf_engine *e, cudaGraph_t g) {
                register_sky_kernel((const void *)k_spline_fwd);
                register_sky_kernel((const void *)k_spline_bwd);
                register_sky_kernel((const void *)k_splint);
+               register_sky_kernel((const void *)k_splint_split);
           });
      }
      size_t n = 0;
@@ -1840,9 +1755,12 @@ int tdf_engine_create(const tdf_segment *seg, const tdf_search_opts *opts, int f
      }
      if (device < 0 || device >= ndev) return set_error(TDF_ERR_INVALID, "device %d of %d", device, ndev);
      CUCHK(cudaSetDevice(device));
+     int sms = 0;
+     CUCHK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
      tdf_engine *e = new tdf_engine();
      e->dev = device;
      e->form = form;
+     e->sms = sms;
      e->sdv.resize(1);
      e->act = 0;
      e->S().seg = *seg;
@@ -1852,8 +1770,6 @@ int tdf_engine_create(const tdf_segment *seg, const tdf_search_opts *opts, int f
      e->nfftf = seg->nfftf;
      e->Ninterp = seg->Ninterp;
      e->nifo = seg->nifo;
-     // a multiple of every row length N2 <= 1024 of the four-step split, so
-     // that the operand arrays view as whole rows for the TMA boxes
      e->Nal = (seg->N + 1023) / 1024 * 1024;
      e->n2N = seg->interpftpad * seg->N;
      e->nF = opts->fr[1] - opts->fr[0] + 1;

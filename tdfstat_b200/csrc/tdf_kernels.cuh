@@ -12,10 +12,10 @@
 //     k_splint        spline evaluation at 2(i - shftf[i]) (auxi.c:120-169),
 //                     division by sig2, conversion to the spindown operands
 //   spindown stage (once per template)
-//     DemodSplit /
-//     DemodSplitStaged /
-//     DemodFP64       column-pass prologues: spindown_modulation
+//     (split form: tdf_split.cuh)
+//     DemodFP64       column-pass prologue: spindown_modulation
 //                     (spinmod.c:490-514) fused into the first FFT pass
+//     DemodSplit      the split form's, for the allocation-free entry point
 //     StoreFstat      row-pass epilogue: F = |Fa|^2/aa + |Fb|^2/bb
 //                     (jobcore.c:481-484)
 //     k_block_means   FStat blocks_avg means (auxi.c:336-363)
@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(256) k_sky_prep(
      const double *__restrict__ cosm, const double *__restrict__ sinm,
      const SkyParam *__restrict__ sp, const DetParam *__restrict__ dp,
      int nifo, int N, int nfft, int Nal, double oms,
-     double2 *__restrict__ W, size_t Wstride, double *__restrict__ shftf,
-     float *__restrict__ s2, double *__restrict__ t1, double *__restrict__ partial)
+     double2 *__restrict__ W, size_t Wstride, double *__restrict__ shft,
+     double *__restrict__ t1, double *__restrict__ partial)
 {
      const int q = blockIdx.y, p = q / nifo, d = q % nifo;
      const int i = blockIdx.x * 256 + threadIdx.x;
@@ -111,12 +111,9 @@ __global__ void __launch_bounds__(256) k_sky_prep(
                // ~1e5 rad, so its rounding must follow the reference's
                const double sh = __dadd_rn(__dadd_rn(__dmul_rn(S.nS0, e[3 * (size_t)i]), __dmul_rn(S.nS1, e[3 * (size_t)i + 1])),
                                            __dmul_rn(S.nS2, e[3 * (size_t)i + 2]));
-               const double sh1 = __dadd_rn(__dadd_rn(__dmul_rn(S.nS0, e[0]), __dmul_rn(S.nS1, e[1])), __dmul_rn(S.nS2, e[2]));
-               shftf[(size_t)q * Nal + i] = __dsub_rn(sh, sh1);
+               shft[(size_t)q * Nal + i] = sh;
                const size_t o = ((size_t)p * nifo + d) * Nal + i;      // planar (FP64 operands)
-               const size_t oi = ((size_t)p * Nal + i) * nifo + d;     // interleaved by detector (split)
                const double di = (double)i;
-               if (s2) s2[oi] = (float)__dmul_rn((double)(2 * i), sh);
                if (t1) t1[o] = __dadd_rn(__dmul_rn(di, di), __dmul_rn((double)(2 * i), sh));
                const double phase = __dadd_rn(__dmul_rn(S.het0, di), __dmul_rn(oms, sh));
                double sn, cn;
@@ -411,28 +408,78 @@ __device__ __forceinline__ double2 splint_eval(const double2 *__restrict__ ya, c
                          a * yl.y + b * yh.y + (ca * sl.y + cb * sh.y) / 6.0);
 }
 
-// grid (ceil(N/256), Q), 256 threads: xDatm{a,b}[i] = splint(...)/sig2 as
-// split (float4 xa.re, xa.im, xb.re, xb.im, interleaved by detector:
-// [slot][i][det]) or FP64 (two double2, planar: [slot][det][i]) operands
-__global__ void __launch_bounds__(256) k_splint(
-     const double2 *__restrict__ Z, const double2 *__restrict__ Y2, size_t stride,
-     const double *__restrict__ shftf, int Nal, int N, int n, int interpftpad,
-     const DetParam *__restrict__ dp, int nifo,
-     float4 *__restrict__ xab, double2 *__restrict__ xa64, double2 *__restrict__ xb64)
+// shft_n[0] as k_sky_prep forms shft_n[i]
+__device__ __forceinline__ double shft0(const SkyParam &S, const double *e) {
+     return __dadd_rn(__dadd_rn(__dmul_rn(S.nS0, e[0]), __dmul_rn(S.nS1, e[1])), __dmul_rn(S.nS2, e[2]));
+}
+
+// The inputs of the resampling (jobcore.c:314-370): samples Z and second
+// derivatives Y2 of array (q, a|b), q = point*nifo + det, `stride` apart.
+struct SplintIn {
+     const double2 *Z, *Y2;
+     size_t stride;
+     const double *shft;      // [q][Nal]
+     const SkyParam *sp;
+     const double *detssb;
+     const DetParam *dp;
+     int Nal, N, n, interpftpad, nifo;
+};
+
+// xDatm{a,b}[i] = splint(interpftpad*(i - (shft[i] - shft[0])))/sig2
+__device__ __forceinline__ void splint_at(const SplintIn &I, int q, int i, double sh, double sh1, double s2, double2 &a,
+                                          double2 &b) {
+     const double x = I.interpftpad * (i - __dsub_rn(sh, sh1));
+     const double2 va = splint_eval(I.Z + ((size_t)q * 2) * I.stride, I.Y2 + ((size_t)q * 2) * I.stride, I.n, x);
+     const double2 vb = splint_eval(I.Z + ((size_t)q * 2 + 1) * I.stride, I.Y2 + ((size_t)q * 2 + 1) * I.stride, I.n, x);
+     a = make_double2(va.x / s2, va.y / s2);
+     b = make_double2(vb.x / s2, vb.y / s2);
+}
+
+// FP64 operands, planar: [slot][det][i].  grid (ceil(N/256), Q), 256 threads
+__global__ void __launch_bounds__(256) k_splint(const __grid_constant__ SplintIn I, double2 *__restrict__ xa64,
+                                                double2 *__restrict__ xb64)
 {
-     const int q = blockIdx.y, p = q / nifo, d = q % nifo;
+     const int q = blockIdx.y, d = q % I.nifo;
      const int i = blockIdx.x * 256 + threadIdx.x;
-     if (i >= N) return;
-     const double x = interpftpad * (i - shftf[(size_t)q * Nal + i]);
-     const double2 va = splint_eval(Z + ((size_t)q * 2) * stride, Y2 + ((size_t)q * 2) * stride, n, x);
-     const double2 vb = splint_eval(Z + ((size_t)q * 2 + 1) * stride, Y2 + ((size_t)q * 2 + 1) * stride, n, x);
-     const double s2 = dp[d].sig2;
-     const double2 a = make_double2(va.x / s2, va.y / s2), b = make_double2(vb.x / s2, vb.y / s2);
-     if (xab) xab[((size_t)p * Nal + i) * nifo + d] = make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
-     if (xa64) {
-          const size_t o = ((size_t)p * nifo + d) * Nal + i;
-          xa64[o] = a;
-          xb64[o] = b;
+     if (i >= I.N) return;
+     double2 a, b;
+     splint_at(I, q, i, I.shft[(size_t)q * I.Nal + i], shft0(I.sp[q / I.nifo], I.detssb + (size_t)d * 3 * I.N),
+               I.dp[d].sig2, a, b);
+     const size_t o = (size_t)q * I.Nal + i;
+     xa64[o] = a;
+     xb64[o] = b;
+}
+
+// Split operands in the column layout of tdf_split.cuh: with i = N2*n1 + n2,
+//   xab[(q*N2 + n2)*CL + n1] = (a.re, b.re, a.im, b.im) in FP32
+//   s2[((p*N2 + n2)*CL + n1)*nifo + d] = 2 i shft[i]
+// A CTA takes a tile of 32 columns and 8 rows: it reads along i (32
+// consecutive samples per warp) and, through shared memory, writes 8
+// consecutive n1 of a column (128 bytes of xab) at a time.
+// grid (N2/32, ceil(ceil(N/N2)/8), Q), 256 threads
+__global__ void __launch_bounds__(256) k_splint_split(const __grid_constant__ SplintIn I, int N2, int CL,
+                                                      float4 *__restrict__ xab, float *__restrict__ s2out)
+{
+     __shared__ float4 xs[32][9];
+     __shared__ float ss[32][9];
+     const int q = blockIdx.z, p = q / I.nifo, d = q % I.nifo;
+     {
+          const int c = threadIdx.x % 32, r = threadIdx.x / 32;
+          const int i = N2 * (blockIdx.y * 8 + r) + blockIdx.x * 32 + c;
+          if (i < I.N) {
+               const double sh = I.shft[(size_t)q * I.Nal + i];
+               double2 a, b;
+               splint_at(I, q, i, sh, shft0(I.sp[p], I.detssb + (size_t)d * 3 * I.N), I.dp[d].sig2, a, b);
+               xs[c][r] = make_float4((float)a.x, (float)b.x, (float)a.y, (float)b.y);
+               ss[c][r] = (float)__dmul_rn((double)(2 * i), sh);
+          }
+     }
+     __syncthreads();
+     const int c = threadIdx.x / 8, r = threadIdx.x % 8;
+     const int n1 = blockIdx.y * 8 + r, n2 = blockIdx.x * 32 + c;
+     if (N2 * n1 + n2 < I.N) {
+          xab[((size_t)q * N2 + n2) * CL + n1] = xs[c][r];
+          s2out[(((size_t)p * N2 + n2) * CL + n1) * I.nifo + d] = ss[c][r];
      }
 }
 
@@ -555,189 +602,6 @@ struct DemodSplit {
      }
 };
 
-// Two detectors' demodulated operands summed in one chain of fused
-// multiply-adds per component: fa + i... = x0 (c0 - i s0) + x1 (c1 - i s1)
-// for the two arrays of x = (a.re, a.im, b.re, b.im).
-__device__ __forceinline__ void demod2(const float4 x0, const float4 x1, float ph0, float ph1, float2 &fa,
-                                       float2 &fb) {
-     float s0, c0, s1, c1;
-     __sincosf(ph0, &s0, &c0);
-     __sincosf(ph1, &s1, &c1);
-     fa.x = fmaf(x0.x, c0, fmaf(x0.y, s0, fmaf(x1.x, c1, x1.y * s1)));
-     fa.y = fmaf(x0.y, c0, fmaf(-x0.x, s0, fmaf(x1.y, c1, -x1.x * s1)));
-     fb.x = fmaf(x0.z, c0, fmaf(x0.w, s0, fmaf(x1.z, c1, x1.w * s1)));
-     fb.y = fmaf(x0.w, c0, fmaf(-x0.z, s0, fmaf(x1.w, c1, -x1.z * s1)));
-}
-
-// DemodSplit over operands interleaved by detector, xab[(slot*Nal + i)*nifo
-// + d] and s2 likewise (the engine's layout): with two detectors a sample's
-// operands are two adjacent 16-byte words and one 8-byte word, each read
-// from one address, and one pointer per operand array steps through the
-// thread's samples.  Same arithmetic, in the same order, as DemodSplit.
-// CN2 / CNIFO > 0 fix the row length N2 and the detector count at compile
-// time (the thread's eight samples are then constant offsets from one
-// pointer); 0 reads them from the struct.
-template <int CN2 = 0, int CNIFO = 0>
-struct DemodSplitILT {
-     const float4 *xab;
-     const float *s2;
-     const TmplParam *tp;
-     int N, N2, Nal, nifo;
-
-     template <int L>
-     __device__ __forceinline__ void load(float2 (&v)[2][8], int b, int n2, int t) const {
-          const int n2s = CN2 > 0 ? CN2 : N2;
-          const int nf = CNIFO > 0 ? CNIFO : nifo;
-          const TmplParam P = tp[b];
-          const float spf = (float)P.spnd;
-          const int i0 = n2s * t + n2;
-          const int di = n2s * (L / 8);   // samples between the thread's elements
-          const int de = di * nf;         // operand words between them
-          const size_t e0 = ((size_t)P.slot * Nal + i0) * nf;
-          const float4 *xp = xab + e0;
-          const float *sp = s2 + e0;
-#pragma unroll
-          for (int m = 0; m < 8; m++) {
-               const int i = i0 + m * di;
-               float2 fa = make_float2(0.f, 0.f), fb = make_float2(0.f, 0.f);
-               if (i < N) {
-                    const double dd = (double)i;
-                    const double ph = fma(P.spnd, dd * dd, P.het1 * dd);
-                    const double kk = rint(ph * INV_TWO_PI);
-                    const float pr = (float)fma(-kk, TWO_PI, ph);
-                    const float4 *x = xp + m * de;
-                    const float *s = sp + m * de;
-                    if (nf == 2) {
-                         // both detectors' rotated operands summed in one
-                         // chain of fused multiply-adds per component
-                         const float2 ss = __ldg(reinterpret_cast<const float2 *>(s));
-                         demod2(__ldg(x), __ldg(x + 1), fmaf(spf, ss.x, pr), fmaf(spf, ss.y, pr), fa, fb);
-                    } else if (nf == 1) {
-                         DemodSplit::rot(__ldg(x), fmaf(spf, __ldg(s), pr), fa, fb);
-                    } else {
-                         CompSum ar, ai, br, bi;
-                         for (int d = 0; d < nf; d++) {
-                              float2 pa, pb;
-                              DemodSplit::rot(__ldg(x + d), fmaf(spf, __ldg(s + d), pr), pa, pb);
-                              if (d == 0) { ar.init(pa.x); ai.init(pa.y); br.init(pb.x); bi.init(pb.y); }
-                              else { ar.add(pa.x); ai.add(pa.y); br.add(pb.x); bi.add(pb.y); }
-                         }
-                         fa = make_float2(ar.value(), ai.value());
-                         fb = make_float2(br.value(), bi.value());
-                    }
-               }
-               v[0][m] = fa;
-               v[1][m] = fb;
-          }
-     }
-};
-using DemodSplitIL = DemodSplitILT<0, 0>;
-
-// DemodSplitIL with its operands brought in by TMA.  Thread (c, t) of the CTA
-// needs, for element m, the samples of row n1 = t + m*R (R = L/8) of column
-// n2 = x0 + c, so the rows of a group m of the CTA's LINES columns, every
-// detector, form one box of each operand tensor (interleaved layout):
-//   xab as floats {4*nifo*N2, rows, slots}, box {4*nifo*LINES, R, 1}
-//   s2            {nifo*N2,   rows, slots}, box {nifo*LINES,   R, 1}
-// (rows = Nal/N2, Nal a multiple of N2).  The groups holding samples < N go
-// through a ring of `stages` shared-memory slots that aliases the line
-// buffers (unused until the first FFT pass stores), each slot completing on
-// its own mbarrier; all copies of the ring are in flight while the threads
-// demodulate, instead of one element's loads per thread at a time.
-// The arithmetic per element is DemodSplit's, in the same order.
-// Opt-in (TDF_STAGED_OPERANDS=1): with the operands L2-resident it measured
-// slower than DemodSplitIL's per-thread loads.
-struct DemodSplitStaged {
-     CUtensorMap mx;    // xab
-     CUtensorMap ms;    // s2
-     const TmplParam *tp;
-     unsigned *err;     // ERR_STAGE_TIMEOUT is or-ed in when a wait gives up
-     int N, N2, nifo;
-     int groups;        // row groups holding samples < N (<= 8)
-     int stages;        // ring slots (>= 1)
-     unsigned bar_off;  // byte offset of the ring's mbarriers in dynamic shared memory
-     unsigned smem;     // dynamic shared memory of the launch
-     static constexpr bool kStaged = true;
-
-     template <int L>
-     __device__ __forceinline__ void issue(int g, int s, unsigned char *ring, uint64_t *bars, unsigned slot_bytes,
-                                           unsigned xbytes, int x0, int w) const {
-          unsigned char *dst = ring + (size_t)s * slot_bytes;
-          mbar_expect_tx(&bars[s], slot_bytes);
-          tma_load_3d(dst, &mx, 4 * nifo * x0, g * (L / 8), w, &bars[s]);
-          tma_load_3d(dst + xbytes, &ms, nifo * x0, g * (L / 8), w, &bars[s]);
-     }
-
-     template <int L>
-     __device__ __forceinline__ void load_staged(float2 (&v)[2][8], int b, int n2, int t, unsigned char *ring,
-                                                 uint64_t *bars) const {
-          constexpr int R = L / 8;
-          const TmplParam P = tp[b];
-          const float spf = (float)P.spnd;
-          const unsigned xbytes = (unsigned)nifo * R * LINES * 16;
-          const unsigned slot_bytes = xbytes + (unsigned)nifo * R * LINES * 4;
-          const int x0 = blockIdx.x * LINES;
-          const int c = threadIdx.x % LINES;
-          if (threadIdx.x == 0) {
-               for (int s = 0; s < stages; s++) mbar_init(&bars[s], 1);
-               mbar_fence_init();
-          }
-          __syncthreads();
-          if (threadIdx.x == 0)
-               for (int g = 0; g < stages; g++) issue<L>(g, g, ring, bars, slot_bytes, xbytes, x0, (int)P.slot);
-          bool waited = true;
-          int s = 0;            // ring slot of group m
-          unsigned par = 0u;    // phase parity of that slot's barrier
-#pragma unroll
-          for (int m = 0; m < 8; m++) {
-               float2 fa = make_float2(0.f, 0.f), fb = make_float2(0.f, 0.f);
-               if (m < groups) {
-                    waited &= mbar_wait(&bars[s], par);
-                    const unsigned char *sl = ring + (size_t)s * slot_bytes;
-                    const float4 *X = reinterpret_cast<const float4 *>(sl);
-                    const float *S2 = reinterpret_cast<const float *>(sl + xbytes);
-                    const int i = N2 * (t + m * R) + n2;
-                    if (i < N) {
-                         const double di = (double)i;
-                         const double ph = fma(P.spnd, di * di, P.het1 * di);
-                         const double kk = rint(ph * INV_TWO_PI);
-                         const float pr = (float)fma(-kk, TWO_PI, ph);
-                         const int e0 = (t * LINES + c) * nifo;
-                         if (nifo == 2) {
-                              demod2(X[e0], X[e0 + 1], fmaf(spf, S2[e0], pr), fmaf(spf, S2[e0 + 1], pr), fa, fb);
-                         } else if (nifo == 1) {
-                              DemodSplit::rot(X[e0], fmaf(spf, S2[e0], pr), fa, fb);
-                         } else {
-                              CompSum ar, ai, br, bi;
-                              for (int d = 0; d < nifo; d++) {
-                                   const int ed = e0 + d;
-                                   float2 pa, pb;
-                                   DemodSplit::rot(X[ed], fmaf(spf, S2[ed], pr), pa, pb);
-                                   if (d == 0) { ar.init(pa.x); ai.init(pa.y); br.init(pb.x); bi.init(pb.y); }
-                                   else { ar.add(pa.x); ai.add(pa.y); br.add(pb.x); bi.add(pb.y); }
-                              }
-                              fa = make_float2(ar.value(), ai.value());
-                              fb = make_float2(br.value(), bi.value());
-                         }
-                    }
-                    if (m + stages < groups) {
-                         // every thread is done with slot s: refill it
-                         __syncthreads();
-                         if (threadIdx.x == 0)
-                              issue<L>(m + stages, s, ring, bars, slot_bytes, xbytes, x0, (int)P.slot);
-                    }
-                    if (++s == stages) {
-                         s = 0;
-                         par ^= 1u;
-                    }
-               }
-               v[0][m] = fa;
-               v[1][m] = fb;
-          }
-          if (!waited) atomicOr(err, ERR_STAGE_TIMEOUT);
-     }
-};
-
 // Plain FP64 form: the reference's DOUBLE-build spindown_modulation.
 struct DemodFP64 {
      const double2 *xa, *xb;
@@ -814,110 +678,11 @@ struct StoreFstat {
      }
 };
 
-// Candidate records of the sparse F store (16 bytes): template (within the
-// resolve group) | kind << 24, bin, F[bin], and one neighbour's F.
-constexpr unsigned CAND_LOCAL = 0u;   // a local maximum decided in the row pass; no tie with bin-1
-constexpr unsigned CAND_LEFT = 1u;    // first bin of a CTA's run of 8: F[bin-1] is in the edge ring (nb = F[bin+1])
-constexpr unsigned CAND_RIGHT = 2u;   // last bin of a run: F[bin+1] is in the edge ring (nb = F[bin-1])
-constexpr unsigned CAND_TIE = 3u;     // F[bin-1] == F[bin]: the MAX_ALG 3 run needs F[bin-2]
-constexpr unsigned ERR_NEED_FULL_F = 4u;   // a batch needs the full F spectra (tie or candidate overflow)
+}  // namespace tdf
 
-// StoreFstat for the split form with the four-step column count N1 fixed at
-// compile time (CN1 > 0, else the struct's N1) and, when HALF, only the
-// outputs k2 < L/2 of each row formed: every bin the search keeps lies below
-// nfftf/2 (fr1 < N1*L/2), so the upper half of the row transform's last
-// pass is never computed (its outputs are dead).  F = |Fa|^2 * (1/aa) +
-// |Fb|^2 * (1/bb), the reciprocals formed once per thread.
-//
-// Two ways to hand F to the trigger selection:
-//   full (E == nullptr): the whole spectrum [fr0, fr1] goes to the F ring
-//     and the bins passing the threshold test to the candidate list (uint2
-//     {template, bin}); used with blocks_avg and as the fallback.
-//   sparse (E != nullptr): no spectrum leaves the SM.  The 8 lanes c of a
-//     thread group hold the consecutive bins k1b + c + N1*k2 of one k2, so a
-//     bin's neighbours are one shuffle away except at the run's ends: the
-//     row pass decides the local-maximum test itself for c = 1..6 and
-//     writes candidate records (uint4, kinds above) for bins passing the
-//     threshold; only the end bins c = 0 and 7 of every run go to the edge
-//     ring E[((b*NJ + j)*L + k2)*2 + (c == 7)] (j = CTA index) for the
-//     neighbours of the other CTAs' end-bin candidates.
-template <int CN1, bool HALF>
-struct StoreFstatT {
-     float *F;
-     const TmplParam *tp;
-     const AaBb *ab;
-     int nF, fr0, fr1, N1;
-     double thr;
-     uint2 *cand;
-     unsigned *cand_cnt;
-     unsigned cand_cap;
-     int boff;        // index of this chunk's first template within its resolve group
-     float *E = nullptr;       // sparse form: edge ring of the resolve group
-     uint4 *scand = nullptr;   // sparse form: candidate records
-     template <int L>
-     __device__ __forceinline__ void store(const float2 (&v)[2][8], int b, int k1, int t) const {
-          const AaBb s = ab[tp[b].slot];
-          const float ia = 1.f / s.aaf, ib = 1.f / s.bbf;
-          const float thrf = (float)thr;
-          const bool exact_thr = (double)thrf == thr;   // then f < thr compares the same in float
-          const int n1 = CN1 > 0 ? CN1 : N1;
-          if (E == nullptr) {
-               float *dst = F + (size_t)b * nF - fr0;
-#pragma unroll
-               for (int m = 0; m < (HALF ? 4 : 8); m++) {
-                    const int k = k1 + n1 * (t + m * (L / 8));
-                    if (k >= fr0 && k <= fr1) {
-                         const float f = fmaf(cnorm(v[0][m]), ia, cnorm(v[1][m]) * ib);
-                         dst[k] = f;
-                         const bool pass = exact_thr ? !(f < thrf) : !((double)f < thr);
-                         if (cand && pass && k >= fr0 + 1 && k < fr1 - 1) {
-                              const unsigned c = atomicAdd(cand_cnt, 1u);
-                              if (c < cand_cap) cand[c] = make_uint2((unsigned)(b + boff), (unsigned)k);
-                         }
-                    }
-               }
-               return;
-          }
-          const int c = k1 & (LINES - 1);
-          const int nj = n1 / LINES;
-          const unsigned bg = (unsigned)(b + boff);
-          float *ej = E + ((size_t)bg * nj + (k1 >> 3)) * (2 * L) + (c == LINES - 1 ? 1 : 0);
-#pragma unroll
-          for (int m = 0; m < (HALF ? 4 : 8); m++) {
-               const int k2 = t + m * (L / 8);
-               const int k = k1 + n1 * k2;
-               const float f = fmaf(cnorm(v[0][m]), ia, cnorm(v[1][m]) * ib);
-               // neighbours within the run of 8 (lanes c-1, c+1 of the same k2)
-               const float fm = __shfl_up_sync(0xffffffffu, f, 1, LINES);
-               const float fp = __shfl_down_sync(0xffffffffu, f, 1, LINES);
-               if (k >= fr0 && k <= fr1) {
-                    if (c == 0 || c == LINES - 1) ej[2 * k2] = f;
-                    const bool pass = exact_thr ? !(f < thrf) : !((double)f < thr);
-                    if (pass && k >= fr0 + 1 && k < fr1 - 1) {
-                         unsigned kind;
-                         float nb = 0.f;
-                         bool keep = true;
-                         if (c == 0) {
-                              kind = CAND_LEFT;
-                              nb = fp;
-                         } else if (c == LINES - 1) {
-                              kind = CAND_RIGHT;
-                              nb = fm;
-                         } else {
-                              keep = !(fm > f || f < fp);   // a local maximum
-                              kind = fm == f ? CAND_TIE : CAND_LOCAL;
-                         }
-                         if (keep) {
-                              const unsigned q = atomicAdd(cand_cnt, 1u);
-                              if (q < cand_cap)
-                                   scand[q] = make_uint4(bg | (kind << 24), (unsigned)k, __float_as_uint(f),
-                                                         __float_as_uint(nb));
-                         }
-                    }
-               }
-          }
-     }
-};
+#include "tdf_split.cuh"
+
+namespace tdf {
 
 // blocks_avg means (auxi.c:349-355): mu_j = sum of the j-th block of NAV
 // values of F[fr0..] / (2 NAV).  grid (nblk, ntmpl), 256 threads
@@ -1073,7 +838,7 @@ __global__ void __launch_bounds__(256) k_resolve_sparse(ThrArgs A, SparseArgs S)
           return;
      }
      const unsigned gs = gridDim.x * blockDim.x;
-     const int nj = S.N1 / LINES;
+     const int nj = S.N1 / RUN;
      for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gs) {
           const uint4 r = S.cand[i];
           const int b = (int)(r.x & 0xffffffu);
@@ -1085,7 +850,7 @@ __global__ void __launch_bounds__(256) k_resolve_sparse(ThrArgs A, SparseArgs S)
                continue;
           }
           if (kind != CAND_LOCAL) {
-               const int k1 = k % S.N1, k2 = k / S.N1, j = k1 / LINES;
+               const int k1 = k % S.N1, k2 = k / S.N1, j = k1 / RUN;
                const float *Eb = S.E + (size_t)b * nj * (2 * S.L);
                float fm, fp;
                if (kind == CAND_LEFT) {
