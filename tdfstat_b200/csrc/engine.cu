@@ -187,6 +187,30 @@ static int launch_row(int L, dim3 grid, const Src &src, const Epi &epi, const cx
      return set_error(TDF_ERR_UNSUPPORTED, "row FFT length %d", L);
 }
 
+template <int L>
+static int launch_interp_mid_L(dim3 grid, const double2 *y, size_t stride, const double2 *tw1, const double2 *tw2,
+                               const double *fac, int N1, StoreFourstep<double, +1, 1> epi, cudaStream_t st) {
+     epi.tab_off = (unsigned)InterpMid<L>::tab_off;
+     const size_t smem = InterpMid<L>::tab_off + StoreFourstep<double, +1, 1>::template table_bytes<2 * L>(epi.N2);
+     auto kern = k_interp_mid<L>;
+     register_sky_kernel((const void *)kern);
+     TRY(set_smem(kern, smem));
+     kern<<<grid, 2 * L, smem, st>>>(y, stride, tw1, tw2, fac, N1, epi);
+     CUCHK(cudaGetLastError());
+     return TDF_OK;
+}
+
+static int launch_interp_mid(int L, dim3 grid, const double2 *y, size_t stride, const double2 *tw1, const double2 *tw2,
+                             const double *fac, int N1, const StoreFourstep<double, +1, 1> &epi, cudaStream_t st) {
+     switch (L) {
+     case 64: return launch_interp_mid_L<64>(grid, y, stride, tw1, tw2, fac, N1, epi, st);
+     case 128: return launch_interp_mid_L<128>(grid, y, stride, tw1, tw2, fac, N1, epi, st);
+     case 256: return launch_interp_mid_L<256>(grid, y, stride, tw1, tw2, fac, N1, epi, st);
+     case 512: return launch_interp_mid_L<512>(grid, y, stride, tw1, tw2, fac, N1, epi, st);
+     }
+     return set_error(TDF_ERR_UNSUPPORTED, "interpolation row length %d", L);
+}
+
 // ------------------------------------------------------------------ device buffers
 
 struct DevBuf {
@@ -352,7 +376,7 @@ struct tdf_engine {
      FFTTables<double> t_nfft, t_ninterp, t_f64;
      FFTTables<float> t_f32;
      // inputs
-     DevBuf pco, gco;
+     DevBuf fac;      // interpolation: scale and spline prefilter per bin
      // sky stage
      DevBuf skyp[2], B0, B1, B2, shft, partial, aabb[2];
      // operands
@@ -507,6 +531,9 @@ static void timing_collect(tdf_engine *e) {
 
 static size_t Wstride(const tdf_engine *e) { return (size_t)e->Ninterp; }
 
+// whether the middle of the interpolation is one kernel (k_interp_mid)
+static bool interp_fused(const tdf_engine *e) { return e->Ninterp == 2 * e->nfft && e->nfft <= (1 << 19); }
+
 // ------------------------------------------------------------------ setup
 
 static int validate(const tdf_segment *s, const tdf_search_opts *o) {
@@ -571,24 +598,18 @@ static int engine_alloc(tdf_engine *e) {
      const int nifo = e->nifo, Bs = e->Bs, Tc = e->TcMax;
      const size_t Q = (size_t)Bs * nifo;
      TRY(seg_alloc(e, e->sdv[0]));
-     // spline recurrence factors (auxi.c:102-108): invp[i] = 2/(g[i-1]+4), g[i] = -0.5 invp[i]
      {
-          const int n = e->n2N;
-          std::vector<double> p(n, 0.), g(n, 0.);
-          for (int i = 1; i < n - 1; i++) {
-               p[i] = 2. / (g[i - 1] + 4.);
-               g[i] = -.5 * p[i];
-          }
-          TRY(e->pco.alloc(n * sizeof(double)));
-          TRY(e->gco.alloc(n * sizeof(double)));
-          CUCHK(cudaMemcpy(e->pco.p, p.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-          CUCHK(cudaMemcpy(e->gco.p, g.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+          const int n = e->nfft / 2 + 1;
+          TRY(e->fac.alloc(n * sizeof(double)));
+          k_interp_factor<<<(n + 255) / 256, 256, 0, e->stream>>>(e->fac.as<double>(), n, 2. / e->Ninterp,
+                                                                  (double)e->S().seg.interpftpad / e->Ninterp);
+          CUCHK(cudaGetLastError());
      }
      for (int k = 0; k < 2; k++) TRY(e->skyp[k].alloc(Bs * sizeof(SkyParam)));
      const size_t ws = Wstride(e);
      TRY(e->B0.alloc(Q * 2 * ws * sizeof(double2)));
      TRY(e->B1.alloc(Q * 2 * ws * sizeof(double2)));
-     TRY(e->B2.alloc(Q * 2 * ws * sizeof(double2)));
+     if (!interp_fused(e)) TRY(e->B2.alloc(Q * 2 * ws * sizeof(double2)));
      TRY(e->shft.alloc(Q * e->Nal * sizeof(double)));
      TRY(e->partial.alloc(Q * (e->nfft / 256) * 2 * sizeof(double)));
      for (int k = 0; k < 2; k++) TRY(e->aabb[k].alloc(Bs * sizeof(AaBb)));
@@ -660,7 +681,7 @@ static void graphs_clear(tdf_engine *e) {
 static void engine_free(tdf_engine *e) {
      graphs_clear(e);
      for (SegData &d : e->sdv) d.release();
-     DevBuf *bufs[] = {&e->pco, &e->gco, &e->plan_sky, &e->plan_tp, &e->plan_pts, &e->skyp[0],
+     DevBuf *bufs[] = {&e->fac, &e->plan_sky, &e->plan_tp, &e->plan_pts, &e->skyp[0],
                        &e->skyp[1], &e->B0, &e->B1, &e->B2, &e->shft, &e->partial, &e->aabb[0], &e->aabb[1],
                        &e->xab[0], &e->xab[1], &e->s2[0], &e->s2[1], &e->xa64[0], &e->xa64[1], &e->xb64[0],
                        &e->xb64[1], &e->t1[0], &e->t1[1], &e->tparam, &e->trig[0], &e->trig[1],
@@ -819,44 +840,45 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
           e->B0.as<double2>(), ws, e->shft.as<double>(), split ? nullptr : e->t1[sl].as<double>(),
           e->partial.as<double>());
      CUCHK(cudaGetLastError());
-     k_sky_sums<<<npts, 256, 0, st>>>(e->partial.as<double>(), nblk, e->S().detp.as<DetParam>(), nifo,
-                                       e->aabb[sl].as<AaBb>());
-     CUCHK(cudaGetLastError());
-     e->launches += 2;
-     // forward FFT (nfft) of every (point, detector, a|b): B0 -> B1 -> B2
+     e->launches++;
+     // Interpolation: forward FFT (nfft) of every (point, detector, a|b),
+     // inverse FFT (Ninterp) of the spread spectrum times fac, which leaves the
+     // spline coefficients of the interpolated series (the first
+     // interpftpad*N + 2 and the last are kept)
+     const DevBuf *coef;
+     const FFTTables<double> &t = e->t_nfft, &ti = e->t_ninterp;
      {
-          const FFTTables<double> &t = e->t_nfft;
           LoadNatural<double> pro{e->B0.as<double2>(), t.N2, (int)ws};
           StoreFourstep<double, -1, 1> epi{e->B1.as<double2>(), t.h(), t.o(), t.N2, (int)ws};
           TRY((launch_col<double, -1, 1>(t.N1, dim3(t.N2 / LINES, 2 * Q), pro, epi, t.l1(), st)));
+     }
+     if (interp_fused(e)) {
+          // B0 -> B1 -> B0 -> B1
+          StoreFourstep<double, +1, 1> epi{e->B0.as<double2>(), ti.h(), ti.o(), ti.N2, (int)ws};
+          TRY(launch_interp_mid(t.N2, dim3(t.N1 / LINES, 2 * Q), e->B1.as<double2>(), ws, t.l2(), ti.l1(),
+                                e->fac.as<double>(), t.N1, epi, st));
+          RowsY<double, 1> src{e->B0.as<double2>(), (int)ws, ti.N2};
+          StoreNatural<double> epi2{e->B1.as<double2>(), ti.N1, (int)ws, e->n2N + 2, e->Ninterp - 1};
+          TRY((launch_row<double, +1, 1>(ti.N2, dim3(ti.N1 / LINES, 2 * Q), src, epi2, ti.l2(), st)));
+          coef = &e->B1;
+          e->launches += 3;
+     } else {
+          // B0 -> B1 -> B2 -> B1 -> B0
           RowsY<double, 1> src{e->B1.as<double2>(), (int)ws, t.N2};
-          StoreNatural<double> epi2{e->B2.as<double2>(), t.N1, (int)ws, e->nfft, 1.0};
+          StoreNatural<double> epi2{e->B2.as<double2>(), t.N1, (int)ws, e->nfft, -1};
           TRY((launch_row<double, -1, 1>(t.N2, dim3(t.N1 / LINES, 2 * Q), src, epi2, t.l2(), st)));
+          LoadShuffled<double> pro{e->B2.as<double2>(), e->fac.as<double>(), ti.N2, (int)ws, e->nfft, e->Ninterp};
+          StoreFourstep<double, +1, 1> epi{e->B1.as<double2>(), ti.h(), ti.o(), ti.N2, (int)ws};
+          TRY((launch_col<double, +1, 1>(ti.N1, dim3(ti.N2 / LINES, 2 * Q), pro, epi, ti.l1(), st)));
+          RowsY<double, 1> src2{e->B1.as<double2>(), (int)ws, ti.N2};
+          StoreNatural<double> epi3{e->B0.as<double2>(), ti.N1, (int)ws, e->n2N + 2, e->Ninterp - 1};
+          TRY((launch_row<double, +1, 1>(ti.N2, dim3(ti.N1 / LINES, 2 * Q), src2, epi3, ti.l2(), st)));
+          coef = &e->B0;
+          e->launches += 4;
      }
-     // inverse FFT (Ninterp) of the spread spectrum, scaled by interpftpad/Ninterp:
-     // B2 -> B1 -> B0 (first interpftpad*N samples kept)
-     {
-          const FFTTables<double> &t = e->t_ninterp;
-          LoadShuffled<double> pro{e->B2.as<double2>(), t.N2, (int)ws, e->nfft, e->Ninterp};
-          StoreFourstep<double, +1, 1> epi{e->B1.as<double2>(), t.h(), t.o(), t.N2, (int)ws};
-          TRY((launch_col<double, +1, 1>(t.N1, dim3(t.N2 / LINES, 2 * Q), pro, epi, t.l1(), st)));
-          RowsY<double, 1> src{e->B1.as<double2>(), (int)ws, t.N2};
-          const double ft = (double)e->S().seg.interpftpad / e->Ninterp;
-          StoreNatural<double> epi2{e->B0.as<double2>(), t.N1, (int)ws, e->n2N, ft};
-          TRY((launch_row<double, +1, 1>(t.N2, dim3(t.N1 / LINES, 2 * Q), src, epi2, t.l2(), st)));
-     }
-     e->launches += 4;
-     // spline: B0 (samples) -> B1 (u) -> B2 (second derivatives)
-     {
-          dim3 g((e->n2N + SPL_TILE - 1) / SPL_TILE, 2 * Q);
-          k_spline_fwd<<<g, SPL_T, 0, st>>>(e->B0.as<double2>(), e->B1.as<double2>(), ws, e->pco.as<double>(), e->n2N);
-          CUCHK(cudaGetLastError());
-          k_spline_bwd<<<g, SPL_T, 0, st>>>(e->B1.as<double2>(), e->B2.as<double2>(), ws, e->gco.as<double>(), e->n2N);
-          CUCHK(cudaGetLastError());
-     }
-     const SplintIn in{e->B0.as<double2>(), e->B2.as<double2>(), ws, e->shft.as<double>(), dsky,
-                       e->S().detssb.as<double>(), e->S().detp.as<DetParam>(), e->Nal, e->N, e->n2N,
-                       e->S().seg.interpftpad, nifo};
+     const SplintIn in{coef->as<double2>(), ws, e->shft.as<double>(), dsky, e->S().detssb.as<double>(),
+                       e->S().detp.as<DetParam>(), e->Nal, e->N, e->n2N, e->Ninterp, e->S().seg.interpftpad, nifo,
+                       e->partial.as<double>(), nblk, e->aabb[sl].as<AaBb>()};
      if (split) {
           const int N2 = e->t_f32.N2;
           k_splint_split<<<dim3(N2 / 32, ((e->N + N2 - 1) / N2 + 7) / 8, Q), 256, 0, st>>>(
@@ -866,7 +888,7 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
                                                                 e->xb64[sl].as<double2>());
      }
      CUCHK(cudaGetLastError());
-     e->launches += 3;
+     e->launches++;
      CUCHK(cudaEventRecord(e->sky_done[sl], st));
      return TDF_OK;
 }
@@ -1155,9 +1177,6 @@ static int set_graph_priorities(const tdf_engine *e, cudaGraph_t g) {
           static std::once_flag once;
           std::call_once(once, [] {
                register_sky_kernel((const void *)k_sky_prep);
-               register_sky_kernel((const void *)k_sky_sums);
-               register_sky_kernel((const void *)k_spline_fwd);
-               register_sky_kernel((const void *)k_spline_bwd);
                register_sky_kernel((const void *)k_splint);
                register_sky_kernel((const void *)k_splint_split);
           });

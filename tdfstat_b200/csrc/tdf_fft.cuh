@@ -206,34 +206,39 @@ __device__ __forceinline__ void pass_load(cx<T> (&v)[8], const cx<T> *s, int t) 
 
 // Full L-point transform of NA lines that share a thread: v[a] in/out as in
 // the register convention above; s[a] = the line's shared memory; tw = line
-// twiddle table (shared).  All threads of the CTA must call it (barriers).
+// twiddle table (shared).  All threads of the CTA must call it (barriers);
+// those that hold no butterfly of the line pass active = false.
 template <typename T, int L, int SIGN, int NA>
-__device__ __forceinline__ void line_fft(cx<T> (&v)[NA][8], cx<T> *const (&s)[NA], const cx<T> *tw, int t) {
+__device__ __forceinline__ void line_fft(cx<T> (&v)[NA][8], cx<T> *const (&s)[NA], const cx<T> *tw, int t,
+                                         bool active = true) {
      using G = LineGeom<T, L>;
      int NS = 1;
 #pragma unroll
      for (int p = 0; p < G::P8; p++) {
-          if (p > 0) pass_twiddle<T, L, 8, SIGN, NA>(v, tw, t, NS);
-#pragma unroll
-          for (int a = 0; a < NA; a++) pass_dft<8, SIGN>(v[a]);
           const bool last = (p == G::P8 - 1) && (G::RL == 1);
-          if (!last) {
+          if (active) {
+               if (p > 0) pass_twiddle<T, L, 8, SIGN, NA>(v, tw, t, NS);
 #pragma unroll
-               for (int a = 0; a < NA; a++) pass_store<T, L, 8>(v[a], s[a], t, NS);
+               for (int a = 0; a < NA; a++) {
+                    pass_dft<8, SIGN>(v[a]);
+                    if (!last) pass_store<T, L, 8>(v[a], s[a], t, NS);
+               }
+          }
+          if (!last) {
                __syncthreads();
                constexpr int RN = 8;   // next pass radix (8, or the last radix)
-               if (p + 1 < G::P8) {
+               if (active) {
 #pragma unroll
-                    for (int a = 0; a < NA; a++) pass_load<T, L, RN>(v[a], s[a], t);
-               } else {
-#pragma unroll
-                    for (int a = 0; a < NA; a++) pass_load<T, L, (G::RL > 1 ? G::RL : 8)>(v[a], s[a], t);
+                    for (int a = 0; a < NA; a++) {
+                         if (p + 1 < G::P8) pass_load<T, L, RN>(v[a], s[a], t);
+                         else pass_load<T, L, (G::RL > 1 ? G::RL : 8)>(v[a], s[a], t);
+                    }
                }
                __syncthreads();
           }
           NS *= 8;
      }
-     if (G::RL > 1) {
+     if (G::RL > 1 && active) {
           constexpr int RR = G::RL > 1 ? G::RL : 2;
           pass_twiddle<T, L, RR, SIGN, NA>(v, tw, t, NS);
 #pragma unroll

@@ -5,12 +5,12 @@
 //     k_sky_prep      modvir + barycentric shift + phase modulation
 //                     (settings.c:254-294, jobcore.c:283-312), zero padding,
 //                     partial sums of aa^2, bb^2 (jobcore.c:373-391)
-//     k_sky_sums      aa, bb network sums (FLOAT_TYPE emulation per form)
-//     k_spline_fwd /
-//     k_spline_bwd    natural cubic spline second derivatives (auxi.c:93-117)
-//                     as blocked recurrences with warm-up
-//     k_splint        spline evaluation at 2(i - shftf[i]) (auxi.c:120-169),
-//                     division by sig2, conversion to the spindown operands
+//     (FFT passes)    interpolation by FFT to twice the rate, delivering the
+//                     coefficients of the cubic spline through the series
+//     k_splint(_split) natural-spline evaluation at 2(i - shftf[i])
+//                     (auxi.c:93-169), division by sig2, conversion to the
+//                     spindown operands; aa, bb network sums (FLOAT_TYPE
+//                     emulation per form)
 //   spindown stage (once per template)
 //     (split form: tdf_split.cuh)
 //     DemodFP64       column-pass prologue: spindown_modulation
@@ -212,14 +212,13 @@ __global__ void __launch_bounds__(256) k_add_signal(float *__restrict__ xdat, co
      if (*x != 0.f) *x = (float)__dadd_rn((double)*x, __dmul_rn(h0, s[(size_t)d * N + i]));
 }
 
-// one CTA per sky point: aa = sum_n sum_i aa_n^2/sig2_n (jobcore.c:373-386);
-// each detector's partials reduced by a fixed tree (reproducible), then
-// accumulated over detectors into FLOAT_TYPE as the reference build does.
-// grid (npts), 256 threads
-__global__ void __launch_bounds__(256) k_sky_sums(const double *__restrict__ partial, int nblk,
-                                                  const DetParam *__restrict__ dp, int nifo, AaBb *__restrict__ out)
+// aa = sum_n sum_i aa_n^2/sig2_n (jobcore.c:373-386) of sky point p by one CTA
+// of 256 threads; each detector's partials reduced by a fixed tree
+// (reproducible), then accumulated over detectors into FLOAT_TYPE as the
+// reference build does.
+__device__ void sky_sums(const double *__restrict__ partial, int nblk, const DetParam *__restrict__ dp, int nifo, int p,
+                         AaBb *__restrict__ out)
 {
-     const int p = blockIdx.x;
      __shared__ double ra[256], rb[256];
      double aa = 0., bb = 0.;
      float aaf = 0.f, bbf = 0.f;
@@ -253,159 +252,50 @@ __global__ void __launch_bounds__(256) k_sky_sums(const double *__restrict__ par
      }
 }
 
-// The natural-spline sweeps (auxi.c:102-115) as blocked recurrences: a
-// thread computes a chunk of SPL_K consecutive indices, started SPL_W indices
-// early from zero -- both recurrences contract by |0.5*invp| ~ 0.27 per step,
-// so the start-up error is below 1e-27 of the values after 48 steps and the
-// results are those of one sequential sweep.  A CTA of SPL_T threads stages
-// its tile of the inputs (and the warm-up margin) in shared memory with
-// per-thread asynchronous copies (all in flight at once); lane j then reads
-// index j*SPL_K + r, and one pad word per 16 elements puts the lanes of a
-// wavefront on distinct banks.  A thread keeps its SPL_K outputs in
-// registers until the whole CTA is done reading the staged inputs, writes
-// them over the tile's part of the staging buffer, and the CTA stores the
-// tile with consecutive lanes on consecutive indices.
-constexpr int SPL_T = 64;                  // threads per CTA
-constexpr int SPL_K = 16;                  // indices per thread
-constexpr int SPL_W = 48;                  // warm-up steps
-constexpr int SPL_TILE = SPL_T * SPL_K;    // indices per CTA
-__device__ __forceinline__ int spl_pad(int s) { return s + (s >> 4); }
-
-// Forward sweep (auxi.c:102-111), u[i] for i in [1, n-2] (u[0] = 0).
-// grid (ceil(n/SPL_TILE), 2*Q), SPL_T threads
-__global__ void __launch_bounds__(SPL_T) k_spline_fwd(const double2 *__restrict__ Z, double2 *__restrict__ U,
-                                                      size_t stride, const double *__restrict__ pco, int n)
-{
-     constexpr int S = SPL_TILE + SPL_W + 2;   // staged samples: [tile0 - W - 1, tile0 + TILE + 1)
-     constexpr int P = SPL_TILE + SPL_W;       // staged factors:  [tile0 - W, tile0 + TILE)
-     __shared__ __align__(16) double2 ys[S + S / 16 + 1];
-     __shared__ __align__(16) double ps[P + P / 16 + 1];
-     const int arr = blockIdx.y;
-     const double2 *y = Z + (size_t)arr * stride;
-     double2 *u = U + (size_t)arr * stride;
-     const int tile0 = blockIdx.x * SPL_TILE;
-     const int yb = tile0 - SPL_W - 1, pb = tile0 - SPL_W;
-     for (int k = threadIdx.x; k < S; k += SPL_T) {
-          const int i = yb + k;
-          if (i >= 0 && i < n) cp_async16(&ys[spl_pad(k)], &y[i]);
-     }
-     for (int k = threadIdx.x; k < P; k += SPL_T) {
-          const int i = pb + k;
-          if (i >= 0 && i < n) cp_async8(&ps[spl_pad(k)], &pco[i]);
-     }
-     cp_async_wait_all();
-     __syncthreads();
-     const int lo = tile0 + threadIdx.x * SPL_K;
-     const int hi = min(n - 1, lo + SPL_K);
-     double2 out[SPL_K];
-     if (lo < n) {
-          const int i0 = max(1, lo - SPL_W);
-          double ur = 0., ui = 0.;
-          double2 ym = ys[spl_pad(i0 - 1 - yb)], y0 = ys[spl_pad(i0 - yb)];
-          auto step = [&](int i) {
-               const double2 yp = ys[spl_pad(i + 1 - yb)];
-               const double p = ps[spl_pad(i - pb)];
-               const double dr = ym.x - 2. * y0.x + yp.x;
-               const double dI = ym.y - 2. * y0.y + yp.y;
-               ur = (-.5 * ur + 3. * dr) * p;
-               ui = (-.5 * ui + 3. * dI) * p;
-               ym = y0;
-               y0 = yp;
-          };
-          for (int i = i0; i < lo; i++) step(i);   // warm-up
-#pragma unroll
-          for (int r = 0; r < SPL_K; r++) {
-               const int i = lo + r;
-               out[r] = make_double2(0., 0.);      // u[0] = 0
-               if (i >= i0 && i < hi) {
-                    step(i);
-                    out[r] = make_double2(ur, ui);
-               }
-          }
-     }
-     __syncthreads();   // every thread is done with the staged samples
-     if (lo < n) {
-#pragma unroll
-          for (int r = 0; r < SPL_K; r++)
-               if (lo + r < hi || lo + r == 0) ys[spl_pad(lo + r - yb)] = out[r];
-     }
-     __syncthreads();
-     for (int k = threadIdx.x; k < SPL_TILE; k += SPL_T) {
-          const int i = tile0 + k;
-          if (i < n - 1) u[i] = ys[spl_pad(k + SPL_W + 1)];
-     }
+// The natural cubic spline (auxi.c:93-169) through y[0..n-1], evaluated at x
+// from B-spline coefficients: with t = x - k, k = floor(x),
+//   s(x) = sum_j w_j(t) c[k + j], j = -1..2 (the four cubic B-spline weights).
+// c0 holds the coefficients of the periodic spline of the whole interpolated
+// series (period np, a power of two), which the inverse FFT delivers; its
+// second derivatives at the ends of the data, D0 and Dn, are not zero.  The
+// natural spline has c[k] = c0[k] + a z^k + b z^(n-1-k), z = sqrt(3) - 2: both
+// added terms leave every y[k] as it is (z + 4 + 1/z = 0) and change the
+// second derivative by -6 times themselves, so
+//   a + b z^(n-1) = D0/6,  a z^(n-1) + b = Dn/6.
+// They decay by 0.27 per sample and are left out 64 samples from the ends
+// (1e-37).  Replaces two recurrence sweeps over every series (u, y2): half of
+// the sky stage's passes over memory.
+__device__ __forceinline__ double zpow(int e) {
+     constexpr double z = -0.26794919243112270647, iz = -3.7320508075688772935;
+     if (e > 128) return 0.;   // below 1e-73
+     double p = 1.;
+     for (int i = 0; i < e; i++) p *= z;
+     for (int i = 0; i > e; i--) p *= iz;
+     return p;
 }
 
-// Back substitution (auxi.c:112-115): y2[n-1] = 0, y2[k] = g[k]*y2[k+1] + u[k];
-// a thread's chunk is started SPL_W indices late from y2 = 0.
-// grid (ceil(n/SPL_TILE), 2*Q), SPL_T threads
-__global__ void __launch_bounds__(SPL_T) k_spline_bwd(const double2 *__restrict__ U, double2 *__restrict__ Y2,
-                                                      size_t stride, const double *__restrict__ gco, int n)
-{
-     constexpr int S = SPL_TILE + SPL_W;       // staged: [tile0, tile0 + TILE + W)
-     __shared__ __align__(16) double2 us[S + S / 16 + 1];
-     __shared__ __align__(16) double gs[S + S / 16 + 1];
-     const int arr = blockIdx.y;
-     const double2 *u = U + (size_t)arr * stride;
-     double2 *y2 = Y2 + (size_t)arr * stride;
-     const int tile0 = blockIdx.x * SPL_TILE;
-     for (int k = threadIdx.x; k < S; k += SPL_T) {
-          const int i = tile0 + k;
-          if (i < n) {
-               cp_async16(&us[spl_pad(k)], &u[i]);
-               cp_async8(&gs[spl_pad(k)], &gco[i]);
-          }
-     }
-     cp_async_wait_all();
-     __syncthreads();
-     const int lo = tile0 + threadIdx.x * SPL_K;
-     const int hi = min(n, lo + SPL_K);
-     double2 out[SPL_K];
-     if (lo < n) {
-          const int ks = min(n - 1, hi + SPL_W);
-          double yr = 0., yi = 0.;
-          auto step = [&](int k) {
-               const double g = gs[spl_pad(k - tile0)];
-               const double2 uk = us[spl_pad(k - tile0)];
-               yr = g * yr + uk.x;
-               yi = g * yi + uk.y;
-          };
-          for (int k = ks - 1; k >= hi; k--) step(k);   // warm-up
-#pragma unroll
-          for (int r = SPL_K - 1; r >= 0; r--) {
-               const int k = lo + r;
-               out[r] = make_double2(0., 0.);      // y2[n-1] = 0
-               if (k < hi && k < ks) {
-                    step(k);
-                    out[r] = make_double2(yr, yi);
-               }
-          }
-     }
-     __syncthreads();   // every thread is done with the staged inputs
-     if (lo < n) {
-#pragma unroll
-          for (int r = 0; r < SPL_K; r++)
-               if (lo + r < hi) us[spl_pad(lo + r - tile0)] = out[r];
-     }
-     __syncthreads();
-     for (int k = threadIdx.x; k < SPL_TILE; k += SPL_T) {
-          const int i = tile0 + k;
-          if (i < n) y2[i] = us[spl_pad(k)];
-     }
-}
-
-__device__ __forceinline__ double2 splint_eval(const double2 *__restrict__ ya, const double2 *__restrict__ y2a, int n, double x)
+__device__ __forceinline__ double2 splint_eval(const double2 *__restrict__ c0, int n, int np, double x)
 {
      if (x < 0 || x > n - 1) return make_double2(0., 0.);
-     const int klo = (int)floor(x);
-     const int khi = klo + 1;
-     const double a = khi - x, b = x - klo;
-     const double2 yl = ya[klo], sl = y2a[klo];
-     const double2 yh = khi < n ? ya[khi] : make_double2(0., 0.);
-     const double2 sh = khi < n ? y2a[khi] : make_double2(0., 0.);
-     const double ca = a * a * a - a, cb = b * b * b - b;
-     return make_double2(a * yl.x + b * yh.x + (ca * sl.x + cb * sh.x) / 6.0,
-                         a * yl.y + b * yh.y + (ca * sl.y + cb * sh.y) / 6.0);
+     const int k = (int)floor(x);
+     const double t = x - k, u = 1. - t;
+     const double2 cm = c0[(k - 1) & (np - 1)], ca = c0[k], cb = c0[(k + 1) & (np - 1)], cd = c0[(k + 2) & (np - 1)];
+     const double wm = u * u * u * (1. / 6.), wd = t * t * t * (1. / 6.);
+     const double wa = (2. / 3.) - t * t * (1. - .5 * t), wb = (2. / 3.) - u * u * (1. - .5 * u);
+     double2 r = make_double2(wm * cm.x + wa * ca.x + wb * cb.x + wd * cd.x, wm * cm.y + wa * ca.y + wb * cb.y + wd * cd.y);
+     if (k < 64 || k > n - 66) {
+          constexpr double z = -0.26794919243112270647;
+          const double2 l0 = c0[np - 1], l1 = c0[0], l2 = c0[1 & (np - 1)];
+          const double2 r0 = c0[(n - 2) & (np - 1)], r1 = c0[n - 1], r2 = c0[n & (np - 1)];
+          const double2 D0 = make_double2((l0.x - 2. * l1.x + l2.x) / 6., (l0.y - 2. * l1.y + l2.y) / 6.);
+          const double2 Dn = make_double2((r0.x - 2. * r1.x + r2.x) / 6., (r0.y - 2. * r1.y + r2.y) / 6.);
+          const double w = zpow(n - 1), q = 1. / (1. - w * w);
+          const double ga = zpow(k - 1) * (wm + z * (wa + z * (wb + z * wd))) * q;               // of a
+          const double gb = zpow(n - 3 - k) * (wd + z * (wb + z * (wa + z * wm))) * q;           // of b
+          r.x += ga * (D0.x - w * Dn.x) + gb * (Dn.x - w * D0.x);
+          r.y += ga * (D0.y - w * Dn.y) + gb * (Dn.y - w * D0.y);
+     }
+     return r;
 }
 
 // shft_n[0] as k_sky_prep forms shft_n[i]
@@ -413,24 +303,28 @@ __device__ __forceinline__ double shft0(const SkyParam &S, const double *e) {
      return __dadd_rn(__dadd_rn(__dmul_rn(S.nS0, e[0]), __dmul_rn(S.nS1, e[1])), __dmul_rn(S.nS2, e[2]));
 }
 
-// The inputs of the resampling (jobcore.c:314-370): samples Z and second
-// derivatives Y2 of array (q, a|b), q = point*nifo + det, `stride` apart.
+// The inputs of the resampling (jobcore.c:314-370): spline coefficients C of
+// array (q, a|b), q = point*nifo + det, `stride` apart; and the sums' partials
+// (the CTA of a point's first tile forms its aa and bb).
 struct SplintIn {
-     const double2 *Z, *Y2;
+     const double2 *C;
      size_t stride;
      const double *shft;      // [q][Nal]
      const SkyParam *sp;
      const double *detssb;
      const DetParam *dp;
-     int Nal, N, n, interpftpad, nifo;
+     int Nal, N, n, np, interpftpad, nifo;
+     const double *partial;
+     int nblk;
+     AaBb *ab;
 };
 
 // xDatm{a,b}[i] = splint(interpftpad*(i - (shft[i] - shft[0])))/sig2
 __device__ __forceinline__ void splint_at(const SplintIn &I, int q, int i, double sh, double sh1, double s2, double2 &a,
                                           double2 &b) {
      const double x = I.interpftpad * (i - __dsub_rn(sh, sh1));
-     const double2 va = splint_eval(I.Z + ((size_t)q * 2) * I.stride, I.Y2 + ((size_t)q * 2) * I.stride, I.n, x);
-     const double2 vb = splint_eval(I.Z + ((size_t)q * 2 + 1) * I.stride, I.Y2 + ((size_t)q * 2 + 1) * I.stride, I.n, x);
+     const double2 va = splint_eval(I.C + ((size_t)q * 2) * I.stride, I.n, I.np, x);
+     const double2 vb = splint_eval(I.C + ((size_t)q * 2 + 1) * I.stride, I.n, I.np, x);
      a = make_double2(va.x / s2, va.y / s2);
      b = make_double2(vb.x / s2, vb.y / s2);
 }
@@ -441,6 +335,7 @@ __global__ void __launch_bounds__(256) k_splint(const __grid_constant__ SplintIn
 {
      const int q = blockIdx.y, d = q % I.nifo;
      const int i = blockIdx.x * 256 + threadIdx.x;
+     if (blockIdx.x == 0 && d == 0) sky_sums(I.partial, I.nblk, I.dp, I.nifo, q / I.nifo, I.ab);
      if (i >= I.N) return;
      double2 a, b;
      splint_at(I, q, i, I.shft[(size_t)q * I.Nal + i], shft0(I.sp[q / I.nifo], I.detssb + (size_t)d * 3 * I.N),
@@ -463,6 +358,7 @@ __global__ void __launch_bounds__(256) k_splint_split(const __grid_constant__ Sp
      __shared__ float4 xs[32][9];
      __shared__ float ss[32][9];
      const int q = blockIdx.z, p = q / I.nifo, d = q % I.nifo;
+     if (blockIdx.x == 0 && blockIdx.y == 0 && d == 0) sky_sums(I.partial, I.nblk, I.dp, I.nifo, p, I.ab);
      {
           const int c = threadIdx.x % 32, r = threadIdx.x / 32;
           const int i = N2 * (blockIdx.y * 8 + r) + blockIdx.x * 32 + c;

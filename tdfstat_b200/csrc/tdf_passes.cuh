@@ -28,16 +28,17 @@ constexpr size_t pass_smem_bytes() {
      return sizeof(cx<T>) * (L + (size_t)NA * LINES * LineGeom<T, L>::STRIDE);
 }
 
-// resident CTAs per SM the FP32 passes are compiled for (register cap):
-// column passes, and row passes (which hold no demodulation operands and fit
-// 64 registers at L <= 256 without spilling)
-template <typename T, int L>
+// resident CTAs per SM the passes are compiled for (register cap): FP32
+// column passes and row passes; FP64 passes at 64 registers with one array
+// (the sky stage; two CTAs of 512 threads fit the shared memory) and 128 with
+// two
+template <typename T, int L, int NA>
 constexpr int pass_min_blocks() {
-     return sizeof(T) == 4 ? (L <= 256 ? 3 : (L == 512 ? 2 : 1)) : 1;
+     return sizeof(T) == 4 ? (L <= 256 ? 3 : (L == 512 ? 2 : 1)) : (1024 / NA / L > 1 ? 1024 / NA / L : 1);
 }
-template <typename T, int L>
+template <typename T, int L, int NA>
 constexpr int row_min_blocks() {
-     return sizeof(T) == 4 ? (L <= 256 ? 4 : (L == 512 ? 2 : 1)) : 1;
+     return sizeof(T) == 4 ? (L <= 256 ? 4 : (L == 512 ? 2 : 1)) : (1024 / NA / L > 1 ? 1024 / NA / L : 1);
 }
 
 // An epilogue with `static constexpr bool kTables = true` keeps tables in
@@ -111,14 +112,14 @@ __device__ __forceinline__ void row_body(const Src &src, const Epi &epi, const c
 }
 
 template <typename T, int L, int SIGN, int NA, class Pro, class Epi>
-__global__ void __launch_bounds__(pass_threads<L>(), (pass_min_blocks<T, L>()))
+__global__ void __launch_bounds__(pass_threads<L>(), (pass_min_blocks<T, L, NA>()))
 k_colpass(const __grid_constant__ Pro pro, Epi epi, const cx<T> *__restrict__ twline) {
      extern __shared__ __align__(128) unsigned char smem_raw[];
      col_body<T, L, SIGN, NA>(pro, epi, twline, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 template <typename T, int L, int SIGN, int NA, class Src, class Epi>
-__global__ void __launch_bounds__(pass_threads<L>(), (row_min_blocks<T, L>())) k_rowpass(Src src, Epi epi, const cx<T> *__restrict__ twline) {
+__global__ void __launch_bounds__(pass_threads<L>(), (row_min_blocks<T, L, NA>())) k_rowpass(Src src, Epi epi, const cx<T> *__restrict__ twline) {
      extern __shared__ __align__(128) unsigned char smem_raw[];
      row_body<T, L, SIGN, NA>(src, epi, twline, blockIdx.x, blockIdx.y, smem_raw);
 }
@@ -270,21 +271,21 @@ struct RowsYBulk {
      }
 };
 
-// Row-pass epilogue: natural-order output X[k1 + N1*k2] * scale for k < nkeep.
+// Row-pass epilogue: natural-order output X[k1 + N1*k2] for k < nkeep and
+// k = klast.
 template <typename T>
 struct StoreNatural {
      cx<T> *x;
      int N1;
      int N;          // array stride
-     int nkeep;
-     T scale;
+     int nkeep, klast;
      template <int L>
      __device__ __forceinline__ void store(const cx<T> (&v)[1][8], int b, int k1, int t) const {
           cx<T> *dst = x + (size_t)b * N;
 #pragma unroll
           for (int m = 0; m < 8; m++) {
                int k = k1 + N1 * (t + m * (L / 8));
-               if (k < nkeep) dst[k] = cscale(v[0][m], scale);
+               if (k < nkeep || k == klast) dst[k] = v[0][m];
           }
      }
 };
@@ -306,10 +307,12 @@ struct LoadNatural {
 
 // Column-pass prologue of the interpolation inverse FFT: the spectrum of
 // length nfft is spread to Ninterp = ratio*nfft, moving bins [nyqst, nfft)
-// to the top and zeroing the middle (jobcore.c:336-350).
+// to the top and zeroing the middle (jobcore.c:336-350), and multiplied by
+// fac (k_interp_factor).
 template <typename T>
 struct LoadShuffled {
      const cx<T> *x;  // forward spectra (nfft values each), arrays `stride` apart
+     const T *fac;
      int N2;          // of the Ninterp transform
      int stride;
      int nfft;
@@ -325,11 +328,83 @@ struct LoadShuffled {
                cx<T> z;
                z.x = 0;
                z.y = 0;
-               if (k < nyqst) z = src[k];
-               else if (k >= nyqst + gap) z = src[k - gap];
+               if (k < nyqst) z = cscale(src[k], fac[k]);
+               else if (k >= nyqst + gap) z = cscale(src[k - gap], fac[Ninterp - k]);
                v[0][m] = z;
           }
      }
 };
+
+// fac[k] = scale * 6/(4 + 2 cos(2 pi k/Ninterp)), k <= nfft/2: the scale of
+// the inverse interpolation FFT and the frequency response of the cubic
+// B-spline prefilter, so that the transform yields the spline coefficients c
+// of the interpolated series y, y[k] = (c[k-1] + 4 c[k] + c[k+1])/6 (periodic;
+// the natural end conditions are put in by splint_eval).
+__global__ void k_interp_factor(double *fac, int n, double dw, double scale) {
+     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+     if (k < n) fac[k] = scale * 6. / (4. + 2. * cospi(dw * k));
+}
+
+// The middle of the interpolation (FP64) when Ninterp = 2 nfft: the rows of
+// the forward transform and the columns of the inverse one in one kernel.
+// With nfft = N1*L (rows of L points) the inverse transform has N1 columns of
+// 2L points, and the outputs X[k1 + N1*k2] of forward row k1 are exactly the
+// inputs of inverse column k1: the spectrum never goes to memory (one kernel
+// and one write and read of every spectrum less).  Half of an inverse
+// column's inputs are the zero padding.
+// CTA: LINES rows k1, 2L threads; the forward rows use half of them.
+// grid (N1/LINES, arrays)
+template <int L>
+struct InterpMid {
+     static constexpr size_t line_bytes = sizeof(double2) * LINES * (size_t)LineGeom<double, 2 * L>::STRIDE;
+     static constexpr size_t tab_off = sizeof(double2) * 3 * L + line_bytes;   // four-step tables of the epilogue
+};
+
+template <int L>
+__global__ void __launch_bounds__(2 * L, 512 / L)
+k_interp_mid(const double2 *__restrict__ y, size_t stride, const double2 *__restrict__ tw1,
+             const double2 *__restrict__ tw2, const double *__restrict__ fac, int N1,
+             StoreFourstep<double, +1, 1> epi) {
+     extern __shared__ __align__(128) unsigned char smem_raw[];
+     double2 *t1 = reinterpret_cast<double2 *>(smem_raw), *t2 = t1 + L, *lines = t2 + 2 * L;
+     const int c = threadIdx.x % LINES, t = threadIdx.x / LINES;
+     const int k1 = blockIdx.x * LINES + c;
+     const bool fwd = t < L / 8;
+     double2 v[1][8];
+     if (fwd) {
+          const double2 *r = y + (size_t)blockIdx.y * stride + (size_t)k1 * L + t;
+#pragma unroll
+          for (int m = 0; m < 8; m++) v[0][m] = r[m * (L / 8)];
+     }
+     load_table<double>(t1, tw1, L);
+     load_table<double>(t2, tw2, 2 * L);
+     epi.template load_tables<2 * L>(smem_raw);
+     double2 *s[1] = {lines + c * LineGeom<double, 2 * L>::STRIDE};
+     __syncthreads();
+     line_fft<double, L, -1, 1>(v, s, t1, t, fwd);
+     if (fwd) {
+          const int nfft = N1 * L;
+#pragma unroll
+          for (int m = 0; m < 8; m++) {
+               const int k2 = t + m * (L / 8), k = k1 + N1 * k2;
+               s[0][pad8(k2)] = cscale(v[0][m], __ldg(&fac[k <= nfft / 2 ? k : nfft - k]));
+          }
+     }
+     __syncthreads();
+     // input n1 = t + m L/4 of the inverse column: bins k2 = n1 below nfft/2,
+     // k2 = n1 - L in the top quarter; bin nfft/2 itself (row 0) on the low side
+#pragma unroll
+     for (int m = 0; m < 8; m++) {
+          const int n1 = t + m * (L / 4);
+          v[0][m] = m < 2 ? s[0][pad8(n1)] : (m >= 6 ? s[0][pad8(n1 - L)] : make_double2(0., 0.));
+     }
+     if (k1 == 0 && t == 0) {
+          v[0][2] = v[0][6];
+          v[0][6] = make_double2(0., 0.);
+     }
+     __syncthreads();
+     line_fft<double, 2 * L, +1, 1>(v, s, t2, t);
+     epi.template store<2 * L>(v, blockIdx.y, k1, t, smem_raw);
+}
 
 }  // namespace tdf
