@@ -367,7 +367,10 @@ struct tdf_engine {
      int N = 0, nfft = 0, nfftf = 0, Ninterp = 0, nifo = 0, Nal = 0, n2N = 0;
      int nF = 0, nblk_mu = 0;
      int CL = 0;        // split form: entries of an operand column (ceil(N/N2), up to a multiple of 32)
-     int Bs = 8;        // sky points per batch
+     // sky points per batch: 8, and more for short segments (2^16 points 16,
+     // 2^15 and less 24), whose sky stage otherwise leaves most of the GPU idle:
+     // 48 points x 33 spindowns of 2^14 points 934 us with 8, 839 with 24
+     int Bs = 8;
      int Tc = 96;       // templates per chunk
      int TcMax = 96;    // buffers are sized for chunks up to this size
      int Gt = 64;       // templates per resolve group at most (whole chunks; TDF_GROUP_TEMPLATES)
@@ -388,7 +391,7 @@ struct tdf_engine {
           DevBuf Ybuf;    // four-step intermediate of a chunk
           DevBuf Fbuf;    // F ring of a resolve group
           DevBuf mubuf;   // blocks_avg means of a resolve group
-          DevBuf tcnt;    // per-template trigger counts + candidate count
+          unsigned *tcnt = nullptr;   // per-template trigger counts + candidate count (in `zeroed`)
           DevBuf cand;    // candidate bins of a resolve group (uint2), or the sparse store's records (uint4)
           DevBuf Ebuf;    // sparse F store: edge ring of a resolve group (split form)
           DevBuf ctl;     // fused pass order: tickets, finished CTAs, column blocks done per template
@@ -403,12 +406,22 @@ struct tdf_engine {
      unsigned cand_cap = 0;
      // two batch slots: while the host drains one slot's triggers the
      // device runs the other slot's batch
-     DevBuf trig[2], counters[2];
+     DevBuf trig[2];
+     // everything a search starts from at zero, cleared by one memset: per
+     // slot {trigger count, error flags}, then the lanes' tcnt
+     DevBuf zeroed;
+     unsigned long long *counters(int slot) const { return zeroed.as<unsigned long long>() + 2 * slot; }
      unsigned long long trig_cap = 0;
      SkyParam *h_sky[2] = {nullptr, nullptr};     // pinned staging per slot
      TmplParam *h_tp[2] = {nullptr, nullptr};
      size_t h_tp_cap = 0;
      unsigned long long *h_cnt = nullptr;         // pinned [slot][count, error flags]
+     // pinned: the first kTrigAhead triggers of a slot's batch come back with
+     // its counts; an F spectrum on its way to the caller
+     static constexpr size_t kTrigAhead = 1024;
+     Trig *h_trig0[2] = {nullptr, nullptr};
+     void *h_F = nullptr;
+     void *pinned = nullptr;                      // h_sky, h_cnt, h_trig0 and h_F lie in it
      cudaEvent_t done[2] = {nullptr, nullptr};
      int cur = 0;                                 // slot the kernels write to
      std::vector<Trig> h_trig;
@@ -594,6 +607,21 @@ static int seg_alloc(const tdf_engine *e, SegData &d) {
      return TDF_OK;
 }
 
+static int ensure_tparam(tdf_engine *e, size_t n) {
+     if (n > e->h_tp_cap) {
+          CUCHK(cudaStreamSynchronize(e->stream));
+          size_t cap = std::max<size_t>(n, 4096);
+          for (int s = 0; s < 2; s++) {
+               if (e->h_tp[s]) cudaFreeHost(e->h_tp[s]);
+               e->h_tp[s] = nullptr;
+               CUCHK(cudaMallocHost((void **)&e->h_tp[s], cap * sizeof(TmplParam)));
+          }
+          e->h_tp_cap = cap;
+          TRY(e->tparam.alloc(cap * sizeof(TmplParam)));
+     }
+     return TDF_OK;
+}
+
 static int engine_alloc(tdf_engine *e) {
      const int nifo = e->nifo, Bs = e->Bs, Tc = e->TcMax;
      const size_t Q = (size_t)Bs * nifo;
@@ -638,13 +666,14 @@ static int engine_alloc(tdf_engine *e) {
      const size_t rsz = e->form == TDF_FORM_SPLIT ? sizeof(float) : sizeof(double);
      const size_t G = (size_t)std::max(tdf_engine::kGtMax, Tc);   // templates per resolve group at most
      e->cand_cap = (unsigned)G * 4096u;
+     TRY(e->zeroed.alloc(4 * sizeof(unsigned long long) + e->lanes_alloc * (G + 1) * sizeof(unsigned)));
+     CUCHK(cudaMemset(e->zeroed.p, 0, e->zeroed.bytes));
      for (int l = 0; l < e->lanes_alloc; l++) {   // every lane the autotuner may use
           tdf_engine::Lane &L = e->ln[l];
           TRY(L.Ybuf.alloc((size_t)Tc * 2 * e->nfftf * csz));
           TRY(L.Fbuf.alloc(G * e->nF * rsz));
           TRY(L.mubuf.alloc(G * std::max(1, e->nblk_mu) * rsz));
-          TRY(L.tcnt.alloc((G + 1) * sizeof(unsigned)));
-          CUCHK(cudaMemset(L.tcnt.p, 0, L.tcnt.bytes));
+          L.tcnt = reinterpret_cast<unsigned *>(e->counters(2)) + l * (G + 1);
           TRY(L.cand.alloc(e->cand_cap * sizeof(uint4)));
           // edge ring: 2 floats per (template, row CTA, k2)
           if (e->form == TDF_FORM_SPLIT) TRY(L.Ebuf.alloc(G * (size_t)e->nfftf / RUN * 2 * sizeof(float)));
@@ -656,13 +685,21 @@ static int engine_alloc(tdf_engine *e) {
           CUCHK(cudaMemcpy(e->linesd.p, e->lines.data(), e->lines.size() * sizeof(double), cudaMemcpyHostToDevice));
      e->trig_cap = 1ull << 21;
      for (int s = 0; s < 2; s++) {
-          TRY(e->counters[s].alloc(2 * sizeof(unsigned long long)));
-          CUCHK(cudaMemset(e->counters[s].p, 0, 2 * sizeof(unsigned long long)));
           TRY(e->trig[s].alloc(e->trig_cap * sizeof(Trig)));
-          CUCHK(cudaMallocHost((void **)&e->h_sky[s], Bs * sizeof(SkyParam)));
           CUCHK(cudaEventCreateWithFlags(&e->done[s], cudaEventDisableTiming));
      }
-     CUCHK(cudaMallocHost((void **)&e->h_cnt, 4 * sizeof(unsigned long long)));
+     {
+          const size_t cnt = 4 * sizeof(unsigned long long), tr = tdf_engine::kTrigAhead * sizeof(Trig),
+                       sky = Bs * sizeof(SkyParam);
+          CUCHK(cudaMallocHost(&e->pinned, cnt + 2 * (tr + sky) + e->nF * rsz));
+          unsigned char *q = static_cast<unsigned char *>(e->pinned);
+          e->h_cnt = reinterpret_cast<unsigned long long *>(q);
+          q += cnt;
+          for (int s = 0; s < 2; s++, q += tr) e->h_trig0[s] = reinterpret_cast<Trig *>(q);
+          for (int s = 0; s < 2; s++, q += sky) e->h_sky[s] = reinterpret_cast<SkyParam *>(q);
+          e->h_F = q;
+     }
+     TRY(ensure_tparam(e, 1));
      TRY(e->t_nfft.build(e->nfft));
      TRY(e->t_ninterp.build(e->Ninterp));
      if (e->form == TDF_FORM_FP64) TRY(e->t_f64.build(e->nfftf));
@@ -685,13 +722,12 @@ static void engine_free(tdf_engine *e) {
                        &e->skyp[1], &e->B0, &e->B1, &e->B2, &e->shft, &e->partial, &e->aabb[0], &e->aabb[1],
                        &e->xab[0], &e->xab[1], &e->s2[0], &e->s2[1], &e->xa64[0], &e->xa64[1], &e->xb64[0],
                        &e->xb64[1], &e->t1[0], &e->t1[1], &e->tparam, &e->trig[0], &e->trig[1],
-                       &e->counters[0], &e->counters[1], &e->linesd};
+                       &e->zeroed, &e->linesd};
      for (DevBuf *b : bufs) b->release();
      for (tdf_engine::Lane &L : e->ln) {
           L.Ybuf.release();
           L.Fbuf.release();
           L.mubuf.release();
-          L.tcnt.release();
           L.cand.release();
           L.Ebuf.release();
      }
@@ -700,15 +736,17 @@ static void engine_free(tdf_engine *e) {
      e->t_f32.release();
      e->t_f64.release();
      for (int s = 0; s < 2; s++) {
-          if (e->h_sky[s]) cudaFreeHost(e->h_sky[s]);
           if (e->h_tp[s]) cudaFreeHost(e->h_tp[s]);
           if (e->done[s]) cudaEventDestroy(e->done[s]);
           e->h_sky[s] = nullptr;
+          e->h_trig0[s] = nullptr;
           e->h_tp[s] = nullptr;
           e->done[s] = nullptr;
      }
-     if (e->h_cnt) cudaFreeHost(e->h_cnt);
+     if (e->pinned) cudaFreeHost(e->pinned);
+     e->pinned = nullptr;
      e->h_cnt = nullptr;
+     e->h_F = nullptr;
      for (cudaEvent_t ev : e->evpool) cudaEventDestroy(ev);
      e->evpool.clear();
      e->evfree.clear();
@@ -1028,8 +1066,8 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
      const int boff = ci * e->Tc;
      const TmplParam *ctp = dtp + boff;
      const unsigned G = (unsigned)group_templates(e);
-     unsigned *tcnt = Ln.tcnt.as<unsigned>();
-     unsigned *errw = reinterpret_cast<unsigned *>(e->counters[e->cur].as<unsigned long long>() + 1);
+     unsigned *tcnt = Ln.tcnt;
+     unsigned *errw = reinterpret_cast<unsigned *>(e->counters(e->cur) + 1);
      const bool blocks = e->opts.blocks_avg && e->nblk_mu > 0;
      size_t tev = e->timing ? timing_begin(e, st) : (size_t)-1;
      if constexpr (std::is_same<T, float>::value) {
@@ -1095,9 +1133,9 @@ static int run_resolve(tdf_engine *e, int l, const TmplParam *dtp, int ntg) {
      tdf_engine::Lane &Ln = e->ln[l];
      const bool split = std::is_same<T, float>::value;
      const unsigned G = (unsigned)group_templates(e);
-     unsigned *tcnt = Ln.tcnt.as<unsigned>();
+     unsigned *tcnt = Ln.tcnt;
      const bool blocks = e->opts.blocks_avg && e->nblk_mu > 0;
-     unsigned long long *cnt = e->counters[e->cur].as<unsigned long long>();
+     unsigned long long *cnt = e->counters(e->cur);
      ThrArgs A;
      A.nF = e->nF;
      A.fr0 = e->opts.fr[0];
@@ -1263,21 +1301,6 @@ static int run_templates_batch(tdf_engine *e, int nt) {
      return TDF_OK;
 }
 
-static int ensure_tparam(tdf_engine *e, size_t n) {
-     if (n > e->h_tp_cap) {
-          CUCHK(cudaStreamSynchronize(e->stream));
-          size_t cap = std::max<size_t>(n, 4096);
-          for (int s = 0; s < 2; s++) {
-               if (e->h_tp[s]) cudaFreeHost(e->h_tp[s]);
-               e->h_tp[s] = nullptr;
-               CUCHK(cudaMallocHost((void **)&e->h_tp[s], cap * sizeof(TmplParam)));
-          }
-          e->h_tp_cap = cap;
-          TRY(e->tparam.alloc(cap * sizeof(TmplParam)));
-     }
-     return TDF_OK;
-}
-
 // the error of a kernel error word whose bounded waits gave up, else TDF_OK
 static int wait_error(unsigned errf) {
      if (errf & ERR_STAGE_TIMEOUT)
@@ -1308,12 +1331,15 @@ static int finish_slot(tdf_engine *e, int slot, bool collect, int64_t *ntrig_tot
      }
      *ntrig_total += (int64_t)nfound;
      if (collect && nfound) {
-          size_t o = e->h_trig.size();
+          const size_t o = e->h_trig.size(), ahead = std::min<size_t>(nfound, tdf_engine::kTrigAhead);
           e->h_trig.resize(o + nfound);
+          memcpy(e->h_trig.data() + o, e->h_trig0[slot], ahead * sizeof(Trig));
           // the batch is complete (event above); the engine stream may run on
-          CUCHK(cudaMemcpy(e->h_trig.data() + o, e->trig[slot].p, nfound * sizeof(Trig), cudaMemcpyDeviceToHost));
+          if (nfound > ahead)
+               CUCHK(cudaMemcpy(e->h_trig.data() + o + ahead, e->trig[slot].as<Trig>() + ahead,
+                                (nfound - ahead) * sizeof(Trig), cudaMemcpyDeviceToHost));
      }
-     CUCHK(cudaMemsetAsync(e->counters[slot].p, 0, 2 * sizeof(unsigned long long), e->stream));
+     CUCHK(cudaMemsetAsync(e->counters(slot), 0, 2 * sizeof(unsigned long long), e->stream));
      return TDF_OK;
 }
 
@@ -1355,8 +1381,7 @@ static int search_core(tdf_engine *e, int npts, const int32_t *pm, const float *
           *ntrig_total = 0;
           CUCHK(cudaStreamSynchronize(e->sky_stream));
           CUCHK(cudaStreamSynchronize(e->stream));
-          for (int s = 0; s < 2; s++) CUCHK(cudaMemsetAsync(e->counters[s].p, 0, 2 * sizeof(unsigned long long), e->stream));
-          for (int l = 0; l < e->lanes_alloc; l++) CUCHK(cudaMemsetAsync(e->ln[l].tcnt.p, 0, e->ln[l].tcnt.bytes, e->stream));
+          CUCHK(cudaMemsetAsync(e->zeroed.p, 0, e->zeroed.bytes, e->stream));
           int pending[2] = {0, 0};
           bool over = false, need_full = false;
           size_t b = 0;
@@ -1397,12 +1422,15 @@ static int search_core(tdf_engine *e, int npts, const int32_t *pm, const float *
                size_t sev = e->timing ? timing_begin(e, sst) : (size_t)-1;
                TRY(run_sky_stage(e, nb));
                if (e->timing) timing_end(e, sev, KT_SKY, nb, sst);
-               CUCHK(cudaStreamWaitEvent(e->stream, e->sky_done[slot], 0));
                CUCHK(cudaMemcpyAsync(e->tparam.p, e->h_tp[slot], nt * sizeof(TmplParam), cudaMemcpyHostToDevice, e->stream));
+               CUCHK(cudaStreamWaitEvent(e->stream, e->sky_done[slot], 0));
                TRY(run_templates_batch(e, nt));
                CUCHK(cudaEventRecord(e->spin_done[slot], e->stream));
-               CUCHK(cudaMemcpyAsync(e->h_cnt + 2 * slot, e->counters[slot].p, 2 * sizeof(unsigned long long),
+               CUCHK(cudaMemcpyAsync(e->h_cnt + 2 * slot, e->counters(slot), 2 * sizeof(unsigned long long),
                                      cudaMemcpyDeviceToHost, e->stream));
+               if (collect)
+                    CUCHK(cudaMemcpyAsync(e->h_trig0[slot], e->trig[slot].p, tdf_engine::kTrigAhead * sizeof(Trig),
+                                          cudaMemcpyDeviceToHost, e->stream));
                CUCHK(cudaEventRecord(e->done[slot], e->stream));
                pending[slot] = 1;
           }
@@ -1578,8 +1606,7 @@ static int enqueue_plan(tdf_engine *e, const std::vector<PlanBatch> &pb) {
                                                             e->form == TDF_FORM_SPLIT);
      CUCHK(cudaGetLastError());
      e->launches++;
-     for (int s = 0; s < 2; s++) CUCHK(cudaMemsetAsync(e->counters[s].p, 0, 2 * sizeof(unsigned long long), e->stream));
-     for (int l = 0; l < e->lanes_alloc; l++) CUCHK(cudaMemsetAsync(e->ln[l].tcnt.p, 0, e->ln[l].tcnt.bytes, e->stream));
+     CUCHK(cudaMemsetAsync(e->zeroed.p, 0, e->zeroed.bytes, e->stream));
      // the sky stream's first work of the plan follows this point of the engine stream
      CUCHK(cudaEventRecord(e->plan_ev, e->stream));
      for (size_t i = 0; i < pb.size(); i++) {
@@ -1593,7 +1620,7 @@ static int enqueue_plan(tdf_engine *e, const std::vector<PlanBatch> &pb) {
           CUCHK(cudaEventRecord(e->spin_done[e->cur], e->stream));
      }
      for (int s = 0; s < 2; s++)
-          CUCHK(cudaMemcpyAsync(e->h_cnt + 2 * s, e->counters[s].p, 2 * sizeof(unsigned long long),
+          CUCHK(cudaMemcpyAsync(e->h_cnt + 2 * s, e->counters(s), 2 * sizeof(unsigned long long),
                                 cudaMemcpyDeviceToHost, e->stream));
      return TDF_OK;
 }
@@ -1793,7 +1820,7 @@ int tdf_engine_create(const tdf_segment *seg, const tdf_search_opts *opts, int f
      e->n2N = seg->interpftpad * seg->N;
      e->nF = opts->fr[1] - opts->fr[0] + 1;
      e->nblk_mu = opts->blocks_avg ? (opts->fr[1] - opts->fr[0]) / TDF_NAVFSTAT : 0;
-     if (max_sky_batch > 0) e->Bs = max_sky_batch;
+     e->Bs = max_sky_batch > 0 ? max_sky_batch : std::max(8, std::min(24, (1 << 20) / seg->nfft));
      const char *tc = getenv("TDF_TEMPLATES_PER_CHUNK");
      if (tc && atoi(tc) > 0) e->Tc = atoi(tc);
      // buffers for chunks up to 96 templates (the autotuner's range), or for
@@ -2279,30 +2306,30 @@ int tdf_fstat_spectrum(tdf_engine *e, int32_t pm, float mm, float nn, float ss, 
      q.slot = 0;
      q.id = 0;
      TRY(run_sky_stage(e, 1));
-     CUCHK(cudaStreamWaitEvent(e->stream, e->sky_done[0], 0));
      CUCHK(cudaMemcpyAsync(e->tparam.p, e->h_tp[0], sizeof(TmplParam), cudaMemcpyHostToDevice, e->stream));
-     CUCHK(cudaMemsetAsync(e->counters[0].p, 0, 2 * sizeof(unsigned long long), e->stream));
-     for (int l = 0; l < e->lanes_alloc; l++) CUCHK(cudaMemsetAsync(e->ln[l].tcnt.p, 0, e->ln[l].tcnt.bytes, e->stream));
+     CUCHK(cudaMemsetAsync(e->zeroed.p, 0, e->zeroed.bytes, e->stream));
+     CUCHK(cudaStreamWaitEvent(e->stream, e->sky_done[0], 0));
      e->sparse_now = false;   // the spectrum itself is the output: the full F store
      TRY(run_templates(e, e->tparam.as<TmplParam>(), 1));
-     CUCHK(cudaMemcpyAsync(e->h_cnt, e->counters[0].p, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->stream));
+     CUCHK(cudaMemcpyAsync(e->h_cnt, e->counters(0), 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->stream));
+     const int n = e->nF;
+     const bool split = e->form == TDF_FORM_SPLIT;
+     const size_t rsz = split ? sizeof(float) : sizeof(double);
+     CUCHK(cudaMemcpyAsync(e->h_F, e->ln[0].Fbuf.p, n * rsz, cudaMemcpyDeviceToHost, e->stream));
+     std::vector<unsigned char> mub(std::max(1, e->nblk_mu) * rsz);
+     if (e->nblk_mu)
+          CUCHK(cudaMemcpyAsync(mub.data(), e->ln[0].mubuf.p, e->nblk_mu * rsz, cudaMemcpyDeviceToHost, e->stream));
      CUCHK(cudaStreamSynchronize(e->stream));
      TRY(wait_error((unsigned)(e->h_cnt[1] & 0xffffffffu)));
-     const int n = e->nF;
-     if (e->form == TDF_FORM_SPLIT) {
-          std::vector<float> f(n), mu(std::max(1, e->nblk_mu));
-          CUCHK(cudaMemcpyAsync(f.data(), e->ln[0].Fbuf.p, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
-          if (e->nblk_mu)
-               CUCHK(cudaMemcpyAsync(mu.data(), e->ln[0].mubuf.p, e->nblk_mu * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
-          CUCHK(cudaStreamSynchronize(e->stream));
-          for (int i = 0; i < n; i++) F[i] = (i < e->nblk_mu * TDF_NAVFSTAT) ? (double)(f[i] / mu[i >> 12]) : (double)f[i];
+     const int nb = std::min(n, e->nblk_mu * TDF_NAVFSTAT);   // values with a block mean
+     if (split) {
+          const float *f = static_cast<const float *>(e->h_F), *mu = reinterpret_cast<const float *>(mub.data());
+          for (int i = 0; i < nb; i++) F[i] = (double)(f[i] / mu[i >> 12]);
+          for (int i = nb; i < n; i++) F[i] = (double)f[i];
      } else {
-          std::vector<double> mu(std::max(1, e->nblk_mu));
-          CUCHK(cudaMemcpyAsync(F, e->ln[0].Fbuf.p, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-          if (e->nblk_mu)
-               CUCHK(cudaMemcpyAsync(mu.data(), e->ln[0].mubuf.p, e->nblk_mu * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-          CUCHK(cudaStreamSynchronize(e->stream));
-          for (int i = 0; i < n && i < e->nblk_mu * TDF_NAVFSTAT; i++) F[i] = F[i] / mu[i >> 12];
+          const double *f = static_cast<const double *>(e->h_F), *mu = reinterpret_cast<const double *>(mub.data());
+          for (int i = 0; i < nb; i++) F[i] = f[i] / mu[i >> 12];
+          for (int i = nb; i < n; i++) F[i] = f[i];
      }
      return TDF_OK;
 }

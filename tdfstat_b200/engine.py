@@ -136,23 +136,24 @@ class Engine:
         else:
             mr = max_recs
         mp = max_pairs if max_pairs is not None else 8 * mr + 4096
-        recs = (_abi.TdfRecord * max(mr, 1))()
+        recs = np.empty(max(mr, 1), dtype=_REC_DTYPE)
         pairs = np.empty(max(mp, 1), dtype=np.float32)
         st = self.lib.tdf_search_points(self.h, npts, _p(pm, C.c_int32), _p(mm, C.c_float), _p(nn, C.c_float), sp,
-                                        recs, mr, C.byref(nrec), _p(pairs, C.c_float), mp, C.byref(npairs),
+                                        _p(recs, _abi.TdfRecord), mr, C.byref(nrec), _p(pairs, C.c_float), mp, C.byref(npairs),
                                         _p(per, C.c_int32))
         if st == _abi.TDF_ERR_CAPACITY and (max_recs is None or max_pairs is None):
             # the engine kept the results: fetch them into arrays of the right size
             mr, mp = nrec.value, npairs.value
-            recs = (_abi.TdfRecord * max(mr, 1))()
+            recs = np.empty(max(mr, 1), dtype=_REC_DTYPE)
             pairs = np.empty(max(mp, 1), dtype=np.float32)
-            st = self.lib.tdf_last_results(self.h, recs, mr, C.byref(nrec), _p(pairs, C.c_float), mp,
+            st = self.lib.tdf_last_results(self.h, _p(recs, _abi.TdfRecord), mr, C.byref(nrec), _p(pairs, C.c_float), mp,
                                            C.byref(npairs), _p(per, C.c_int32))
         _check(self.lib, st)
         n = nrec.value
-        a = np.frombuffer(memoryview(recs), dtype=_REC_DTYPE)[:n]
-        hdr = np.stack([a["m"], a["n"], a["s"], a["ra"], a["dec"], a["fdot"]], axis=1) if n else np.zeros((0, 6), np.float32)
-        return Result(hdr.astype(np.float32), a["len"].astype(np.int64), a["offset"].astype(np.int64),
+        a = recs[:n]
+        # the six float fields m, n, s, ra, dec, fdot lead the record
+        hdr = a.view(np.float32).reshape(n, _REC_DTYPE.itemsize // 4)[:, :6].copy()
+        return Result(hdr, a["len"].astype(np.int64), a["offset"].astype(np.int64),
                       pairs[: npairs.value].copy(), per[:npts].copy())
 
     def search_device(self, pm, mm, nn, sst=None) -> Tuple[int, int]:
@@ -193,7 +194,7 @@ class Engine:
         return nrec.value, ntrig.value
 
     def fstat(self, pm: int, mm: float, nn: float, ss: float) -> np.ndarray:
-        F = np.zeros(self.nF, dtype=np.float64)
+        F = np.empty(self.nF, dtype=np.float64)
         st = self.lib.tdf_fstat_spectrum(self.h, int(pm), float(mm), float(nn), float(ss), _p(F, C.c_double), len(F))
         _check(self.lib, st)
         return F
