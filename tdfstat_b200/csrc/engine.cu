@@ -138,15 +138,8 @@ static int launch_col_L(dim3 grid, const Pro &pro, const Epi &epi_in, const cx<T
 }
 
 template <typename T, int L, int SIGN, int NA, class Src, class Epi>
-static int launch_row_L(dim3 grid, const Src &src_in, const Epi &epi, const cx<T> *tw, cudaStream_t st) {
-     size_t smem = pass_smem_bytes<T, L, NA>();
-     Src src = src_in;
-     if constexpr (is_bulk<Src>::value) {
-          // the copies' barrier after the line buffers
-          smem = (smem + 15) / 16 * 16;
-          src.bar_off = (unsigned)smem;
-          smem += 16;
-     }
+static int launch_row_L(dim3 grid, const Src &src, const Epi &epi, const cx<T> *tw, cudaStream_t st) {
+     const size_t smem = pass_smem_bytes<T, L, NA>();
      auto kern = k_rowpass<T, L, SIGN, NA, Src, Epi>;
      if constexpr (NA == 1) register_sky_kernel((const void *)kern);
      TRY(set_smem(kern, smem));
@@ -239,7 +232,7 @@ template <typename T>
 struct FFTTables {
      int N = 0, N1 = 0, N2 = 0;
      DevBuf line1, line2, hi, lo;
-     DevBuf base, step, ltw1, ltw2;   // split-form passes (build_split)
+     DevBuf base, step, ltw1, ltw2;   // spindown passes (build_split)
      int build(int n) {
           N = n;
           int l = ilog2i(n);
@@ -259,15 +252,22 @@ struct FFTTables {
           CUCHK(cudaMemcpy(lo.p, o.data(), 1024 * sizeof(cx<T>), cudaMemcpyHostToDevice));
           return TDF_OK;
      }
-     // tables of the split-form passes (tdf_split.cuh): the columns' base
-     // twiddles base[n2*N1/8 + t] = W^(n2*t), t < N1/8, and step[n2] =
-     // W^(n2*N1/8); the pass twiddles of the two line lengths
+     // tables of the spindown passes (tdf_split.cuh): the columns' base
+     // twiddles base[n2*N1/8 + t] = W^(n2*t), t < N1/8; step[n2] = W^(n2*N1/8)
+     // (FP64: its powers, step[n2*8 + m] = W^(n2*m*N1/8)); the pass twiddles of
+     // the two line lengths
      int build_split() {
           const int R = N1 / 8;
-          std::vector<cx<T>> b((size_t)R * N2), st(N2);
+          constexpr bool powers = std::is_same<T, double>::value;
+          std::vector<cx<T>> b((size_t)R * N2), st((size_t)N2 * (powers ? 8 : 1));
           for (int n2 = 0; n2 < N2; n2++)
                for (int t = 0; t < R; t++) b[(size_t)n2 * R + t] = tw((long)n2 * t, N);
-          for (int n2 = 0; n2 < N2; n2++) st[n2] = tw((long)n2 * R, N);
+          for (int n2 = 0; n2 < N2; n2++) {
+               if (powers)
+                    for (int m = 0; m < 8; m++) st[(size_t)n2 * 8 + m] = tw((long)n2 * m * R, N);
+               else
+                    st[n2] = tw((long)n2 * R, N);
+          }
           TRY(put(base, b));
           TRY(put(step, st));
           TRY(put(ltw1, pass_twiddles(N1)));
@@ -366,7 +366,7 @@ struct tdf_engine {
      std::vector<double> lines;
      int N = 0, nfft = 0, nfftf = 0, Ninterp = 0, nifo = 0, Nal = 0, n2N = 0;
      int nF = 0, nblk_mu = 0;
-     int CL = 0;        // split form: entries of an operand column (ceil(N/N2), up to a multiple of 32)
+     int CL = 0;        // entries of an operand column (ceil(N/N2), up to a multiple of 32)
      // sky points per batch: 8, and more for short segments (2^16 points 16,
      // 2^15 and less 24), whose sky stage otherwise leaves most of the GPU idle:
      // 48 points x 33 spindowns of 2^14 points 934 us with 8, 839 with 24
@@ -383,7 +383,7 @@ struct tdf_engine {
      // sky stage
      DevBuf skyp[2], B0, B1, B2, shft, partial, aabb[2];
      // operands
-     DevBuf xab[2], s2[2], xa64[2], xb64[2], t1[2];   // per batch slot
+     DevBuf xab[2], s2[2], xre[2], xim[2], t1[2];   // per batch slot
      // spindown stage: consecutive resolve groups alternate between lanes,
      // each with its own stream and buffers, so that one lane's kernel tails
      // and trigger resolution overlap the other lane's passes
@@ -469,7 +469,6 @@ struct tdf_engine {
      uint64_t graph_tick = 0;
      bool use_graphs = true;   // TDF_GRAPHS=0 launches every kernel from the host
      bool graph_prio = true;   // TDF_GRAPH_PRIORITY=0 leaves captured kernel nodes at their default priority
-     bool row_bulk = true;     // FP64 form: row passes fetch their rows by bulk copies (TDF_ROW_BULK=0: per thread)
      // split form, N1 = N2: TDF_FUSED_PASSES=1 runs the column and row
      // passes of a chunk as one ordered launch of persistent CTAs
      // (k_spinpass), a template's rows fuse_lag templates behind its
@@ -641,26 +640,29 @@ static int engine_alloc(tdf_engine *e) {
      TRY(e->shft.alloc(Q * e->Nal * sizeof(double)));
      TRY(e->partial.alloc(Q * (e->nfft / 256) * 2 * sizeof(double)));
      for (int k = 0; k < 2; k++) TRY(e->aabb[k].alloc(Bs * sizeof(AaBb)));
-     const size_t ops = Q * e->Nal;
-     if (e->form == TDF_FORM_SPLIT) {
+     const bool split = e->form == TDF_FORM_SPLIT;
+     if (split) {
           TRY(e->t_f32.build(e->nfftf));
           TRY(e->t_f32.build_split());
-          const int N2 = e->t_f32.N2;
-          e->CL = ((e->N + N2 - 1) / N2 + 31) / 32 * 32;
-          const size_t cols = Q * N2 * (size_t)e->CL;
-          for (int k = 0; k < 2; k++) {
+     } else {
+          TRY(e->t_f64.build(e->nfftf));
+          TRY(e->t_f64.build_split());
+     }
+     const int N2 = split ? e->t_f32.N2 : e->t_f64.N2;
+     e->CL = ((e->N + N2 - 1) / N2 + 31) / 32 * 32;
+     const size_t cols = Q * N2 * (size_t)e->CL;
+     for (int k = 0; k < 2; k++) {
+          if (split) {
                TRY(e->xab[k].alloc(cols * sizeof(float4)));
                TRY(e->s2[k].alloc(cols * sizeof(float)));
-               // entries past the last sample are never written and stay zero
-               CUCHK(cudaMemset(e->xab[k].p, 0, e->xab[k].bytes));
-               CUCHK(cudaMemset(e->s2[k].p, 0, e->s2[k].bytes));
+          } else {
+               TRY(e->xre[k].alloc(cols * sizeof(double2)));
+               TRY(e->xim[k].alloc(cols * sizeof(double2)));
+               TRY(e->t1[k].alloc(cols * sizeof(double)));
           }
-     } else {
-          for (int k = 0; k < 2; k++) {
-               TRY(e->xa64[k].alloc(ops * sizeof(double2)));
-               TRY(e->xb64[k].alloc(ops * sizeof(double2)));
-               TRY(e->t1[k].alloc(ops * sizeof(double)));
-          }
+          // entries past the last sample are never written and stay zero
+          for (DevBuf *b : {&e->xab[k], &e->s2[k], &e->xre[k], &e->xim[k], &e->t1[k]})
+               if (b->p) CUCHK(cudaMemset(b->p, 0, b->bytes));
      }
      const size_t csz = e->form == TDF_FORM_SPLIT ? sizeof(float2) : sizeof(double2);
      const size_t rsz = e->form == TDF_FORM_SPLIT ? sizeof(float) : sizeof(double);
@@ -702,7 +704,6 @@ static int engine_alloc(tdf_engine *e) {
      TRY(ensure_tparam(e, 1));
      TRY(e->t_nfft.build(e->nfft));
      TRY(e->t_ninterp.build(e->Ninterp));
-     if (e->form == TDF_FORM_FP64) TRY(e->t_f64.build(e->nfftf));
      return TDF_OK;
 }
 
@@ -720,8 +721,8 @@ static void engine_free(tdf_engine *e) {
      for (SegData &d : e->sdv) d.release();
      DevBuf *bufs[] = {&e->fac, &e->plan_sky, &e->plan_tp, &e->plan_pts, &e->skyp[0],
                        &e->skyp[1], &e->B0, &e->B1, &e->B2, &e->shft, &e->partial, &e->aabb[0], &e->aabb[1],
-                       &e->xab[0], &e->xab[1], &e->s2[0], &e->s2[1], &e->xa64[0], &e->xa64[1], &e->xb64[0],
-                       &e->xb64[1], &e->t1[0], &e->t1[1], &e->tparam, &e->trig[0], &e->trig[1],
+                       &e->xab[0], &e->xab[1], &e->s2[0], &e->s2[1], &e->xre[0], &e->xre[1], &e->xim[0],
+                       &e->xim[1], &e->t1[0], &e->t1[1], &e->tparam, &e->trig[0], &e->trig[1],
                        &e->zeroed, &e->linesd};
      for (DevBuf *b : bufs) b->release();
      for (tdf_engine::Lane &L : e->ln) {
@@ -875,8 +876,7 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
      k_sky_prep<<<dim3(nblk, Q), 256, 0, st>>>(
           e->S().xdat.as<float>(), e->S().detssb.as<double>(), e->S().cosm.as<double>(), e->S().sinm.as<double>(),
           dsky, e->S().detp.as<DetParam>(), nifo, e->N, e->nfft, e->Nal, e->S().seg.oms,
-          e->B0.as<double2>(), ws, e->shft.as<double>(), split ? nullptr : e->t1[sl].as<double>(),
-          e->partial.as<double>());
+          e->B0.as<double2>(), ws, e->shft.as<double>(), e->partial.as<double>());
      CUCHK(cudaGetLastError());
      e->launches++;
      // Interpolation: forward FFT (nfft) of every (point, detector, a|b),
@@ -917,14 +917,11 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
      const SplintIn in{coef->as<double2>(), ws, e->shft.as<double>(), dsky, e->S().detssb.as<double>(),
                        e->S().detp.as<DetParam>(), e->Nal, e->N, e->n2N, e->Ninterp, e->S().seg.interpftpad, nifo,
                        e->partial.as<double>(), nblk, e->aabb[sl].as<AaBb>()};
-     if (split) {
-          const int N2 = e->t_f32.N2;
-          k_splint_split<<<dim3(N2 / 32, ((e->N + N2 - 1) / N2 + 7) / 8, Q), 256, 0, st>>>(
-               in, N2, e->CL, e->xab[sl].as<float4>(), e->s2[sl].as<float>());
-     } else {
-          k_splint<<<dim3((e->N + 255) / 256, Q), 256, 0, st>>>(in, e->xa64[sl].as<double2>(),
-                                                                e->xb64[sl].as<double2>());
-     }
+     const int N2 = split ? e->t_f32.N2 : e->t_f64.N2;
+     const dim3 g(N2 / 32, ((e->N + N2 - 1) / N2 + 7) / 8, Q);
+     auto splint = split ? k_splint<true> : k_splint<false>;
+     splint<<<g, 256, 0, st>>>(in, N2, e->CL, e->xab[sl].as<float4>(), e->s2[sl].as<float>(), e->xre[sl].as<double2>(),
+                               e->xim[sl].as<double2>(), e->t1[sl].as<double>());
      CUCHK(cudaGetLastError());
      e->launches++;
      CUCHK(cudaEventRecord(e->sky_done[sl], st));
@@ -945,7 +942,7 @@ static int group_templates(const tdf_engine *e) { return std::max(1, e->Gt / e->
 template <int L, int N2, int NIFO, int T>
 static int launch_split_col_t(const SplitCol &a, cudaStream_t st) {
      auto kern = k_split_col<L, N2, NIFO, T>;
-     const size_t smem = split_col_lines<L>() * T * SplitLine<L, false>::BYTES;
+     const size_t smem = split_col_lines<L>() * T * SplitLine<float2, L, false>::BYTES;
      TRY(set_smem(kern, smem));
      kern<<<dim3(N2 / split_col_lines<L>(), (a.nt + T - 1) / T), split_col_threads<L>(), smem, st>>>(a);
      CUCHK(cudaGetLastError());
@@ -985,32 +982,67 @@ static int launch_split_col(int N1, int N2, int sms, const SplitCol &a, cudaStre
      return set_error(TDF_ERR_UNSUPPORTED, "column FFT length %d", N1);
 }
 
-template <int L, int N1, bool HALF>
-static int launch_split_row_c(int sms, const SplitRow &a, cudaStream_t st) {
-     auto kern = k_split_row<L, N1, HALF>;
-     const size_t smem = split_row_smem<L>();
+template <int L, int NIFO>
+static int launch_fp64_col_c(int nt, const Fp64Col &a, cudaStream_t st) {
+     auto kern = k_fp64_col<L, NIFO>;
+     const size_t smem = fp64_col_lines<L>() * SplitLine<double2, L, false>::BYTES;
      TRY(set_smem(kern, smem));
-     kern<<<std::min(sms, a.nt * (N1 / RUN)), 512, smem, st>>>(a);
+     kern<<<dim3(a.N2 / fp64_col_lines<L>(), nt), fp64_col_threads<L>(), smem, st>>>(a);
+     CUCHK(cudaGetLastError());
+     return TDF_OK;
+}
+
+template <int L>
+static int launch_fp64_col_n(int nt, const Fp64Col &a, cudaStream_t st) {
+     switch (a.nifo) {
+     case 1: return launch_fp64_col_c<L, 1>(nt, a, st);
+     case 2: return launch_fp64_col_c<L, 2>(nt, a, st);
+     }
+     return launch_fp64_col_c<L, 0>(nt, a, st);
+}
+
+static int launch_fp64_col(int N1, int nt, const Fp64Col &a, cudaStream_t st) {
+     switch (N1) {
+     case 64: return launch_fp64_col_n<64>(nt, a, st);
+     case 128: return launch_fp64_col_n<128>(nt, a, st);
+     case 256: return launch_fp64_col_n<256>(nt, a, st);
+     case 512: return launch_fp64_col_n<512>(nt, a, st);
+     }
+     return set_error(TDF_ERR_UNSUPPORTED, "FP64 column FFT length %d", N1);
+}
+
+template <class V, int L, int N1, bool HALF>
+static int launch_row_hc(int sms, const RowArgs<V> &a, cudaStream_t st) {
+     auto kern = k_row<V, L, N1, HALF>;
+     const size_t smem = split_row_smem<V, L>();
+     TRY(set_smem(kern, smem));
+     kern<<<std::min(sms, a.nt * (N1 / run_of<V>)), 512, smem, st>>>(a);
      CUCHK(cudaGetLastError());
      return TDF_OK;
 }
 
 // the row pass keeps only bins <= fr1; with fr1 < nfftf/2 = N1*N2/2 every
 // kept output has k2 < N2/2
-template <int L, int N1>
-static int launch_split_row_h(int sms, const SplitRow &a, cudaStream_t st) {
-     return (int64_t)a.fr1 < (int64_t)N1 * L / 2 ? launch_split_row_c<L, N1, true>(sms, a, st)
-                                                 : launch_split_row_c<L, N1, false>(sms, a, st);
+template <class V, int L, int N1>
+static int launch_row_h(int sms, const RowArgs<V> &a, cudaStream_t st) {
+     return (int64_t)a.fr1 < (int64_t)N1 * L / 2 ? launch_row_hc<V, L, N1, true>(sms, a, st)
+                                                 : launch_row_hc<V, L, N1, false>(sms, a, st);
 }
 
-static int launch_split_row(int N1, int N2, int sms, const SplitRow &a, cudaStream_t st) {
+template <class V>
+static int launch_spin_row(int N1, int N2, int sms, const RowArgs<V> &a, cudaStream_t st) {
      const bool square = N1 == N2;
      switch (N2) {
-     case 64: return square ? launch_split_row_h<64, 64>(sms, a, st) : launch_split_row_h<64, 128>(sms, a, st);
-     case 128: return square ? launch_split_row_h<128, 128>(sms, a, st) : launch_split_row_h<128, 256>(sms, a, st);
-     case 256: return square ? launch_split_row_h<256, 256>(sms, a, st) : launch_split_row_h<256, 512>(sms, a, st);
-     case 512: return square ? launch_split_row_h<512, 512>(sms, a, st) : launch_split_row_h<512, 1024>(sms, a, st);
-     case 1024: return launch_split_row_h<1024, 1024>(sms, a, st);
+     case 64: return square ? launch_row_h<V, 64, 64>(sms, a, st) : launch_row_h<V, 64, 128>(sms, a, st);
+     case 128: return square ? launch_row_h<V, 128, 128>(sms, a, st) : launch_row_h<V, 128, 256>(sms, a, st);
+     case 256: return square ? launch_row_h<V, 256, 256>(sms, a, st) : launch_row_h<V, 256, 512>(sms, a, st);
+     case 512:
+          if (square) return launch_row_h<V, 512, 512>(sms, a, st);
+          if constexpr (sizeof(V) == 8) return launch_row_h<V, 512, 1024>(sms, a, st);
+          break;
+     case 1024:
+          if constexpr (sizeof(V) == 8) return launch_row_h<V, 1024, 1024>(sms, a, st);
+          break;
      }
      return set_error(TDF_ERR_UNSUPPORTED, "row FFT length %d", N2);
 }
@@ -1021,7 +1053,7 @@ static int launch_split_row(int N1, int N2, int sms, const SplitRow &a, cudaStre
 template <int L, bool HALF>
 static int launch_spin_c(int nt, int lag, const SplitCol &col, const SplitRow &row, unsigned *ctl, unsigned *err,
                          cudaStream_t st) {
-     const size_t smem = std::max(RUN / 2 * SplitLine<L, false>::BYTES, SplitLine<L, true>::BYTES);
+     const size_t smem = std::max(RUN / 2 * SplitLine<float2, L, false>::BYTES, SplitLine<float2, L, true>::BYTES);
      SpinOrder o{ctl, err, nt, L / RUN, L / RUN, std::max(1, std::min(lag, nt)), 1 << 20};
      auto kern = k_spinpass<L, HALF>;
      TRY(set_smem(kern, smem));
@@ -1074,7 +1106,7 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
           const SplitCol col{e->xab[e->cur].as<float4>(), e->s2[e->cur].as<float>(), ctp, Ln.Ybuf.as<float4>(),
                              t.base.template as<float2>(), t.step.template as<float2>(), t.ltw1.template as<float2>(),
                              e->N, e->CL, (e->N + t.N2 - 1) / t.N2, e->nifo, nt};
-          SplitRow row{Ln.Ybuf.as<float4>(), t.ltw2.template as<float2>(), Ln.Fbuf.as<float>() + (size_t)boff * e->nF,
+          SplitRow row{Ln.Ybuf.as<float2>(), t.ltw2.template as<float2>(), Ln.Fbuf.as<float>() + (size_t)boff * e->nF,
                        ctp, e->aabb[e->cur].as<AaBb>(), e->nF, e->opts.fr[0], e->opts.fr[1], e->opts.thr,
                        blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff, nullptr, nullptr, nt, errw};
           if (e->sparse_now) {
@@ -1100,24 +1132,19 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
           TRY(launch_split_col(t.N1, t.N2, e->sms, col, st));
           if (e->timing) timing_end(e, tev, KT_COL, nt, st);
           tev = e->timing ? timing_begin(e, st) : (size_t)-1;
-          TRY(launch_split_row(t.N1, t.N2, e->sms, row, st));
+          TRY(launch_spin_row(t.N1, t.N2, e->sms, row, st));
      } else {
-          StoreFourstep<T, -1, 2> epi{Ln.Ybuf.as<cx<T>>(), t.h(), t.o(), t.N2, e->nfftf};
-          DemodFP64 pro{e->xa64[e->cur].as<double2>(), e->xb64[e->cur].as<double2>(), e->t1[e->cur].as<double>(), ctp,
-                        e->N, t.N2, e->Nal, e->nifo};
-          TRY((launch_col<T, -1, 2>(t.N1, dim3(t.N2 / LINES, nt), pro, epi, t.l1(), st)));
+          const Fp64Col col{e->xre[e->cur].as<double2>(), e->xim[e->cur].as<double2>(), e->t1[e->cur].as<double>(), ctp,
+                            Ln.Ybuf.as<double2>(), t.base.template as<double2>(), t.step.template as<double2>(),
+                            t.ltw1.template as<double2>(), e->CL, (e->N + t.N2 - 1) / t.N2, t.N2, e->nifo};
+          TRY(launch_fp64_col(t.N1, nt, col, st));
           if (e->timing) timing_end(e, tev, KT_COL, nt, st);
           tev = e->timing ? timing_begin(e, st) : (size_t)-1;
-          StoreFstat<T> epi2{Ln.Fbuf.as<T>() + (size_t)boff * e->nF, ctp, e->aabb[e->cur].as<AaBb>(), e->nF,
-                             e->opts.fr[0], e->opts.fr[1], t.N1, e->opts.thr,
-                             blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff};
-          if (e->row_bulk) {
-               RowsYBulk<T> src{Ln.Ybuf.as<cx<T>>(), e->nfftf, t.N2, errw};
-               TRY((launch_row<T, -1, 2>(t.N2, dim3(t.N1 / LINES, nt), src, epi2, t.l2(), st)));
-          } else {
-               RowsY<T, 2> src{Ln.Ybuf.as<cx<T>>(), e->nfftf, t.N2};
-               TRY((launch_row<T, -1, 2>(t.N2, dim3(t.N1 / LINES, nt), src, epi2, t.l2(), st)));
-          }
+          const Fp64Row row{Ln.Ybuf.as<double2>(), t.ltw2.template as<double2>(),
+                            Ln.Fbuf.as<double>() + (size_t)boff * e->nF, ctp, e->aabb[e->cur].as<AaBb>(), e->nF,
+                            e->opts.fr[0], e->opts.fr[1], e->opts.thr, blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G,
+                            e->cand_cap, boff, nullptr, nullptr, nt, errw};
+          TRY(launch_spin_row(t.N1, t.N2, e->sms, row, st));
      }
      if (e->timing) timing_end(e, tev, KT_ROW, nt, st);
      e->launches += 2;
@@ -1215,8 +1242,8 @@ static int set_graph_priorities(const tdf_engine *e, cudaGraph_t g) {
           static std::once_flag once;
           std::call_once(once, [] {
                register_sky_kernel((const void *)k_sky_prep);
-               register_sky_kernel((const void *)k_splint);
-               register_sky_kernel((const void *)k_splint_split);
+               register_sky_kernel((const void *)k_splint<true>);
+               register_sky_kernel((const void *)k_splint<false>);
           });
      }
      size_t n = 0;
@@ -1840,8 +1867,6 @@ int tdf_engine_create(const tdf_segment *seg, const tdf_search_opts *opts, int f
      if (gp && gp[0] == '0') e->graph_prio = false;
      const char *ff = getenv("TDF_FULL_F");
      if (ff && ff[0] == '1') e->sparse_f = false;
-     const char *rb = getenv("TDF_ROW_BULK");
-     if (rb && rb[0] == '0') e->row_bulk = false;
      const char *fp = getenv("TDF_FUSED_PASSES");
      if (fp && fp[0] == '1') e->fused = true;
      const char *fl = getenv("TDF_FUSE_LAG");

@@ -7,16 +7,15 @@
 //                     partial sums of aa^2, bb^2 (jobcore.c:373-391)
 //     (FFT passes)    interpolation by FFT to twice the rate, delivering the
 //                     coefficients of the cubic spline through the series
-//     k_splint(_split) natural-spline evaluation at 2(i - shftf[i])
+//     k_splint        natural-spline evaluation at 2(i - shftf[i])
 //                     (auxi.c:93-169), division by sig2, conversion to the
 //                     spindown operands; aa, bb network sums (FLOAT_TYPE
 //                     emulation per form)
 //   spindown stage (once per template)
-//     (split form: tdf_split.cuh)
-//     DemodFP64       column-pass prologue: spindown_modulation
-//                     (spinmod.c:490-514) fused into the first FFT pass
-//     DemodSplit      the split form's, for the allocation-free entry point
-//     StoreFstat      row-pass epilogue: F = |Fa|^2/aa + |Fb|^2/bb
+//     (the passes: tdf_split.cuh)
+//     DemodSplit      column-pass prologue of the allocation-free entry point:
+//                     spindown_modulation (spinmod.c:490-514)
+//     StoreFstat      its row-pass epilogue: F = |Fa|^2/aa + |Fb|^2/bb
 //                     (jobcore.c:481-484)
 //     k_block_means   FStat blocks_avg means (auxi.c:336-363)
 //     k_threshold     MAX_ALG 3 local maxima, veto, trigger append
@@ -24,6 +23,9 @@
 #pragma once
 
 #include <float.h>
+
+#include <type_traits>
+
 #include "tdf_bulk.cuh"
 #include "tdf_passes.cuh"
 
@@ -92,8 +94,7 @@ __global__ void __launch_bounds__(256) k_sky_prep(
      const double *__restrict__ cosm, const double *__restrict__ sinm,
      const SkyParam *__restrict__ sp, const DetParam *__restrict__ dp,
      int nifo, int N, int nfft, int Nal, double oms,
-     double2 *__restrict__ W, size_t Wstride, double *__restrict__ shft,
-     double *__restrict__ t1, double *__restrict__ partial)
+     double2 *__restrict__ W, size_t Wstride, double *__restrict__ shft, double *__restrict__ partial)
 {
      const int q = blockIdx.y, p = q / nifo, d = q % nifo;
      const int i = blockIdx.x * 256 + threadIdx.x;
@@ -112,9 +113,7 @@ __global__ void __launch_bounds__(256) k_sky_prep(
                const double sh = __dadd_rn(__dadd_rn(__dmul_rn(S.nS0, e[3 * (size_t)i]), __dmul_rn(S.nS1, e[3 * (size_t)i + 1])),
                                            __dmul_rn(S.nS2, e[3 * (size_t)i + 2]));
                shft[(size_t)q * Nal + i] = sh;
-               const size_t o = ((size_t)p * nifo + d) * Nal + i;      // planar (FP64 operands)
                const double di = (double)i;
-               if (t1) t1[o] = __dadd_rn(__dmul_rn(di, di), __dmul_rn((double)(2 * i), sh));
                const double phase = __dadd_rn(__dmul_rn(S.het0, di), __dmul_rn(oms, sh));
                double sn, cn;
                sincos(phase, &sn, &cn);
@@ -329,34 +328,31 @@ __device__ __forceinline__ void splint_at(const SplintIn &I, int q, int i, doubl
      b = make_double2(vb.x / s2, vb.y / s2);
 }
 
-// FP64 operands, planar: [slot][det][i].  grid (ceil(N/256), Q), 256 threads
-__global__ void __launch_bounds__(256) k_splint(const __grid_constant__ SplintIn I, double2 *__restrict__ xa64,
-                                                double2 *__restrict__ xb64)
-{
-     const int q = blockIdx.y, d = q % I.nifo;
-     const int i = blockIdx.x * 256 + threadIdx.x;
-     if (blockIdx.x == 0 && d == 0) sky_sums(I.partial, I.nblk, I.dp, I.nifo, q / I.nifo, I.ab);
-     if (i >= I.N) return;
-     double2 a, b;
-     splint_at(I, q, i, I.shft[(size_t)q * I.Nal + i], shft0(I.sp[q / I.nifo], I.detssb + (size_t)d * 3 * I.N),
-               I.dp[d].sig2, a, b);
-     const size_t o = (size_t)q * I.Nal + i;
-     xa64[o] = a;
-     xb64[o] = b;
-}
+struct D4 {
+     double x, y, z, w;
+};
 
-// Split operands in the column layout of tdf_split.cuh: with i = N2*n1 + n2,
+// Operands in the column layout of tdf_split.cuh: with i = N2*n1 + n2, split
+// form (SPLIT)
 //   xab[(q*N2 + n2)*CL + n1] = (a.re, b.re, a.im, b.im) in FP32
 //   s2[((p*N2 + n2)*CL + n1)*nifo + d] = 2 i shft[i]
+// FP64 form
+//   xre, xim[(q*N2 + n2)*CL + n1] = (a.re, b.re), (a.im, b.im)
+//   t1[(q*N2 + n2)*CL + n1] = i^2 + 2 i shft[i]
 // A CTA takes a tile of 32 columns and 8 rows: it reads along i (32
 // consecutive samples per warp) and, through shared memory, writes 8
-// consecutive n1 of a column (128 bytes of xab) at a time.
+// consecutive n1 of a column (128 bytes) at a time.
 // grid (N2/32, ceil(ceil(N/N2)/8), Q), 256 threads
-__global__ void __launch_bounds__(256) k_splint_split(const __grid_constant__ SplintIn I, int N2, int CL,
-                                                      float4 *__restrict__ xab, float *__restrict__ s2out)
+template <bool SPLIT>
+__global__ void __launch_bounds__(256) k_splint(const __grid_constant__ SplintIn I, int N2, int CL,
+                                                float4 *__restrict__ xab, float *__restrict__ s2out,
+                                                double2 *__restrict__ xre, double2 *__restrict__ xim,
+                                                double *__restrict__ t1)
 {
-     __shared__ float4 xs[32][9];
-     __shared__ float ss[32][9];
+     using X = typename std::conditional<SPLIT, float4, D4>::type;
+     using S = typename std::conditional<SPLIT, float, double>::type;
+     __shared__ X xs[32][9];
+     __shared__ S ss[32][9];
      const int q = blockIdx.z, p = q / I.nifo, d = q % I.nifo;
      if (blockIdx.x == 0 && blockIdx.y == 0 && d == 0) sky_sums(I.partial, I.nblk, I.dp, I.nifo, p, I.ab);
      {
@@ -366,16 +362,30 @@ __global__ void __launch_bounds__(256) k_splint_split(const __grid_constant__ Sp
                const double sh = I.shft[(size_t)q * I.Nal + i];
                double2 a, b;
                splint_at(I, q, i, sh, shft0(I.sp[p], I.detssb + (size_t)d * 3 * I.N), I.dp[d].sig2, a, b);
-               xs[c][r] = make_float4((float)a.x, (float)b.x, (float)a.y, (float)b.y);
-               ss[c][r] = (float)__dmul_rn((double)(2 * i), sh);
+               X v;
+               v.x = a.x;
+               v.y = b.x;
+               v.z = a.y;
+               v.w = b.y;
+               xs[c][r] = v;
+               const double di = (double)i, e = __dmul_rn((double)(2 * i), sh);
+               ss[c][r] = SPLIT ? (S)(float)e : (S)__dadd_rn(__dmul_rn(di, di), e);
           }
      }
      __syncthreads();
      const int c = threadIdx.x / 8, r = threadIdx.x % 8;
      const int n1 = blockIdx.y * 8 + r, n2 = blockIdx.x * 32 + c;
      if (N2 * n1 + n2 < I.N) {
-          xab[((size_t)q * N2 + n2) * CL + n1] = xs[c][r];
-          s2out[(((size_t)p * N2 + n2) * CL + n1) * I.nifo + d] = ss[c][r];
+          const size_t o = ((size_t)q * N2 + n2) * CL + n1;
+          const X v = xs[c][r];
+          if constexpr (SPLIT) {
+               xab[o] = v;
+               s2out[(((size_t)p * N2 + n2) * CL + n1) * I.nifo + d] = ss[c][r];
+          } else {
+               xre[o] = make_double2(v.x, v.y);
+               xim[o] = make_double2(v.z, v.w);
+               t1[o] = ss[c][r];
+          }
      }
 }
 
@@ -494,40 +504,6 @@ struct DemodSplit {
                     v[0][kQ * h + q] = fa[q];
                     v[1][kQ * h + q] = fb[q];
                }
-          }
-     }
-};
-
-// Plain FP64 form: the reference's DOUBLE-build spindown_modulation.
-struct DemodFP64 {
-     const double2 *xa, *xb;
-     const double *t1;
-     const TmplParam *tp;
-     int N, N2, Nal, nifo;
-     template <int L>
-     __device__ __forceinline__ void load(double2 (&v)[2][8], int b, int n2, int t) const {
-          const TmplParam P = tp[b];
-          const size_t base = (size_t)P.slot * nifo * Nal;
-#pragma unroll
-          for (int m = 0; m < 8; m++) {
-               const int i = N2 * (t + m * (L / 8)) + n2;
-               double2 fa = make_double2(0., 0.), fb = make_double2(0., 0.);
-               if (i < N) {
-                    for (int d = 0; d < nifo; d++) {
-                         const size_t o = base + (size_t)d * Nal + i;
-                         const double phase = __dadd_rn(__dmul_rn(P.het1, (double)i), __dmul_rn(P.spnd, __ldg(&t1[o])));
-                         double sn, cs;
-                         sincos(phase, &sn, &cs);
-                         const double2 x = __ldg(&xa[o]), y = __ldg(&xb[o]);
-                         const double er = cs, ei = -sn;
-                         fa.x += x.x * er - x.y * ei;
-                         fa.y += x.x * ei + x.y * er;
-                         fb.x += y.x * er - y.y * ei;
-                         fb.y += y.x * ei + y.y * er;
-                    }
-               }
-               v[0][m] = fa;
-               v[1][m] = fb;
           }
      }
 };

@@ -14,7 +14,6 @@
 
 #include <type_traits>
 
-#include "tdf_bulk.cuh"
 #include "tdf_fft.cuh"
 
 namespace tdf {
@@ -29,30 +28,20 @@ constexpr size_t pass_smem_bytes() {
 }
 
 // resident CTAs per SM the passes are compiled for (register cap): FP32
-// column passes and row passes; FP64 passes at 64 registers with one array
-// (the sky stage; two CTAs of 512 threads fit the shared memory) and 128 with
-// two
-template <typename T, int L, int NA>
+// column passes and row passes; FP64 passes at 64 registers (two CTAs of 512
+// threads fit the shared memory)
+template <typename T, int L>
 constexpr int pass_min_blocks() {
-     return sizeof(T) == 4 ? (L <= 256 ? 3 : (L == 512 ? 2 : 1)) : (1024 / NA / L > 1 ? 1024 / NA / L : 1);
+     return sizeof(T) == 4 ? (L <= 256 ? 3 : (L == 512 ? 2 : 1)) : (1024 / L > 1 ? 1024 / L : 1);
 }
-template <typename T, int L, int NA>
+template <typename T, int L>
 constexpr int row_min_blocks() {
-     return sizeof(T) == 4 ? (L <= 256 ? 4 : (L == 512 ? 2 : 1)) : (1024 / NA / L > 1 ? 1024 / NA / L : 1);
+     return sizeof(T) == 4 ? (L <= 256 ? 4 : (L == 512 ? 2 : 1)) : (1024 / L > 1 ? 1024 / L : 1);
 }
 
 // An epilogue with `static constexpr bool kTables = true` keeps tables in
 // dynamic shared memory at byte offset tab_off: load_tables<L>() fills them
 // before the first barrier and store() gets the shared memory base.
-// A row-pass source with `static constexpr bool kBulk = true` brings the
-// CTA's rows into shared memory itself: load_bulk() gets the line-buffer
-// area (free until the first pass stores) and its barrier at pro.bar_off,
-// and loads the line twiddle table on the way.
-template <class P, class = void>
-struct is_bulk : std::false_type {};
-template <class P>
-struct is_bulk<P, std::void_t<decltype(P::kBulk)>> : std::integral_constant<bool, P::kBulk> {};
-
 template <class P, class = void>
 struct has_tables : std::false_type {};
 template <class P>
@@ -95,15 +84,10 @@ __device__ __forceinline__ void row_body(const Src &src, const Epi &epi, const c
      const int c = tid % LINES, t = tid / LINES;
      cx<T> v[NA][8];
      cx<T> *s[NA];
-     if constexpr (is_bulk<Src>::value) {
-          src.template load_bulk<L>(v, b, k1b, c, t, reinterpret_cast<unsigned char *>(lines),
-                                    reinterpret_cast<uint64_t *>(smem_raw + src.bar_off), tw, twline);
-     } else {
-          // first-pass inputs straight from the rows into registers: per load
-          // instruction a warp reads 4 consecutive elements of each of 8 rows
-          src.template load<L>(v, b, k1b + c, t);
-          load_table<T>(tw, twline, L);
-     }
+     // first-pass inputs straight from the rows into registers: per load
+     // instruction a warp reads 4 consecutive elements of each of 8 rows
+     src.template load<L>(v, b, k1b + c, t);
+     load_table<T>(tw, twline, L);
 #pragma unroll
      for (int a = 0; a < NA; a++) s[a] = lines + (a * LINES + c) * G::STRIDE;
      __syncthreads();
@@ -112,14 +96,14 @@ __device__ __forceinline__ void row_body(const Src &src, const Epi &epi, const c
 }
 
 template <typename T, int L, int SIGN, int NA, class Pro, class Epi>
-__global__ void __launch_bounds__(pass_threads<L>(), (pass_min_blocks<T, L, NA>()))
+__global__ void __launch_bounds__(pass_threads<L>(), (pass_min_blocks<T, L>()))
 k_colpass(const __grid_constant__ Pro pro, Epi epi, const cx<T> *__restrict__ twline) {
      extern __shared__ __align__(128) unsigned char smem_raw[];
      col_body<T, L, SIGN, NA>(pro, epi, twline, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 template <typename T, int L, int SIGN, int NA, class Src, class Epi>
-__global__ void __launch_bounds__(pass_threads<L>(), (row_min_blocks<T, L, NA>())) k_rowpass(Src src, Epi epi, const cx<T> *__restrict__ twline) {
+__global__ void __launch_bounds__(pass_threads<L>(), (row_min_blocks<T, L>())) k_rowpass(Src src, Epi epi, const cx<T> *__restrict__ twline) {
      extern __shared__ __align__(128) unsigned char smem_raw[];
      row_body<T, L, SIGN, NA>(src, epi, twline, blockIdx.x, blockIdx.y, smem_raw);
 }
@@ -206,68 +190,6 @@ struct RowsY {
                     for (int a = 0; a < NA; a++) v[a][m] = e[a];
                }
           }
-     }
-};
-
-// RowsY<T, 2> with the CTA's LINES rows brought in by bulk copies: row r
-// (N2 elements of 2 cx<T>, both arrays) goes to shared offset
-// r * (EB*N2 + 16).  A 16-byte load is served 8 lanes at a time, here the 8
-// rows at one element; the 16-byte pad puts those on 8 different 16-byte
-// bank groups (EB*N2 is a multiple of 128).  The slots alias the line
-// buffers, which the first
-// pass only writes after k_rowpass's barrier that follows the reads.  Thread
-// 0 issues the copies; everyone waits on one mbarrier (bounded: on time-out
-// ERR_STAGE_TIMEOUT is or-ed into *err).
-template <typename T>
-struct RowsYBulk {
-     const cx<T> *y;
-     int N;            // N1*N2
-     int rowstride;    // N2
-     unsigned *err;
-     unsigned bar_off = 0;   // byte offset of the barrier in dynamic shared memory (set by the launcher)
-     static constexpr bool kBulk = true;
-     static constexpr unsigned kPad = 16;
-     static constexpr unsigned EB = 2 * sizeof(cx<T>);   // bytes of an element, both arrays
-
-     template <int L>
-     __host__ __device__ static constexpr size_t stage_bytes() { return (size_t)LINES * (EB * L + kPad); }
-
-     template <int L>
-     __device__ __forceinline__ void load_bulk(cx<T> (&v)[2][8], int b, int k1b, int c, int t, unsigned char *stage,
-                                               uint64_t *bar, cx<T> *tw, const cx<T> *twline) const {
-          constexpr unsigned RB = EB * L;   // bytes of a row
-          static_assert(stage_bytes<L>() <= sizeof(cx<T>) * 2 * LINES * LineGeom<T, L>::STRIDE,
-                        "row slots must fit in the line buffers");
-          if (threadIdx.x == 0) {
-               mbar_init(bar, 1);
-               mbar_fence_init();
-          }
-          __syncthreads();   // the barrier is initialised before anyone waits on it
-          if (threadIdx.x == 0) {
-               mbar_expect_tx(bar, LINES * RB);
-               const cx<T> *r0 = y + ((size_t)b * N + (size_t)k1b * rowstride) * 2;
-#pragma unroll
-               for (int r = 0; r < LINES; r++)
-                    bulk_load(stage + r * (RB + kPad), r0 + (size_t)r * rowstride * 2, RB, bar);
-          }
-          load_table<T>(tw, twline, L);
-          const bool ok = mbar_wait(bar, 0u);
-          const unsigned char *row = stage + c * (RB + kPad);
-#pragma unroll
-          for (int m = 0; m < 8; m++) {
-               const int e = t + m * (L / 8);
-               if constexpr (sizeof(T) == 4) {
-                    const float4 q = reinterpret_cast<const float4 *>(row)[e];
-                    v[0][m] = make_float2(q.x, q.y);
-                    v[1][m] = make_float2(q.z, q.w);
-               } else {
-                    v[0][m] = reinterpret_cast<const cx<T> *>(row)[2 * e];
-                    v[1][m] = reinterpret_cast<const cx<T> *>(row)[2 * e + 1];
-               }
-          }
-          if (!ok) atomicOr(err, ERR_STAGE_TIMEOUT);
-          // k_rowpass's barrier after this call keeps the first pass's stores
-          // (the slots alias the line buffers) behind every thread's reads
      }
 };
 

@@ -1,9 +1,14 @@
-// tdf_split.cuh -- the spindown passes of the split form (FP32, two arrays):
+// tdf_split.cuh -- the spindown passes of both forms (two arrays):
 //
-//   k_split_col   demodulation of a template's samples, the N1-point FFTs of
+//   k_split_col /
+//   k_fp64_col    demodulation of a template's samples, the N1-point FFTs of
 //                 its columns and the four-step twiddle -> Y
-//   k_split_row   the N2-point FFTs of the rows of Y and the F-statistic
-//   k_spinpass    both as one ordered launch of persistent CTAs (opt-in)
+//   k_row<V>      the N2-point FFTs of the rows of Y and the F-statistic
+//   k_spinpass    split form: both as one ordered launch of persistent CTAs
+//                 (opt-in)
+//
+// V = float2 (split form) or double2 (FP64 form) is a pair of one component
+// of both arrays.
 //
 // Arithmetic.  The two arrays (a, b) go through the same transform with the
 // same twiddles, so every value is held as a P2: the real parts of both
@@ -24,16 +29,19 @@
 //   operands  xab[(slot*nifo + d)*N2 + n2][n1] float4 (a.re, b.re, a.im, b.im)
 //             s2[slot*N2 + n2][n1][d]           (rows of CL >= N/N2 entries)
 //   Y         [template][k1/RUN][n2][k1%RUN]  float4, likewise (re, im)
-// The column pass reads 512 consecutive bytes per warp and load and writes
-// Y in full 128-byte lines (RUN consecutive k1); the row pass of CTA k1/RUN
-// reads one contiguous block.
+// (FP64: xre, xim double2 and t1 double in the same order of columns, Y in
+// blocks of a real plane [n2][k1%RUN] double2 and an imaginary one).  The
+// column pass reads 512 consecutive bytes per warp and load and writes Y in
+// runs of RUN consecutive k1 (128-byte lines; FP64 64 bytes in each plane);
+// the row pass reads one contiguous block per k1/RUN.
 #pragma once
 
 namespace tdf {
 
-// consecutive k1 of Y (full 128-byte lines for the column pass's stores) =
-// rows per row-pass CTA, the run of consecutive bins it holds
-constexpr int RUN = 8;
+// consecutive k1 of Y = rows per row block, the run of consecutive bins it
+// holds; a block has 128 N2 bytes in both forms
+template <class V> constexpr int run_of = sizeof(V) == 8 ? 8 : 4;
+constexpr int RUN = run_of<float2>;
 
 // ------------------------------------------------------------------ packed arithmetic
 
@@ -50,14 +58,22 @@ __device__ __forceinline__ float2 psub(float2 a, float2 b) {
      return r;
 }
 __device__ __forceinline__ float2 pdup(float x) { return make_float2(x, x); }
+__device__ __forceinline__ double2 padd(double2 a, double2 b) { return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)); }
+__device__ __forceinline__ double2 psub(double2 a, double2 b) { return make_double2(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y)); }
+__device__ __forceinline__ double2 pmul(double2 a, double2 b) { return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)); }
+__device__ __forceinline__ double2 pfma(double2 a, double2 b, double2 c) { return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)); }
+__device__ __forceinline__ double2 pdup(double x) { return make_double2(x, x); }
 
 // one complex value of both arrays: re = (a.re, b.re), im = (a.im, b.im)
-struct P2 {
-     float2 re, im;
+template <class V> struct PV {
+     V re, im;
 };
-__device__ __forceinline__ P2 operator+(P2 a, P2 b) { return P2{padd(a.re, b.re), padd(a.im, b.im)}; }
-__device__ __forceinline__ P2 operator-(P2 a, P2 b) { return P2{psub(a.re, b.re), psub(a.im, b.im)}; }
-__device__ __forceinline__ P2 pzero() { return P2{pdup(0.f), pdup(0.f)}; }
+using P2 = PV<float2>;
+using D2 = PV<double2>;
+template <class V> __device__ __forceinline__ PV<V> operator+(PV<V> a, PV<V> b) { return PV<V>{padd(a.re, b.re), padd(a.im, b.im)}; }
+template <class V> __device__ __forceinline__ PV<V> operator-(PV<V> a, PV<V> b) { return PV<V>{psub(a.re, b.re), psub(a.im, b.im)}; }
+template <class V> __device__ __forceinline__ PV<V> pzero_of() { return PV<V>{pdup(decltype(V::x)(0)), pdup(decltype(V::x)(0))}; }
+__device__ __forceinline__ P2 pzero() { return pzero_of<float2>(); }
 __device__ __forceinline__ float4 pack4(P2 a) { return make_float4(a.re.x, a.re.y, a.im.x, a.im.y); }
 __device__ __forceinline__ P2 unpack4(float4 q) { return P2{make_float2(q.x, q.y), make_float2(q.z, q.w)}; }
 // product of two twiddles; the rounding is fixed here, whatever the compiler
@@ -65,49 +81,53 @@ __device__ __forceinline__ P2 unpack4(float4 q) { return P2{make_float2(q.x, q.y
 __device__ __forceinline__ float2 cmul_tw(float2 a, float2 b) {
      return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
+__device__ __forceinline__ double2 cmul_tw(double2 a, double2 b) {
+     return make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
 // both arrays' value times one complex factor
-__device__ __forceinline__ P2 pcmul(P2 a, float2 w) {
-     const float2 wr = pdup(w.x), wi = pdup(w.y), ni = pdup(-w.y);
-     return P2{pfma(a.im, ni, pmul(a.re, wr)), pfma(a.im, wr, pmul(a.re, wi))};
+template <class V> __device__ __forceinline__ PV<V> pcmul(PV<V> a, V w) {
+     const V wr = pdup(w.x), wi = pdup(w.y), ni = pdup(-w.y);
+     return PV<V>{pfma(a.im, ni, pmul(a.re, wr)), pfma(a.im, wr, pmul(a.re, wi))};
 }
 
 // forward 4-point DFT in place, natural-order outputs
-__device__ __forceinline__ void pdft4(P2 &y0, P2 &y1, P2 &y2, P2 &y3) {
-     const P2 c0 = y0 + y2, c1 = y0 - y2, c2 = y1 + y3, d = y1 - y3;
+template <class V> __device__ __forceinline__ void pdft4(PV<V> &y0, PV<V> &y1, PV<V> &y2, PV<V> &y3) {
+     const PV<V> c0 = y0 + y2, c1 = y0 - y2, c2 = y1 + y3, d = y1 - y3;
      y0 = c0 + c2;
      y2 = c0 - c2;
-     y1 = P2{padd(c1.re, d.im), psub(c1.im, d.re)};   // c1 - i d
-     y3 = P2{psub(c1.re, d.im), padd(c1.im, d.re)};   // c1 + i d
+     y1 = PV<V>{padd(c1.re, d.im), psub(c1.im, d.re)};   // c1 - i d
+     y3 = PV<V>{psub(c1.re, d.im), padd(c1.im, d.re)};   // c1 + i d
 }
 
 // forward 8-point DFT in place, natural-order outputs.  The odd half's
 // factors h(1 -+ i), h = sqrt(1/2), are applied in the last additions (fused
 // multiply-adds): 52 packed instructions.
-__device__ __forceinline__ void pdft8(P2 (&v)[8]) {
-     const float2 h = pdup(0.70710678118654752440f), mh = pdup(-0.70710678118654752440f);
-     P2 a0 = v[0] + v[4], b0 = v[0] - v[4];
-     P2 a1 = v[1] + v[5], b1 = v[1] - v[5];
-     P2 a2 = v[2] + v[6], b2 = v[2] - v[6];
-     P2 a3 = v[3] + v[7], b3 = v[3] - v[7];
+template <class V> __device__ __forceinline__ void pdft8(PV<V> (&v)[8]) {
+     using R1 = decltype(V::x);
+     const V h = pdup(R1(0.70710678118654752440)), mh = pdup(R1(-0.70710678118654752440));
+     PV<V> a0 = v[0] + v[4], b0 = v[0] - v[4];
+     PV<V> a1 = v[1] + v[5], b1 = v[1] - v[5];
+     PV<V> a2 = v[2] + v[6], b2 = v[2] - v[6];
+     PV<V> a3 = v[3] + v[7], b3 = v[3] - v[7];
      pdft4(a0, a1, a2, a3);
      // b1 W8 = h (p + i q), b3 W8^3 = h (r - i s)
-     const float2 p = padd(b1.re, b1.im), q = psub(b1.im, b1.re);
-     const float2 r = psub(b3.im, b3.re), s = padd(b3.re, b3.im);
-     const float2 P = padd(p, r), Q = psub(q, s), R = psub(p, r), S = padd(q, s);
-     const P2 c0{padd(b0.re, b2.im), psub(b0.im, b2.re)};   // b0 - i b2
-     const P2 c1{psub(b0.re, b2.im), padd(b0.im, b2.re)};   // b0 + i b2
+     const V p = padd(b1.re, b1.im), q = psub(b1.im, b1.re);
+     const V r = psub(b3.im, b3.re), s = padd(b3.re, b3.im);
+     const V P = padd(p, r), Q = psub(q, s), R = psub(p, r), S = padd(q, s);
+     const PV<V> c0{padd(b0.re, b2.im), psub(b0.im, b2.re)};   // b0 - i b2
+     const PV<V> c1{psub(b0.re, b2.im), padd(b0.im, b2.re)};   // b0 + i b2
      v[0] = a0;
      v[2] = a1;
      v[4] = a2;
      v[6] = a3;
-     v[1] = P2{pfma(P, h, c0.re), pfma(Q, h, c0.im)};
-     v[5] = P2{pfma(P, mh, c0.re), pfma(Q, mh, c0.im)};
-     v[3] = P2{pfma(S, h, c1.re), pfma(R, mh, c1.im)};
-     v[7] = P2{pfma(S, mh, c1.re), pfma(R, h, c1.im)};
+     v[1] = PV<V>{pfma(P, h, c0.re), pfma(Q, h, c0.im)};
+     v[5] = PV<V>{pfma(P, mh, c0.re), pfma(Q, mh, c0.im)};
+     v[3] = PV<V>{pfma(S, h, c1.re), pfma(R, mh, c1.im)};
+     v[7] = PV<V>{pfma(S, mh, c1.re), pfma(R, h, c1.im)};
 }
 
-template <int R>
-__device__ __forceinline__ void ppass_dft(P2 (&v)[8]) {
+template <int R, class V>
+__device__ __forceinline__ void ppass_dft(PV<V> (&v)[8]) {
      if (R == 8) {
           pdft8(v);
      } else if (R == 4) {
@@ -116,7 +136,7 @@ __device__ __forceinline__ void ppass_dft(P2 (&v)[8]) {
      } else {
 #pragma unroll
           for (int q = 0; q < 4; q++) {
-               const P2 t = v[q];
+               const PV<V> t = v[q];
                v[q] = t + v[q + 4];
                v[q + 4] = t - v[q + 4];
           }
@@ -148,10 +168,10 @@ __host__ __device__ constexpr int ltw_entries(int L) {
 
 // A pass's twiddles W^jm, W^2jm, W^4jm of the butterflies a thread owns
 // (loaded ahead of the exchange that precedes the pass).
-template <int L, int NS> struct PassTw {
+template <class V, int L, int NS> struct PassTw {
      static constexpr int R = pass_radix(L, NS), Q = 8 / R, K = pass_powers(R);
-     float2 w[Q][K];
-     __device__ __forceinline__ void load(const float2 *__restrict__ ltw, int t) {
+     V w[Q][K];
+     __device__ __forceinline__ void load(const V *__restrict__ ltw, int t) {
 #pragma unroll
           for (int q = 0; q < Q; q++)
 #pragma unroll
@@ -160,12 +180,12 @@ template <int L, int NS> struct PassTw {
 };
 
 // applied to the T templates whose lines a thread holds
-template <int L, int NS, int T>
-__device__ __forceinline__ void ppass_twiddle(P2 (&v)[T][8], const PassTw<L, NS> &tw) {
+template <int L, int NS, int T, class V>
+__device__ __forceinline__ void ppass_twiddle(PV<V> (&v)[T][8], const PassTw<V, L, NS> &tw) {
      constexpr int R = pass_radix(L, NS);
 #pragma unroll
      for (int q = 0; q < 8 / R; q++) {
-          float2 w[8];
+          V w[8];
           w[1] = tw.w[q][0];
           if constexpr (R >= 4) {
                w[2] = tw.w[q][1];
@@ -202,37 +222,41 @@ __device__ __forceinline__ void ppass_twiddle(P2 (&v)[T][8], const PassTw<L, NS>
 // elements, served 16 lanes (4 pairs at 4 t) at a time; lines 2 (mod 16)
 // elements apart put those on different banks.
 
-template <int L, bool ROW> struct SplitLine {
-     // elements between lines: of 16 bytes (columns) or of 8 in each plane (rows)
+// FP64: 16-byte elements in two planes everywhere, served 8 lanes at a time;
+// columns as above, rows 4 lines at 2 consecutive t (lines 2 (mod 8) elements
+// apart).
+
+template <class V, int L, bool ROW> struct SplitLine {
+     // elements between lines: a value (split-form columns) or one component in each plane
      static constexpr int STRIDE = L + L / 8 + (ROW ? 2 : 0);
-     static constexpr int PLANE = RUN * STRIDE;
+     static constexpr int PLANE = (ROW ? run_of<V> : 1) * STRIDE;
+     static constexpr bool WHOLE = !ROW && sizeof(V) == 8;   // one 16-byte element per value
      static __device__ __forceinline__ int pos(int p) { return p + (p >> 3); }
      // distance of positions d apart, d a multiple of 8
      static __host__ __device__ constexpr int dist(int d) { return d + d / 8; }
-     // bytes of a column line, of the RUN rows of a CTA
-     static constexpr size_t BYTES = 16 * (size_t)(ROW ? PLANE : STRIDE);
+     // bytes of a column line, of the rows of a block
+     static constexpr size_t BYTES = 2 * sizeof(V) * (size_t)PLANE;
+
+     static __device__ __forceinline__ void put(unsigned char *s, int p, PV<V> a) {
+          if constexpr (WHOLE) {
+               reinterpret_cast<float4 *>(s)[p] = pack4(a);
+          } else {
+               V *f = reinterpret_cast<V *>(s) + p;
+               f[0] = a.re;
+               f[PLANE] = a.im;
+          }
+     }
+     static __device__ __forceinline__ PV<V> get(const unsigned char *s, int p) {
+          if constexpr (WHOLE) {
+               return unpack4(reinterpret_cast<const float4 *>(s)[p]);
+          } else {
+               const V *f = reinterpret_cast<const V *>(s) + p;
+               return PV<V>{f[0], f[PLANE]};
+          }
+     }
 };
 
-template <int L, bool ROW>
-__device__ __forceinline__ void line_put(unsigned char *s, int p, P2 a) {
-     if (ROW) {
-          float2 *f = reinterpret_cast<float2 *>(s) + p;
-          f[0] = a.re;
-          f[SplitLine<L, ROW>::PLANE] = a.im;
-     } else {
-          reinterpret_cast<float4 *>(s)[p] = pack4(a);
-     }
-}
-template <int L, bool ROW>
-__device__ __forceinline__ P2 line_get(const unsigned char *s, int p) {
-     if (ROW) {
-          const float2 *f = reinterpret_cast<const float2 *>(s) + p;
-          return P2{f[0], f[SplitLine<L, ROW>::PLANE]};
-     }
-     return unpack4(reinterpret_cast<const float4 *>(s)[p]);
-}
-
-// the L/8 threads of one column, or the L/2 of RUN rows, wait for one another
+// the L/8 threads of one column, or the L/2 of a row block, wait for one another
 // (id: the group's number within the CTA)
 template <int L, bool ROW>
 __device__ __forceinline__ void group_sync(int id) {
@@ -246,10 +270,10 @@ __device__ __forceinline__ void group_sync(int id) {
 // The passes from span NS on, the data and the pass's twiddles at hand.
 // s: the memory of the thread's first line, the k-th one's `next` bytes
 // further; read() is called when the thread has read the last exchange.
-template <int L, bool ROW, int NS, int T, class F>
-__device__ __forceinline__ void line_pass(P2 (&v)[T][8], unsigned char *s, int next, const float2 *__restrict__ ltw,
-                                          int t, int id, const PassTw<L, (NS > 1 ? NS : 8)> &tw, const F &read) {
-     using G = SplitLine<L, ROW>;
+template <int L, bool ROW, int NS, int T, class V, class F>
+__device__ __forceinline__ void line_pass(PV<V> (&v)[T][8], unsigned char *s, int next, const V *__restrict__ ltw,
+                                          int t, int id, const PassTw<V, L, (NS > 1 ? NS : 8)> &tw, const F &read) {
+     using G = SplitLine<V, L, ROW>;
      constexpr int R = pass_radix(L, NS);
      if constexpr (NS > 1) ppass_twiddle<L, NS, T>(v, tw);
 #pragma unroll
@@ -257,14 +281,14 @@ __device__ __forceinline__ void line_pass(P2 (&v)[T][8], unsigned char *s, int n
      if constexpr (NS * R < L) {
           // (R = 8 here) output r of butterfly t goes to (t/NS)*8 NS + t%NS + r NS
           constexpr int RN = pass_radix(L, NS * 8);
-          PassTw<L, NS * 8> tn;
+          PassTw<V, L, NS * 8> tn;
           tn.load(ltw, t);
           if constexpr (NS > 1) group_sync<L, ROW>(id);   // the previous exchange is read
           const int d = NS == 1 ? G::dist(8) * t : G::pos((t / NS) * NS * 8 + (t % NS));
 #pragma unroll
           for (int k = 0; k < T; k++)
 #pragma unroll
-               for (int r = 0; r < 8; r++) line_put<L, ROW>(s + k * next, d + (NS == 1 ? r : r * G::dist(NS)), v[k][r]);
+               for (int r = 0; r < 8; r++) G::put(s + k * next, d + (NS == 1 ? r : r * G::dist(NS)), v[k][r]);
           group_sync<L, ROW>(id);
 #pragma unroll
           for (int k = 0; k < T; k++)
@@ -273,7 +297,7 @@ __device__ __forceinline__ void line_pass(P2 (&v)[T][8], unsigned char *s, int n
                     const int d1 = G::pos(t + q * (L / 8));
 #pragma unroll
                     for (int r = 0; r < RN; r++)
-                         v[k][q + r * (8 / RN)] = line_get<L, ROW>(s + k * next, d1 + r * G::dist(L / RN));
+                         v[k][q + r * (8 / RN)] = G::get(s + k * next, d1 + r * G::dist(L / RN));
                }
           if constexpr (NS * 8 * RN >= L) read();
           line_pass<L, ROW, NS * 8, T>(v, s, next, ltw, t, id, tn, read);
@@ -283,10 +307,10 @@ __device__ __forceinline__ void line_pass(P2 (&v)[T][8], unsigned char *s, int n
 // L-point forward transform of a thread's T lines: thread t holds
 // x[t + m L/8] on entry and X[t + m L/8] on exit.  The lines' shared memory
 // must be free on entry.
-template <int L, bool ROW, int T, class F>
-__device__ __forceinline__ void split_fft(P2 (&v)[T][8], unsigned char *s, int next, const float2 *__restrict__ ltw,
+template <int L, bool ROW, int T, class V, class F>
+__device__ __forceinline__ void split_fft(PV<V> (&v)[T][8], unsigned char *s, int next, const V *__restrict__ ltw,
                                           int t, int id, const F &read) {
-     line_pass<L, ROW, 1, T>(v, s, next, ltw, t, id, PassTw<L, 8>(), read);
+     line_pass<L, ROW, 1, T>(v, s, next, ltw, t, id, PassTw<V, L, 8>(), read);
 }
 
 // ------------------------------------------------------------------ column pass
@@ -545,7 +569,7 @@ __device__ __forceinline__ void split_col_line(const SplitCol &a, int b0, int n2
      split_demod<L, N2, NIFO, T>(v, a, b0, n2, t);
      float2 w = __ldg(&a.w0[n2 * (L / 8) + t]);
      const float2 st = __ldg(&a.ws[n2]);
-     split_fft<L, false, T>(v, s, (int)SplitLine<L, false>::BYTES, a.ltw, t, line, [] {});
+     split_fft<L, false, T>(v, s, (int)SplitLine<float2, L, false>::BYTES, a.ltw, t, line, [] {});
      // times W^(n2 k1), k1 = t + m L/8, by recurrence from the base twiddle
      // (seven products: relative error below 1e-6)
      float4 *dst = a.y + (size_t)b0 * (L * N2) + ((size_t)(t / RUN) * N2 + n2) * RUN + t % RUN;
@@ -574,7 +598,121 @@ k_split_col(const __grid_constant__ SplitCol a) {
      extern __shared__ __align__(128) unsigned char smem_raw[];
      const int line = threadIdx.x / (L / 8), t = threadIdx.x % (L / 8);
      split_col_line<L, N2, NIFO, T>(a, blockIdx.y * T, blockIdx.x * split_col_lines<L>() + line, t, line,
-                                    smem_raw + line * (T * SplitLine<L, false>::BYTES));
+                                    smem_raw + line * (T * SplitLine<float2, L, false>::BYTES));
+}
+
+// ------------------------------------------------------------------ column pass, FP64 form
+
+struct Fp64Col {
+     const double2 *xre, *xim;   // operands (a.re, b.re), (a.im, b.im), layout above
+     const double *t1;           // i^2 + 2 i shft_n[i]
+     const TmplParam *tp;
+     double2 *y;
+     const double2 *w0;          // W^(n2 t) [N2][L/8], W = e^{-2 pi i/nfftf}
+     const double2 *ws;          // W^(n2 m L/8) [N2][8]
+     const double2 *ltw;         // pass twiddles of an L-point line
+     int CL;                     // entries per operand column (a multiple of 32, zero past the last sample)
+     int rows;                   // ceil(N / N2)
+     int N2, nifo;
+};
+
+// sin and cos of the spindown phase: reduced by multiples of pi/2 (two
+// fused multiply-adds, exact to 1e-16 for |x| < 2^30 rad; larger phases go to
+// the library), then the Taylor series on [-pi/4, pi/4] up to x^17 and x^16
+// (remainders below 7e-17).  Within 2 ulp of sincos(); the library's version
+// costs the column pass half its time (argument checks and a branch per call).
+__device__ __noinline__ void sincos_large(double x, double *s, double *c) { sincos(x, s, c); }
+
+__device__ __forceinline__ void sincos_spin(double x, double &sn, double &cs) {
+     const double big = 6755399441055744.;   // 1.5*2^52
+     const double kb = fma(x, 0.63661977236758134308, big);
+     const int q = __double2loint(kb);
+     const double k = __dsub_rn(kb, big);
+     double r = fma(-k, 1.5707963267948965580, x);
+     r = fma(-k, 6.1232339957367660359e-17, r);
+     const double z = r * r;
+     double p = fma(z, 1. / 355687428096000., -1. / 1307674368000.);
+     p = fma(z, p, 1. / 6227020800.);
+     p = fma(z, p, -1. / 39916800.);
+     p = fma(z, p, 1. / 362880.);
+     p = fma(z, p, -1. / 5040.);
+     p = fma(z, p, 1. / 120.);
+     p = fma(z, p, -1. / 6.);
+     const double s = fma(r * z, p, r);
+     p = fma(z, 1. / 20922789888000., -1. / 87178291200.);
+     p = fma(z, p, 1. / 479001600.);
+     p = fma(z, p, -1. / 3628800.);
+     p = fma(z, p, 1. / 40320.);
+     p = fma(z, p, -1. / 720.);
+     p = fma(z, p, 1. / 24.);
+     p = fma(z, p, -1. / 2.);
+     const double c = fma(z, p, 1.);
+     const double a = q & 1 ? c : s, b = q & 1 ? s : c;
+     sn = q & 2 ? -a : a;
+     cs = (q + 1) & 2 ? -b : b;
+     if (!(fabs(x) < 1073741824.)) sincos_large(x, &sn, &cs);
+}
+
+// The first MC samples n1 = t + m L/8 of column n2 for template b: the
+// reference's DOUBLE-build spindown_modulation (spinmod.c:490-514), the phase
+// het1*i + spnd*t1 with its products and sum rounded as there.
+template <int L, int NIFO, int MC>
+__device__ __forceinline__ void fp64_demod(D2 (&v)[8], const Fp64Col &a, const TmplParam &P, int n2, int t, int mc) {
+     const int nf = NIFO > 0 ? NIFO : a.nifo;
+     const size_t plane = (size_t)a.N2 * a.CL, o = ((size_t)P.slot * nf * a.N2 + n2) * a.CL + t;
+     const double2 *xre = a.xre + o, *xim = a.xim + o;
+     const double *t1 = a.t1 + o;
+     const double d0 = (double)(a.N2 * t + n2), dm = (double)(a.N2 * (L / 8));
+#pragma unroll
+     for (int m = 0; m < 8; m++) {
+          v[m] = pzero_of<double2>();
+          if (m < (MC > 0 ? MC : mc)) {
+               const double hi = __dmul_rn(P.het1, d0 + m * dm);
+#pragma unroll (NIFO > 0 ? NIFO : 1)
+               for (int d = 0; d < nf; d++) {
+                    const size_t e = d * plane + m * (L / 8);
+                    const double2 re = __ldg(&xre[e]), im = __ldg(&xim[e]);
+                    double sn, cs;
+                    sincos_spin(__dadd_rn(hi, __dmul_rn(P.spnd, __ldg(&t1[e]))), sn, cs);
+                    const double2 C = pdup(cs), S = pdup(sn), M = pdup(-sn);
+                    v[m].re = pfma(re, C, pfma(im, S, v[m].re));
+                    v[m].im = pfma(im, C, pfma(re, M, v[m].im));
+               }
+          }
+     }
+}
+
+// columns per CTA (256 threads, the shortest columns 64)
+template <int L> __host__ __device__ constexpr int fp64_col_lines() { return L >= 512 ? 4 : 8; }
+template <int L> __host__ __device__ constexpr int fp64_col_threads() { return fp64_col_lines<L>() * L / 8; }
+
+// grid (N2 / fp64_col_lines<L>(), templates); 16 warps of 128 registers per SM
+template <int L, int NIFO>
+__global__ void __launch_bounds__(fp64_col_threads<L>(), 512 / fp64_col_threads<L>())
+k_fp64_col(const __grid_constant__ Fp64Col a) {
+     extern __shared__ __align__(128) unsigned char smem_raw[];
+     using G = SplitLine<double2, L, false>;
+     constexpr int R = run_of<double2>;
+     const int line = threadIdx.x / (L / 8), t = threadIdx.x % (L / 8);
+     const int n2 = blockIdx.x * fp64_col_lines<L>() + line, b = blockIdx.y;
+     const TmplParam P = a.tp[b];
+     const int wt = L / 8 >= 32 ? (t & ~31) : 0;   // the warp's first t
+     const int mc = (a.rows - wt + L / 8 - 1) / (L / 8);   // samples m < mc lie before the last row
+     D2 v[1][8];
+     if (mc >= 8) fp64_demod<L, NIFO, 8>(v[0], a, P, n2, t, mc);
+     else if (mc == 6) fp64_demod<L, NIFO, 6>(v[0], a, P, n2, t, mc);
+     else fp64_demod<L, NIFO, 0>(v[0], a, P, n2, t, mc);
+     split_fft<L, false, 1>(v, smem_raw + line * G::BYTES, 0, a.ltw, t, line, [] {});
+     // times W^(n2 k1), k1 = t + m L/8: one product of table entries each
+     const double2 w = __ldg(&a.w0[n2 * (L / 8) + t]);
+     double2 *dst = a.y + ((size_t)b * (L / R) + t / R) * (2 * R * a.N2) + n2 * R + t % R;
+#pragma unroll
+     for (int m = 0; m < 8; m++) {
+          const D2 q = pcmul(v[0][m], m == 0 ? w : cmul_tw(w, __ldg(&a.ws[n2 * 8 + m])));
+          double2 *d = dst + (size_t)m * (L / 8 / R) * (2 * R * a.N2);
+          d[0] = q.re;
+          d[R * a.N2] = q.im;
+     }
 }
 
 // ------------------------------------------------------------------ row pass
@@ -599,10 +737,11 @@ constexpr unsigned ERR_NEED_FULL_F = 4u;   // a batch needs the full F spectra (
 //     threshold; only the end bins c = 0 and RUN-1 of every run go to the
 //     edge ring E[((b*NJ + j)*L + k2)*2 + (c > 0)] (j = CTA index) for the
 //     neighbours of the other CTAs' end-bin candidates.
-struct SplitRow {
-     const float4 *y;
-     const float2 *ltw;
-     float *F;
+template <class V> struct RowArgs {
+     using R1 = decltype(V::x);
+     const V *y;
+     const V *ltw;
+     R1 *F;
      const TmplParam *tp;
      const AaBb *ab;
      int nF, fr0, fr1;
@@ -616,6 +755,8 @@ struct SplitRow {
      int nt;          // templates of the launch
      unsigned *err;
 };
+using SplitRow = RowArgs<float2>;
+using Fp64Row = RowArgs<double2>;
 
 // F = |Fa|^2 * (1/aa) + |Fb|^2 * (1/bb) of the outputs k2 = t + m L/8 of the
 // rows k1, k1 + 1 (k1 = RUN blk + 2c, lanes c of a group of 4 adjacent; v[0]
@@ -708,11 +849,11 @@ __device__ __forceinline__ void split_fstat(const P2 (&v)[2][8], const SplitRow 
 // tid / 4) of the group on rows 2c and 2c + 1; y: element (n2 = 0, row 0)
 // of the CTA's rows, in shared (copied by the caller) or global memory
 template <int L, int N1, bool HALF, class F>
-__device__ __forceinline__ void split_row_block(const SplitRow &a, int b, int blk, int tid, int id, const float4 *y,
+__device__ __forceinline__ void split_row_block(const SplitRow &a, int b, int blk, int tid, int id, const float2 *y,
                                                 bool shared, unsigned char *lines, const F &read) {
-     constexpr int LB = 8 * SplitLine<L, true>::STRIDE;   // bytes between lines in a plane
+     constexpr int LB = 8 * SplitLine<float2, L, true>::STRIDE;   // bytes between lines in a plane
      const int c = tid % (RUN / 2), t = tid / (RUN / 2), odd = t & 1;
-     const float4 *src = y + t * RUN + 2 * c + odd;
+     const float4 *src = reinterpret_cast<const float4 *>(y) + t * RUN + 2 * c + odd;
      P2 v[2][8];
 #pragma unroll
      for (int m = 0; m < 8; m++) {
@@ -723,6 +864,44 @@ __device__ __forceinline__ void split_row_block(const SplitRow &a, int b, int bl
      if (shared) group_sync<L, true>(id);   // the exchanges reuse the rows' memory
      split_fft<L, true, 2>(v, lines + (2 * c + odd) * LB, LB * (1 - 2 * odd), a.ltw, t, id, read);
      split_fstat<L, N1, HALF>(v, a, b, blk * RUN + 2 * c, t);
+}
+
+// F of row k1 in the FP64 form, the full store (see RowArgs), HALF as above
+template <int L, int N1, bool HALF>
+__device__ __forceinline__ void fp64_fstat(const D2 (&v)[8], const Fp64Row &a, int b, int k1, int t) {
+     const AaBb sums = a.ab[a.tp[b].slot];
+     const double ia = 1. / sums.aa, ib = 1. / sums.bb;
+     double *dst = a.F + (size_t)b * a.nF - a.fr0;
+#pragma unroll
+     for (int m = 0; m < (HALF ? 4 : 8); m++) {
+          const int k = k1 + N1 * (t + m * (L / 8));
+          const double2 q = pfma(v[m].re, v[m].re, pmul(v[m].im, v[m].im));
+          const double f = fma(q.x, ia, __dmul_rn(q.y, ib));
+          if (k >= a.fr0 && k <= a.fr1) {
+               dst[k] = f;
+               if (a.cand && !(f < a.thr) && k >= a.fr0 + 1 && k < a.fr1 - 1) {
+                    const unsigned c = atomicAdd(a.cand_cnt, 1u);
+                    if (c < a.cand_cap) a.cand[c] = make_uint2((unsigned)(b + a.boff), (unsigned)k);
+               }
+          }
+     }
+}
+
+// the FP64 form's block: rows k1 = 4 blk + c, one line per thread (c, t) = (tid % 4, tid / 4)
+template <int L, int N1, bool HALF, class F>
+__device__ __forceinline__ void split_row_block(const Fp64Row &a, int b, int blk, int tid, int id, const double2 *y,
+                                                bool, unsigned char *lines, const F &read) {
+     constexpr int R = run_of<double2>;
+     const int c = tid % R, t = tid / R;
+     D2 v[1][8];
+#pragma unroll
+     for (int m = 0; m < 8; m++) {
+          v[0][m].re = y[tid + m * (L / 8 * R)];
+          v[0][m].im = y[L * R + tid + m * (L / 8 * R)];
+     }
+     group_sync<L, true>(id);   // the exchanges reuse the rows' memory
+     split_fft<L, true, 1>(v, lines + c * (SplitLine<double2, L, true>::STRIDE * sizeof(double2)), 0, a.ltw, t, id, read);
+     fp64_fstat<L, N1, HALF>(v[0], a, b, blk * R + c, t);
 }
 
 // The row pass: one persistent CTA per SM.  A row block (RUN rows, one
@@ -740,33 +919,34 @@ __device__ __forceinline__ void split_row_block(const SplitRow &a, int b, int bl
 // user's barrier phase for its own).  A block's copy depends on the block NB
 // before it only, so every wait ends; all are bounded (ERR_STAGE_TIMEOUT in
 // *err), and every copy started is waited for.
-template <int L> __host__ __device__ constexpr int split_row_threads() { return L / 8 * RUN / 2; }   // of a group
+// (FP64: the same block and buffer bytes, four rows, one line per thread.)
+template <int L> __host__ __device__ constexpr int split_row_threads() { return L / 2; }   // of a group
 template <int L> __host__ __device__ constexpr int split_row_groups() { return 512 / split_row_threads<L>(); }
 template <int L> __host__ __device__ constexpr int split_row_bufs() {
      return L >= 1024 ? 1 : split_row_groups<L>() * 3 / 2;
 }
-template <int L> __host__ __device__ constexpr size_t split_row_smem() {
-     return split_row_bufs<L>() * (SplitLine<L, true>::BYTES + sizeof(uint64_t) + sizeof(int));
+template <class V, int L> __host__ __device__ constexpr size_t split_row_smem() {
+     return split_row_bufs<L>() * (SplitLine<V, L, true>::BYTES + sizeof(uint64_t) + sizeof(int));
 }
 
 // makes this thread's earlier accesses to shared memory (and those it has
 // observed) precede the bulk copies it starts next
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-template <int L, int N1, bool HALF>
-__global__ void __launch_bounds__(512, 1) k_split_row(const __grid_constant__ SplitRow a) {
+template <class V, int L, int N1, bool HALF>
+__global__ void __launch_bounds__(512, 1) k_row(const __grid_constant__ RowArgs<V> a) {
      extern __shared__ __align__(128) unsigned char smem_raw[];
      constexpr int GT = split_row_threads<L>(), G = split_row_groups<L>(), NB = split_row_bufs<L>();
-     constexpr unsigned BYTES = SplitLine<L, true>::BYTES, COPY = L * RUN * sizeof(float4);
+     constexpr unsigned BYTES = SplitLine<V, L, true>::BYTES, COPY = 2 * sizeof(V) * L * run_of<V>;
      static_assert(COPY <= BYTES, "a row block must fit in its exchange buffer");
-     constexpr int BPT = N1 / RUN;   // blocks per template
+     constexpr int BPT = N1 / run_of<V>;   // blocks per template
      uint64_t *full = reinterpret_cast<uint64_t *>(smem_raw + NB * BYTES);
      volatile int *issued = reinterpret_cast<volatile int *>(full + NB);   // the block a buffer's copy brings
      const int n = (a.nt * BPT - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // this CTA's blocks
      auto copy = [&](int j) {
           const size_t item = blockIdx.x + (size_t)j * gridDim.x;
           mbar_expect_tx(&full[j % NB], COPY);
-          bulk_load(smem_raw + (j % NB) * BYTES, a.y + item * (L * RUN), COPY, &full[j % NB]);
+          bulk_load(smem_raw + (j % NB) * BYTES, a.y + item * (COPY / sizeof(V)), COPY, &full[j % NB]);
           __threadfence_block();
           issued[j % NB] = j;
      };
@@ -788,7 +968,7 @@ __global__ void __launch_bounds__(512, 1) k_split_row(const __grid_constant__ Sp
           __threadfence_block();
           ok &= probes > 0 && mbar_wait(&full[j % NB], (unsigned)(j / NB) & 1u);
           const int item = (int)blockIdx.x + j * (int)gridDim.x;
-          split_row_block<L, N1, HALF>(a, item / BPT, item % BPT, tid, g, reinterpret_cast<const float4 *>(buf), true, buf,
+          split_row_block<L, N1, HALF>(a, item / BPT, item % BPT, tid, g, reinterpret_cast<const V *>(buf), true, buf,
                                        [&] {
                                             group_sync<L, true>(g);   // the group is done with the buffer
                                             if (tid == 0 && j + NB < n) {
@@ -897,7 +1077,7 @@ k_spinpass(const __grid_constant__ SplitCol col, const __grid_constant__ SplitRo
           spin_item(o, k, b, blk, row);
           if (!row) {
                const int line = threadIdx.x / (L / 8), t = threadIdx.x % (L / 8);
-               unsigned char *s = smem_raw + line * SplitLine<L, false>::BYTES;
+               unsigned char *s = smem_raw + line * SplitLine<float2, L, false>::BYTES;
                // RUN columns, two in turn for each of the CTA's RUN/2 thread groups
                split_col_line<L, L, 2, 1>(col, b, blk * RUN + 2 * line, t, line, s);
                group_sync<L, false>(line);
@@ -909,7 +1089,7 @@ k_spinpass(const __grid_constant__ SplitCol col, const __grid_constant__ SplitRo
                }
                __syncthreads();
                split_row_block<L, L, HALF>(row_, b, blk, threadIdx.x, 0,
-                                                row_.y + ((size_t)b * L + (size_t)blk * RUN) * L, false, smem_raw, [] {});
+                                                row_.y + ((size_t)b * L + (size_t)blk * RUN) * (2 * L), false, smem_raw, [] {});
           }
           __syncthreads();   // the item's shared memory is free; the next ticket is visible
      }
