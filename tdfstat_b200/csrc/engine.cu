@@ -997,6 +997,7 @@ static int launch_fp64_col_n(int nt, const Fp64Col &a, cudaStream_t st) {
      switch (a.nifo) {
      case 1: return launch_fp64_col_c<L, 1>(nt, a, st);
      case 2: return launch_fp64_col_c<L, 2>(nt, a, st);
+     case 3: return launch_fp64_col_c<L, 3>(nt, a, st);
      }
      return launch_fp64_col_c<L, 0>(nt, a, st);
 }

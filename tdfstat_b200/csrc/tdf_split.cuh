@@ -616,13 +616,11 @@ struct Fp64Col {
      int N2, nifo;
 };
 
-// sin and cos of the spindown phase: reduced by multiples of pi/2 (two
-// fused multiply-adds, exact to 1e-16 for |x| < 2^30 rad; larger phases go to
-// the library), then the Taylor series on [-pi/4, pi/4] up to x^17 and x^16
-// (remainders below 7e-17).  Within 2 ulp of sincos(); the library's version
-// costs the column pass half its time (argument checks and a branch per call).
-__device__ __noinline__ void sincos_large(double x, double *s, double *c) { sincos(x, s, c); }
-
+// sin and cos of the spindown phase, |x| < 2^30 rad: reduced by multiples of
+// pi/2 (two fused multiply-adds, exact to 1e-16), then the Taylor series on
+// [-pi/4, pi/4] up to x^17 and x^16 (remainders below 7e-17).  Within 2 ulp of
+// sincos(), without its argument checks and branches, so that several samples'
+// chains are in flight.
 __device__ __forceinline__ void sincos_spin(double x, double &sn, double &cs) {
      const double big = 6755399441055744.;   // 1.5*2^52
      const double kb = fma(x, 0.63661977236758134308, big);
@@ -650,33 +648,109 @@ __device__ __forceinline__ void sincos_spin(double x, double &sn, double &cs) {
      const double a = q & 1 ? c : s, b = q & 1 ? s : c;
      sn = q & 2 ? -a : a;
      cs = (q + 1) & 2 ? -b : b;
-     if (!(fabs(x) < 1073741824.)) sincos_large(x, &sn, &cs);
+}
+__device__ __noinline__ void sincos_large(double x, double *s, double *c) { sincos(x, s, c); }
+
+__device__ __forceinline__ double2 ldgd2_v(const double2 *p) {
+     double2 q;
+     asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(q.x), "=d"(q.y) : "l"(p));
+     return q;
+}
+__device__ __forceinline__ double ldgd_v(const double *p) {
+     double q;
+     asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(q) : "l"(p));
+     return q;
 }
 
-// The first MC samples n1 = t + m L/8 of column n2 for template b: the
-// reference's DOUBLE-build spindown_modulation (spinmod.c:490-514), the phase
-// het1*i + spnd*t1 with its products and sum rounded as there.
+// acc + (re + i im) (c - i s) for both arrays
+__device__ __forceinline__ D2 rot64(const double2 re, const double2 im, double sn, double cs, D2 acc) {
+     const double2 C = pdup(cs), S = pdup(sn), M = pdup(-sn);
+     return D2{pfma(re, C, pfma(im, S, acc.re)), pfma(im, C, pfma(re, M, acc.im))};
+}
+
+// Samples n1 = t + m L/8, m < 8, of column n2 for template P: the reference's
+// DOUBLE-build spindown_modulation (spinmod.c:490-514), the phase het1*i +
+// spnd*t1 with its products and sum rounded as there.  fp64_run() takes the
+// first MC in straight-line code, the operands of the next sample loaded
+// before one is worked on (without: 4.3 of 9 cycles per instruction waiting
+// for loads, 5.0 us per template of 2^18 points); it returns whether a phase
+// reached 2^30 rad.
+struct Fp64In {
+     const double2 *xre, *xim;
+     const double *t1;
+     size_t plane;     // operands of one detector
+     double d0, dm;    // sample number of m = 0, step in m
+};
+
 template <int L, int NIFO, int MC>
-__device__ __forceinline__ void fp64_demod(D2 (&v)[8], const Fp64Col &a, const TmplParam &P, int n2, int t, int mc) {
+__device__ __forceinline__ bool fp64_run(D2 (&v)[8], const Fp64In &in, const TmplParam &P) {
+     double2 re[2][NIFO], im[2][NIFO];
+     double t1[2][NIFO];
+     double far = 0.;
+     auto load = [&](int m) {
+#pragma unroll
+          for (int d = 0; d < NIFO; d++) {
+               const size_t e = d * in.plane + m * (L / 8);
+               re[m & 1][d] = ldgd2_v(&in.xre[e]);
+               im[m & 1][d] = ldgd2_v(&in.xim[e]);
+               t1[m & 1][d] = ldgd_v(&in.t1[e]);
+          }
+     };
+     load(0);
+#pragma unroll
+     for (int m = 0; m < MC; m++) {
+          if (m + 1 < MC) load(m + 1);
+          const double hi = __dmul_rn(P.het1, in.d0 + m * in.dm);
+          v[m] = pzero_of<double2>();
+#pragma unroll
+          for (int d = 0; d < NIFO; d++) {
+               const double x = __dadd_rn(hi, __dmul_rn(P.spnd, t1[m & 1][d]));
+               far = fmax(far, fabs(x));
+               double sn, cs;
+               sincos_spin(x, sn, cs);
+               v[m] = rot64(re[m & 1][d], im[m & 1][d], sn, cs, v[m]);
+          }
+     }
+#pragma unroll
+     for (int m = MC; m < 8; m++) v[m] = pzero_of<double2>();
+     return !(far < 1073741824.);
+}
+
+template <int L, int NIFO>
+__device__ __forceinline__ void fp64_demod(D2 (&v)[8], const Fp64Col &a, const TmplParam &P, int n2, int t) {
      const int nf = NIFO > 0 ? NIFO : a.nifo;
-     const size_t plane = (size_t)a.N2 * a.CL, o = ((size_t)P.slot * nf * a.N2 + n2) * a.CL + t;
-     const double2 *xre = a.xre + o, *xim = a.xim + o;
-     const double *t1 = a.t1 + o;
-     const double d0 = (double)(a.N2 * t + n2), dm = (double)(a.N2 * (L / 8));
+     Fp64In in;
+     in.plane = (size_t)a.N2 * a.CL;
+     const size_t o = ((size_t)P.slot * nf * a.N2 + n2) * a.CL + t;
+     in.xre = a.xre + o;
+     in.xim = a.xim + o;
+     in.t1 = a.t1 + o;
+     in.d0 = (double)(a.N2 * t + n2);
+     in.dm = (double)(a.N2 * (L / 8));
+     const int wt = L / 8 >= 32 ? (t & ~31) : 0;   // the warp's first t
+     const int mc = (a.rows - wt + L / 8 - 1) / (L / 8);   // samples m < mc lie before the last row
+     bool far = true;
+     if constexpr (NIFO > 0) {
+          if (mc >= 8) far = fp64_run<L, NIFO, 8>(v, in, P);
+          else if (mc == 7) far = fp64_run<L, NIFO, 7>(v, in, P);
+          else if (mc == 6) far = fp64_run<L, NIFO, 6>(v, in, P);
+          else if (mc == 5) far = fp64_run<L, NIFO, 5>(v, in, P);
+          else if (mc == 4) far = fp64_run<L, NIFO, 4>(v, in, P);
+     }
+     if (!far) return;
+     // phases past 2^30 rad, few rows, more than three detectors
 #pragma unroll
      for (int m = 0; m < 8; m++) {
           v[m] = pzero_of<double2>();
-          if (m < (MC > 0 ? MC : mc)) {
-               const double hi = __dmul_rn(P.het1, d0 + m * dm);
-#pragma unroll (NIFO > 0 ? NIFO : 1)
+          if (m < mc) {
+               const double hi = __dmul_rn(P.het1, in.d0 + m * in.dm);
                for (int d = 0; d < nf; d++) {
-                    const size_t e = d * plane + m * (L / 8);
-                    const double2 re = __ldg(&xre[e]), im = __ldg(&xim[e]);
+                    const size_t e = d * in.plane + m * (L / 8);
+                    const double x = __dadd_rn(hi, __dmul_rn(P.spnd, __ldg(&in.t1[e])));
                     double sn, cs;
-                    sincos_spin(__dadd_rn(hi, __dmul_rn(P.spnd, __ldg(&t1[e]))), sn, cs);
-                    const double2 C = pdup(cs), S = pdup(sn), M = pdup(-sn);
-                    v[m].re = pfma(re, C, pfma(im, S, v[m].re));
-                    v[m].im = pfma(im, C, pfma(re, M, v[m].im));
+                    if (fabs(x) < 1073741824.) sincos_spin(x, sn, cs);
+                    else sincos_large(x, &sn, &cs);
+                    v[m] = rot64(__ldg(&in.xre[e]), __ldg(&in.xim[e]), sn, cs, v[m]);
                }
           }
      }
@@ -696,12 +770,8 @@ k_fp64_col(const __grid_constant__ Fp64Col a) {
      const int line = threadIdx.x / (L / 8), t = threadIdx.x % (L / 8);
      const int n2 = blockIdx.x * fp64_col_lines<L>() + line, b = blockIdx.y;
      const TmplParam P = a.tp[b];
-     const int wt = L / 8 >= 32 ? (t & ~31) : 0;   // the warp's first t
-     const int mc = (a.rows - wt + L / 8 - 1) / (L / 8);   // samples m < mc lie before the last row
      D2 v[1][8];
-     if (mc >= 8) fp64_demod<L, NIFO, 8>(v[0], a, P, n2, t, mc);
-     else if (mc == 6) fp64_demod<L, NIFO, 6>(v[0], a, P, n2, t, mc);
-     else fp64_demod<L, NIFO, 0>(v[0], a, P, n2, t, mc);
+     fp64_demod<L, NIFO>(v[0], a, P, n2, t);
      split_fft<L, false, 1>(v, smem_raw + line * G::BYTES, 0, a.ltw, t, line, [] {});
      // times W^(n2 k1), k1 = t + m L/8: one product of table entries each
      const double2 w = __ldg(&a.w0[n2 * (L / 8) + t]);
