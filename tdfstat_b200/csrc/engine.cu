@@ -181,27 +181,91 @@ static int launch_row(int L, dim3 grid, const Src &src, const Epi &epi, const cx
 }
 
 template <int L>
-static int launch_interp_mid_L(dim3 grid, const double2 *y, size_t stride, const double2 *tw1, const double2 *tw2,
-                               const double *fac, int N1, StoreFourstep<double, +1, 1> epi, cudaStream_t st) {
-     epi.tab_off = (unsigned)InterpMid<L>::tab_off;
-     const size_t smem = InterpMid<L>::tab_off + StoreFourstep<double, +1, 1>::template table_bytes<2 * L>(epi.N2);
-     auto kern = k_interp_mid<L>;
+static int launch_sky_col_L(int Q, const SkyCol &a, cudaStream_t st) {
+     auto kern = k_sky_col<L>;
+     const size_t smem = fp64_col_lines<L>() * SplitLine<double2, L, false>::BYTES;
      register_sky_kernel((const void *)kern);
      TRY(set_smem(kern, smem));
-     kern<<<grid, 2 * L, smem, st>>>(y, stride, tw1, tw2, fac, N1, epi);
+     kern<<<dim3(a.N2 / fp64_col_lines<L>(), Q), fp64_col_threads<L>(), smem, st>>>(a);
      CUCHK(cudaGetLastError());
      return TDF_OK;
 }
 
-static int launch_interp_mid(int L, dim3 grid, const double2 *y, size_t stride, const double2 *tw1, const double2 *tw2,
-                             const double *fac, int N1, const StoreFourstep<double, +1, 1> &epi, cudaStream_t st) {
+// the partial sums a pair gets: one per warp
+template <int L>
+constexpr int sky_col_warps(int N2) { return N2 / fp64_col_lines<L>() * (fp64_col_threads<L>() / 32); }
+
+static int launch_sky_col(int N1, int Q, const SkyCol &a, int *nblk, cudaStream_t st) {
+     switch (N1) {
+     case 64: *nblk = sky_col_warps<64>(a.N2); return launch_sky_col_L<64>(Q, a, st);
+     case 128: *nblk = sky_col_warps<128>(a.N2); return launch_sky_col_L<128>(Q, a, st);
+     case 256: *nblk = sky_col_warps<256>(a.N2); return launch_sky_col_L<256>(Q, a, st);
+     case 512: *nblk = sky_col_warps<512>(a.N2); return launch_sky_col_L<512>(Q, a, st);
+     case 1024: *nblk = sky_col_warps<1024>(a.N2); return launch_sky_col_L<1024>(Q, a, st);
+     }
+     return set_error(TDF_ERR_UNSUPPORTED, "interpolation column length %d", N1);
+}
+
+template <int L>
+static int launch_sky_mid_L(int Q, const SkyMid &a, cudaStream_t st) {
+     auto kern = k_sky_mid<L>;
+     const size_t smem = SplitLine<double2, 2 * L, true>::BYTES;
+     register_sky_kernel((const void *)kern);
+     TRY(set_smem(kern, smem));
+     kern<<<dim3(a.N1 / run_of<double2>, Q), L, smem, st>>>(a);
+     CUCHK(cudaGetLastError());
+     return TDF_OK;
+}
+
+static int launch_sky_mid(int L, int Q, const SkyMid &a, cudaStream_t st) {
      switch (L) {
-     case 64: return launch_interp_mid_L<64>(grid, y, stride, tw1, tw2, fac, N1, epi, st);
-     case 128: return launch_interp_mid_L<128>(grid, y, stride, tw1, tw2, fac, N1, epi, st);
-     case 256: return launch_interp_mid_L<256>(grid, y, stride, tw1, tw2, fac, N1, epi, st);
-     case 512: return launch_interp_mid_L<512>(grid, y, stride, tw1, tw2, fac, N1, epi, st);
+     case 64: return launch_sky_mid_L<64>(Q, a, st);
+     case 128: return launch_sky_mid_L<128>(Q, a, st);
+     case 256: return launch_sky_mid_L<256>(Q, a, st);
+     case 512: return launch_sky_mid_L<512>(Q, a, st);
      }
      return set_error(TDF_ERR_UNSUPPORTED, "interpolation row length %d", L);
+}
+
+template <class A, int L, int N1, bool HALF>
+static int launch_row_hc(int sms, const A &a, cudaStream_t st) {
+     using V = typename A::V;
+     auto kern = k_row<A, L, N1, HALF>;
+     const size_t smem = split_row_smem<V, L>();
+     if constexpr (std::is_same<A, CoefRow>::value) register_sky_kernel((const void *)kern);
+     TRY(set_smem(kern, smem));
+     kern<<<std::min(sms, a.nt * (N1 / run_of<V>)), 512, smem, st>>>(a);
+     CUCHK(cudaGetLastError());
+     return TDF_OK;
+}
+
+// the spindown row passes keep only bins <= fr1; with fr1 < nfftf/2 = N1*N2/2
+// every kept output has k2 < N2/2
+template <class A, int L, int N1>
+static int launch_row_h(int sms, const A &a, cudaStream_t st) {
+     if constexpr (!std::is_same<A, CoefRow>::value)
+          if ((int64_t)a.fr1 < (int64_t)N1 * L / 2) return launch_row_hc<A, L, N1, true>(sms, a, st);
+     return launch_row_hc<A, L, N1, false>(sms, a, st);
+}
+
+// the FP64 form goes to 2^18 points
+template <class A>
+static int launch_rows(int N1, int N2, int sms, const A &a, cudaStream_t st) {
+     constexpr bool large = !std::is_same<A, Fp64Row>::value;
+     const bool square = N1 == N2;
+     switch (N2) {
+     case 64: return square ? launch_row_h<A, 64, 64>(sms, a, st) : launch_row_h<A, 64, 128>(sms, a, st);
+     case 128: return square ? launch_row_h<A, 128, 128>(sms, a, st) : launch_row_h<A, 128, 256>(sms, a, st);
+     case 256: return square ? launch_row_h<A, 256, 256>(sms, a, st) : launch_row_h<A, 256, 512>(sms, a, st);
+     case 512:
+          if (square) return launch_row_h<A, 512, 512>(sms, a, st);
+          if constexpr (large) return launch_row_h<A, 512, 1024>(sms, a, st);
+          break;
+     case 1024:
+          if constexpr (large) return launch_row_h<A, 1024, 1024>(sms, a, st);
+          break;
+     }
+     return set_error(TDF_ERR_UNSUPPORTED, "row FFT length %d", N2);
 }
 
 // ------------------------------------------------------------------ device buffers
@@ -381,7 +445,7 @@ struct tdf_engine {
      // inputs
      DevBuf fac;      // interpolation: scale and spline prefilter per bin
      // sky stage
-     DevBuf skyp[2], B0, B1, B2, shft, partial, aabb[2];
+     DevBuf skyp[2], B0, B1, B2, partial, aabb[2];
      // operands
      DevBuf xab[2], s2[2], xre[2], xim[2], t1[2];   // per batch slot
      // spindown stage: consecutive resolve groups alternate between lanes,
@@ -543,7 +607,7 @@ static void timing_collect(tdf_engine *e) {
 
 static size_t Wstride(const tdf_engine *e) { return (size_t)e->Ninterp; }
 
-// whether the middle of the interpolation is one kernel (k_interp_mid)
+// whether the interpolation runs on pairs (k_sky_col, k_sky_mid)
 static bool interp_fused(const tdf_engine *e) { return e->Ninterp == 2 * e->nfft && e->nfft <= (1 << 19); }
 
 // ------------------------------------------------------------------ setup
@@ -637,7 +701,6 @@ static int engine_alloc(tdf_engine *e) {
      TRY(e->B0.alloc(Q * 2 * ws * sizeof(double2)));
      TRY(e->B1.alloc(Q * 2 * ws * sizeof(double2)));
      if (!interp_fused(e)) TRY(e->B2.alloc(Q * 2 * ws * sizeof(double2)));
-     TRY(e->shft.alloc(Q * e->Nal * sizeof(double)));
      TRY(e->partial.alloc(Q * (e->nfft / 256) * 2 * sizeof(double)));
      for (int k = 0; k < 2; k++) TRY(e->aabb[k].alloc(Bs * sizeof(AaBb)));
      const bool split = e->form == TDF_FORM_SPLIT;
@@ -704,6 +767,10 @@ static int engine_alloc(tdf_engine *e) {
      TRY(ensure_tparam(e, 1));
      TRY(e->t_nfft.build(e->nfft));
      TRY(e->t_ninterp.build(e->Ninterp));
+     if (interp_fused(e)) {
+          TRY(e->t_nfft.build_split());
+          TRY(e->t_ninterp.build_split());
+     }
      return TDF_OK;
 }
 
@@ -720,7 +787,7 @@ static void engine_free(tdf_engine *e) {
      graphs_clear(e);
      for (SegData &d : e->sdv) d.release();
      DevBuf *bufs[] = {&e->fac, &e->plan_sky, &e->plan_tp, &e->plan_pts, &e->skyp[0],
-                       &e->skyp[1], &e->B0, &e->B1, &e->B2, &e->shft, &e->partial, &e->aabb[0], &e->aabb[1],
+                       &e->skyp[1], &e->B0, &e->B1, &e->B2, &e->partial, &e->aabb[0], &e->aabb[1],
                        &e->xab[0], &e->xab[1], &e->s2[0], &e->s2[1], &e->xre[0], &e->xre[1], &e->xim[0],
                        &e->xim[1], &e->t1[0], &e->t1[1], &e->tparam, &e->trig[0], &e->trig[1],
                        &e->zeroed, &e->linesd};
@@ -871,37 +938,40 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
           CUCHK(cudaMemcpyAsync(e->skyp[sl].p, e->h_sky[sl], npts * sizeof(SkyParam), cudaMemcpyHostToDevice, st));
           dsky = e->skyp[sl].as<SkyParam>();
      }
-     const int nblk = e->nfft / 256;
      const bool split = e->form == TDF_FORM_SPLIT;
-     k_sky_prep<<<dim3(nblk, Q), 256, 0, st>>>(
-          e->S().xdat.as<float>(), e->S().detssb.as<double>(), e->S().cosm.as<double>(), e->S().sinm.as<double>(),
-          dsky, e->S().detp.as<DetParam>(), nifo, e->N, e->nfft, e->Nal, e->S().seg.oms,
-          e->B0.as<double2>(), ws, e->shft.as<double>(), e->partial.as<double>());
-     CUCHK(cudaGetLastError());
-     e->launches++;
-     // Interpolation: forward FFT (nfft) of every (point, detector, a|b),
+     // Interpolation: forward FFT (nfft) of every point, detector and array,
      // inverse FFT (Ninterp) of the spread spectrum times fac, which leaves the
      // spline coefficients of the interpolated series (the first
      // interpftpad*N + 2 and the last are kept)
      const DevBuf *coef;
+     int nblk;   // partial sums per pair
      const FFTTables<double> &t = e->t_nfft, &ti = e->t_ninterp;
-     {
-          LoadNatural<double> pro{e->B0.as<double2>(), t.N2, (int)ws};
-          StoreFourstep<double, -1, 1> epi{e->B1.as<double2>(), t.h(), t.o(), t.N2, (int)ws};
-          TRY((launch_col<double, -1, 1>(t.N1, dim3(t.N2 / LINES, 2 * Q), pro, epi, t.l1(), st)));
-     }
      if (interp_fused(e)) {
-          // B0 -> B1 -> B0 -> B1
-          StoreFourstep<double, +1, 1> epi{e->B0.as<double2>(), ti.h(), ti.o(), ti.N2, (int)ws};
-          TRY(launch_interp_mid(t.N2, dim3(t.N1 / LINES, 2 * Q), e->B1.as<double2>(), ws, t.l2(), ti.l1(),
-                                e->fac.as<double>(), t.N1, epi, st));
-          RowsY<double, 1> src{e->B0.as<double2>(), (int)ws, ti.N2};
-          StoreNatural<double> epi2{e->B1.as<double2>(), ti.N1, (int)ws, e->n2N + 2, e->Ninterp - 1};
-          TRY((launch_row<double, +1, 1>(ti.N2, dim3(ti.N1 / LINES, 2 * Q), src, epi2, ti.l2(), st)));
-          coef = &e->B1;
+          // -> B0 -> B1 -> B0
+          const SkyCol col{e->S().xdat.as<float>(), e->S().detssb.as<double>(), e->S().cosm.as<double>(),
+                           e->S().sinm.as<double>(), dsky, e->S().detp.as<DetParam>(), nifo, e->N, e->Nal, t.N2,
+                           e->S().seg.oms, e->B0.as<double2>(), t.base.as<double2>(), t.step.as<double2>(),
+                           t.ltw1.as<double2>(), e->partial.as<double>()};
+          TRY(launch_sky_col(t.N1, Q, col, &nblk, st));
+          const SkyMid mid{e->B0.as<double2>(), e->B1.as<double2>(), t.ltw2.as<double2>(), ti.ltw1.as<double2>(),
+                           ti.base.as<double2>(), ti.step.as<double2>(), e->fac.as<double>(), t.N1};
+          TRY(launch_sky_mid(t.N2, Q, mid, st));
+          const CoefRow row{e->B1.as<double2>(), ti.ltw2.as<double2>(), e->B0.as<D2>(), ws, e->n2N + 2, e->Ninterp - 1, Q,
+                            reinterpret_cast<unsigned *>(e->counters(sl) + 1)};
+          TRY(launch_rows(ti.N1, ti.N2, e->sms, row, st));
+          coef = &e->B0;
           e->launches += 3;
      } else {
           // B0 -> B1 -> B2 -> B1 -> B0
+          nblk = e->nfft / 256;
+          k_sky_prep<<<dim3(nblk, Q), 256, 0, st>>>(
+               e->S().xdat.as<float>(), e->S().detssb.as<double>(), e->S().cosm.as<double>(), e->S().sinm.as<double>(),
+               dsky, e->S().detp.as<DetParam>(), nifo, e->N, e->nfft, e->Nal, e->S().seg.oms,
+               e->B0.as<double2>(), ws, e->partial.as<double>());
+          CUCHK(cudaGetLastError());
+          LoadNatural<double> nat{e->B0.as<double2>(), t.N2, (int)ws};
+          StoreFourstep<double, -1, 1> epi0{e->B1.as<double2>(), t.h(), t.o(), t.N2, (int)ws};
+          TRY((launch_col<double, -1, 1>(t.N1, dim3(t.N2 / LINES, 2 * Q), nat, epi0, t.l1(), st)));
           RowsY<double, 1> src{e->B1.as<double2>(), (int)ws, t.N2};
           StoreNatural<double> epi2{e->B2.as<double2>(), t.N1, (int)ws, e->nfft, -1};
           TRY((launch_row<double, -1, 1>(t.N2, dim3(t.N1 / LINES, 2 * Q), src, epi2, t.l2(), st)));
@@ -909,14 +979,13 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
           StoreFourstep<double, +1, 1> epi{e->B1.as<double2>(), ti.h(), ti.o(), ti.N2, (int)ws};
           TRY((launch_col<double, +1, 1>(ti.N1, dim3(ti.N2 / LINES, 2 * Q), pro, epi, ti.l1(), st)));
           RowsY<double, 1> src2{e->B1.as<double2>(), (int)ws, ti.N2};
-          StoreNatural<double> epi3{e->B0.as<double2>(), ti.N1, (int)ws, e->n2N + 2, e->Ninterp - 1};
+          StorePairs epi3{e->B0.as<double>(), ti.N1, (int)ws, e->n2N + 2, e->Ninterp - 1};
           TRY((launch_row<double, +1, 1>(ti.N2, dim3(ti.N1 / LINES, 2 * Q), src2, epi3, ti.l2(), st)));
           coef = &e->B0;
-          e->launches += 4;
+          e->launches += 5;
      }
-     const SplintIn in{coef->as<double2>(), ws, e->shft.as<double>(), dsky, e->S().detssb.as<double>(),
-                       e->S().detp.as<DetParam>(), e->Nal, e->N, e->n2N, e->Ninterp, e->S().seg.interpftpad, nifo,
-                       e->partial.as<double>(), nblk, e->aabb[sl].as<AaBb>()};
+     const SplintIn in{coef->as<D2>(), ws, dsky, e->S().detssb.as<double>(), e->S().detp.as<DetParam>(), e->N, e->n2N,
+                       e->Ninterp, e->S().seg.interpftpad, nifo, e->partial.as<double>(), nblk, e->aabb[sl].as<AaBb>()};
      const int N2 = split ? e->t_f32.N2 : e->t_f64.N2;
      const dim3 g(N2 / 32, ((e->N + N2 - 1) / N2 + 7) / 8, Q);
      auto splint = split ? k_splint<true> : k_splint<false>;
@@ -1012,42 +1081,6 @@ static int launch_fp64_col(int N1, int nt, const Fp64Col &a, cudaStream_t st) {
      return set_error(TDF_ERR_UNSUPPORTED, "FP64 column FFT length %d", N1);
 }
 
-template <class V, int L, int N1, bool HALF>
-static int launch_row_hc(int sms, const RowArgs<V> &a, cudaStream_t st) {
-     auto kern = k_row<V, L, N1, HALF>;
-     const size_t smem = split_row_smem<V, L>();
-     TRY(set_smem(kern, smem));
-     kern<<<std::min(sms, a.nt * (N1 / run_of<V>)), 512, smem, st>>>(a);
-     CUCHK(cudaGetLastError());
-     return TDF_OK;
-}
-
-// the row pass keeps only bins <= fr1; with fr1 < nfftf/2 = N1*N2/2 every
-// kept output has k2 < N2/2
-template <class V, int L, int N1>
-static int launch_row_h(int sms, const RowArgs<V> &a, cudaStream_t st) {
-     return (int64_t)a.fr1 < (int64_t)N1 * L / 2 ? launch_row_hc<V, L, N1, true>(sms, a, st)
-                                                 : launch_row_hc<V, L, N1, false>(sms, a, st);
-}
-
-template <class V>
-static int launch_spin_row(int N1, int N2, int sms, const RowArgs<V> &a, cudaStream_t st) {
-     const bool square = N1 == N2;
-     switch (N2) {
-     case 64: return square ? launch_row_h<V, 64, 64>(sms, a, st) : launch_row_h<V, 64, 128>(sms, a, st);
-     case 128: return square ? launch_row_h<V, 128, 128>(sms, a, st) : launch_row_h<V, 128, 256>(sms, a, st);
-     case 256: return square ? launch_row_h<V, 256, 256>(sms, a, st) : launch_row_h<V, 256, 512>(sms, a, st);
-     case 512:
-          if (square) return launch_row_h<V, 512, 512>(sms, a, st);
-          if constexpr (sizeof(V) == 8) return launch_row_h<V, 512, 1024>(sms, a, st);
-          break;
-     case 1024:
-          if constexpr (sizeof(V) == 8) return launch_row_h<V, 1024, 1024>(sms, a, st);
-          break;
-     }
-     return set_error(TDF_ERR_UNSUPPORTED, "row FFT length %d", N2);
-}
-
 // The two split-form passes of nt templates as one ordered launch of
 // persistent CTAs (k_spinpass), for N1 = N2 = L (nfftf 2^16, 2^18) and two
 // detectors; ctl (2 + nt words) is zeroed first, on the same stream.
@@ -1133,7 +1166,7 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
           TRY(launch_split_col(t.N1, t.N2, e->sms, col, st));
           if (e->timing) timing_end(e, tev, KT_COL, nt, st);
           tev = e->timing ? timing_begin(e, st) : (size_t)-1;
-          TRY(launch_spin_row(t.N1, t.N2, e->sms, row, st));
+          TRY(launch_rows(t.N1, t.N2, e->sms, row, st));
      } else {
           const Fp64Col col{e->xre[e->cur].as<double2>(), e->xim[e->cur].as<double2>(), e->t1[e->cur].as<double>(), ctp,
                             Ln.Ybuf.as<double2>(), t.base.template as<double2>(), t.step.template as<double2>(),
@@ -1145,7 +1178,7 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
                             Ln.Fbuf.as<double>() + (size_t)boff * e->nF, ctp, e->aabb[e->cur].as<AaBb>(), e->nF,
                             e->opts.fr[0], e->opts.fr[1], e->opts.thr, blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G,
                             e->cand_cap, boff, nullptr, nullptr, nt, errw};
-          TRY(launch_spin_row(t.N1, t.N2, e->sms, row, st));
+          TRY(launch_rows(t.N1, t.N2, e->sms, row, st));
      }
      if (e->timing) timing_end(e, tev, KT_ROW, nt, st);
      e->launches += 2;

@@ -1,16 +1,8 @@
 // tdf_kernels.cuh -- the hot-path kernels of the job_core() chain
 // (search/network/openmp/jobcore.c:193-630) other than the FFT passes:
 //
-//   sky stage (FP64, once per sky point and detector)
-//     k_sky_prep      modvir + barycentric shift + phase modulation
-//                     (settings.c:254-294, jobcore.c:283-312), zero padding,
-//                     partial sums of aa^2, bb^2 (jobcore.c:373-391)
-//     (FFT passes)    interpolation by FFT to twice the rate, delivering the
-//                     coefficients of the cubic spline through the series
-//     k_splint        natural-spline evaluation at 2(i - shftf[i])
-//                     (auxi.c:93-169), division by sig2, conversion to the
-//                     spindown operands; aa, bb network sums (FLOAT_TYPE
-//                     emulation per form)
+//   sky stage (FP64, once per sky point and detector): tdf_sky.cuh
+//   injection: k_signal, k_add_signal
 //   spindown stage (once per template)
 //     (the passes: tdf_split.cuh)
 //     DemodSplit      column-pass prologue of the allocation-free entry point:
@@ -72,76 +64,19 @@ constexpr double M_PI_D = 3.14159265358979323846;
 // |xDat[t]| <= DBL_MIN
 __device__ __forceinline__ void modvir_at(const DetParam &D, double sinal, double cosal, double sindel, double cosdel,
                                           double cosm, double sinm, float x, double &aa, double &bb) {
-     aa = 0.;
-     bb = 0.;
-     if (fabs((double)x) > DBL_MIN) {
-          const double cosalfr = cosal * D.cphir + sinal * D.sphir;
-          const double sinalfr = sinal * D.cphir - cosal * D.sphir;
-          const double c2d = cosdel * cosdel, c2sd = sindel * cosdel;
-          const double c = cosalfr * cosm + sinalfr * sinm;
-          const double s = sinalfr * cosm - cosalfr * sinm;
-          const double c2s = 2. * c * c, cs = c * s;
-          aa = D.amod[0] * (2. - c2d) * c2s + D.amod[1] * (2. - c2d) * 2. * cs +
-               D.amod[2] * c2sd * c + D.amod[3] * c2sd * s - D.amod[0] * (2. - c2d) + D.amod[4] * c2d;
-          bb = D.amod[5] * sindel * c2s + D.amod[6] * sindel * 2. * cs +
-               D.amod[7] * cosdel * c + D.amod[8] * cosdel * s - D.amod[5] * sindel;
-     }
-}
-
-// grid (ceil(nfft/256), Q = npts*nifo), 256 threads
-__global__ void __launch_bounds__(256) k_sky_prep(
-     const float *__restrict__ xdat, const double *__restrict__ detssb,
-     const double *__restrict__ cosm, const double *__restrict__ sinm,
-     const SkyParam *__restrict__ sp, const DetParam *__restrict__ dp,
-     int nifo, int N, int nfft, int Nal, double oms,
-     double2 *__restrict__ W, size_t Wstride, double *__restrict__ shft, double *__restrict__ partial)
-{
-     const int q = blockIdx.y, p = q / nifo, d = q % nifo;
-     const int i = blockIdx.x * 256 + threadIdx.x;
-     double a2 = 0., b2 = 0.;
-     if (i < nfft) {
-          double2 xa = make_double2(0., 0.), xb = make_double2(0., 0.);
-          if (i < N) {
-               const SkyParam S = sp[p];
-               const DetParam &D = dp[d];
-               const float x = xdat[(size_t)d * Nal + i];
-               double aa, bb;
-               modvir_at(D, S.sinalt, S.cosalt, S.sindelt, S.cosdelt, cosm[i], sinm[i], x, aa, bb);
-               const double *e = detssb + (size_t)d * 3 * N;
-               // shift and phase without FMA contraction: the phase reaches
-               // ~1e5 rad, so its rounding must follow the reference's
-               const double sh = __dadd_rn(__dadd_rn(__dmul_rn(S.nS0, e[3 * (size_t)i]), __dmul_rn(S.nS1, e[3 * (size_t)i + 1])),
-                                           __dmul_rn(S.nS2, e[3 * (size_t)i + 2]));
-               shft[(size_t)q * Nal + i] = sh;
-               const double di = (double)i;
-               const double phase = __dadd_rn(__dmul_rn(S.het0, di), __dmul_rn(oms, sh));
-               double sn, cn;
-               sincos(phase, &sn, &cn);
-               const double ra = (double)x * aa, rb = (double)x * bb;
-               xa = make_double2(ra * cn, ra * -sn);
-               xb = make_double2(rb * cn, rb * -sn);
-               a2 = aa * aa;
-               b2 = bb * bb;
-          }
-          W[((size_t)q * 2 + 0) * Wstride + i] = xa;
-          W[((size_t)q * 2 + 1) * Wstride + i] = xb;
-     }
-     // block partial sums of aa^2, bb^2
-     __shared__ double ra_[8], rb_[8];
-#pragma unroll
-     for (int o = 16; o > 0; o >>= 1) {
-          a2 += __shfl_down_sync(0xffffffffu, a2, o);
-          b2 += __shfl_down_sync(0xffffffffu, b2, o);
-     }
-     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-     if (l == 0) { ra_[w] = a2; rb_[w] = b2; }
-     __syncthreads();
-     if (threadIdx.x == 0) {
-          double sa = 0., sb = 0.;
-          for (int k = 0; k < 8; k++) { sa += ra_[k]; sb += rb_[k]; }
-          partial[((size_t)q * gridDim.x + blockIdx.x) * 2 + 0] = sa;
-          partial[((size_t)q * gridDim.x + blockIdx.x) * 2 + 1] = sb;
-     }
+     const double cosalfr = cosal * D.cphir + sinal * D.sphir;
+     const double sinalfr = sinal * D.cphir - cosal * D.sphir;
+     const double c2d = cosdel * cosdel, c2sd = sindel * cosdel;
+     const double c = cosalfr * cosm + sinalfr * sinm;
+     const double s = sinalfr * cosm - cosalfr * sinm;
+     const double c2s = 2. * c * c, cs = c * s;
+     const bool on = fabs((double)x) > DBL_MIN;
+     aa = D.amod[0] * (2. - c2d) * c2s + D.amod[1] * (2. - c2d) * 2. * cs +
+          D.amod[2] * c2sd * c + D.amod[3] * c2sd * s - D.amod[0] * (2. - c2d) + D.amod[4] * c2d;
+     bb = D.amod[5] * sindel * c2s + D.amod[6] * sindel * 2. * cs +
+          D.amod[7] * cosdel * c + D.amod[8] * cosdel * s - D.amod[5] * sindel;
+     aa = on ? aa : 0.;
+     bb = on ? bb : 0.;
 }
 
 // ------------------------------------------------------------------ injection
@@ -209,184 +144,6 @@ __global__ void __launch_bounds__(256) k_add_signal(float *__restrict__ xdat, co
      if (i >= N) return;
      float *x = xdat + (size_t)d * Nal + i;
      if (*x != 0.f) *x = (float)__dadd_rn((double)*x, __dmul_rn(h0, s[(size_t)d * N + i]));
-}
-
-// aa = sum_n sum_i aa_n^2/sig2_n (jobcore.c:373-386) of sky point p by one CTA
-// of 256 threads; each detector's partials reduced by a fixed tree
-// (reproducible), then accumulated over detectors into FLOAT_TYPE as the
-// reference build does.
-__device__ void sky_sums(const double *__restrict__ partial, int nblk, const DetParam *__restrict__ dp, int nifo, int p,
-                         AaBb *__restrict__ out)
-{
-     __shared__ double ra[256], rb[256];
-     double aa = 0., bb = 0.;
-     float aaf = 0.f, bbf = 0.f;
-     for (int d = 0; d < nifo; d++) {
-          const double *pp = partial + (size_t)(p * nifo + d) * nblk * 2;
-          double sa = 0., sb = 0.;
-          for (int k = threadIdx.x; k < nblk; k += 256) { sa += pp[2 * k]; sb += pp[2 * k + 1]; }
-          ra[threadIdx.x] = sa;
-          rb[threadIdx.x] = sb;
-          __syncthreads();
-          for (int o = 128; o > 0; o >>= 1) {
-               if (threadIdx.x < o) {
-                    ra[threadIdx.x] += ra[threadIdx.x + o];
-                    rb[threadIdx.x] += rb[threadIdx.x + o];
-               }
-               __syncthreads();
-          }
-          sa = ra[0];
-          sb = rb[0];
-          __syncthreads();
-          aa += sa / dp[d].sig2;
-          bb += sb / dp[d].sig2;
-          aaf = (float)((double)aaf + sa / dp[d].sig2);
-          bbf = (float)((double)bbf + sb / dp[d].sig2);
-     }
-     if (threadIdx.x == 0) {
-          out[p].aa = aa;
-          out[p].bb = bb;
-          out[p].aaf = aaf;
-          out[p].bbf = bbf;
-     }
-}
-
-// The natural cubic spline (auxi.c:93-169) through y[0..n-1], evaluated at x
-// from B-spline coefficients: with t = x - k, k = floor(x),
-//   s(x) = sum_j w_j(t) c[k + j], j = -1..2 (the four cubic B-spline weights).
-// c0 holds the coefficients of the periodic spline of the whole interpolated
-// series (period np, a power of two), which the inverse FFT delivers; its
-// second derivatives at the ends of the data, D0 and Dn, are not zero.  The
-// natural spline has c[k] = c0[k] + a z^k + b z^(n-1-k), z = sqrt(3) - 2: both
-// added terms leave every y[k] as it is (z + 4 + 1/z = 0) and change the
-// second derivative by -6 times themselves, so
-//   a + b z^(n-1) = D0/6,  a z^(n-1) + b = Dn/6.
-// They decay by 0.27 per sample and are left out 64 samples from the ends
-// (1e-37).  Replaces two recurrence sweeps over every series (u, y2): half of
-// the sky stage's passes over memory.
-__device__ __forceinline__ double zpow(int e) {
-     constexpr double z = -0.26794919243112270647, iz = -3.7320508075688772935;
-     if (e > 128) return 0.;   // below 1e-73
-     double p = 1.;
-     for (int i = 0; i < e; i++) p *= z;
-     for (int i = 0; i > e; i--) p *= iz;
-     return p;
-}
-
-__device__ __forceinline__ double2 splint_eval(const double2 *__restrict__ c0, int n, int np, double x)
-{
-     if (x < 0 || x > n - 1) return make_double2(0., 0.);
-     const int k = (int)floor(x);
-     const double t = x - k, u = 1. - t;
-     const double2 cm = c0[(k - 1) & (np - 1)], ca = c0[k], cb = c0[(k + 1) & (np - 1)], cd = c0[(k + 2) & (np - 1)];
-     const double wm = u * u * u * (1. / 6.), wd = t * t * t * (1. / 6.);
-     const double wa = (2. / 3.) - t * t * (1. - .5 * t), wb = (2. / 3.) - u * u * (1. - .5 * u);
-     double2 r = make_double2(wm * cm.x + wa * ca.x + wb * cb.x + wd * cd.x, wm * cm.y + wa * ca.y + wb * cb.y + wd * cd.y);
-     if (k < 64 || k > n - 66) {
-          constexpr double z = -0.26794919243112270647;
-          const double2 l0 = c0[np - 1], l1 = c0[0], l2 = c0[1 & (np - 1)];
-          const double2 r0 = c0[(n - 2) & (np - 1)], r1 = c0[n - 1], r2 = c0[n & (np - 1)];
-          const double2 D0 = make_double2((l0.x - 2. * l1.x + l2.x) / 6., (l0.y - 2. * l1.y + l2.y) / 6.);
-          const double2 Dn = make_double2((r0.x - 2. * r1.x + r2.x) / 6., (r0.y - 2. * r1.y + r2.y) / 6.);
-          const double w = zpow(n - 1), q = 1. / (1. - w * w);
-          const double ga = zpow(k - 1) * (wm + z * (wa + z * (wb + z * wd))) * q;               // of a
-          const double gb = zpow(n - 3 - k) * (wd + z * (wb + z * (wa + z * wm))) * q;           // of b
-          r.x += ga * (D0.x - w * Dn.x) + gb * (Dn.x - w * D0.x);
-          r.y += ga * (D0.y - w * Dn.y) + gb * (Dn.y - w * D0.y);
-     }
-     return r;
-}
-
-// shft_n[0] as k_sky_prep forms shft_n[i]
-__device__ __forceinline__ double shft0(const SkyParam &S, const double *e) {
-     return __dadd_rn(__dadd_rn(__dmul_rn(S.nS0, e[0]), __dmul_rn(S.nS1, e[1])), __dmul_rn(S.nS2, e[2]));
-}
-
-// The inputs of the resampling (jobcore.c:314-370): spline coefficients C of
-// array (q, a|b), q = point*nifo + det, `stride` apart; and the sums' partials
-// (the CTA of a point's first tile forms its aa and bb).
-struct SplintIn {
-     const double2 *C;
-     size_t stride;
-     const double *shft;      // [q][Nal]
-     const SkyParam *sp;
-     const double *detssb;
-     const DetParam *dp;
-     int Nal, N, n, np, interpftpad, nifo;
-     const double *partial;
-     int nblk;
-     AaBb *ab;
-};
-
-// xDatm{a,b}[i] = splint(interpftpad*(i - (shft[i] - shft[0])))/sig2
-__device__ __forceinline__ void splint_at(const SplintIn &I, int q, int i, double sh, double sh1, double s2, double2 &a,
-                                          double2 &b) {
-     const double x = I.interpftpad * (i - __dsub_rn(sh, sh1));
-     const double2 va = splint_eval(I.C + ((size_t)q * 2) * I.stride, I.n, I.np, x);
-     const double2 vb = splint_eval(I.C + ((size_t)q * 2 + 1) * I.stride, I.n, I.np, x);
-     a = make_double2(va.x / s2, va.y / s2);
-     b = make_double2(vb.x / s2, vb.y / s2);
-}
-
-struct D4 {
-     double x, y, z, w;
-};
-
-// Operands in the column layout of tdf_split.cuh: with i = N2*n1 + n2, split
-// form (SPLIT)
-//   xab[(q*N2 + n2)*CL + n1] = (a.re, b.re, a.im, b.im) in FP32
-//   s2[((p*N2 + n2)*CL + n1)*nifo + d] = 2 i shft[i]
-// FP64 form
-//   xre, xim[(q*N2 + n2)*CL + n1] = (a.re, b.re), (a.im, b.im)
-//   t1[(q*N2 + n2)*CL + n1] = i^2 + 2 i shft[i]
-// A CTA takes a tile of 32 columns and 8 rows: it reads along i (32
-// consecutive samples per warp) and, through shared memory, writes 8
-// consecutive n1 of a column (128 bytes) at a time.
-// grid (N2/32, ceil(ceil(N/N2)/8), Q), 256 threads
-template <bool SPLIT>
-__global__ void __launch_bounds__(256) k_splint(const __grid_constant__ SplintIn I, int N2, int CL,
-                                                float4 *__restrict__ xab, float *__restrict__ s2out,
-                                                double2 *__restrict__ xre, double2 *__restrict__ xim,
-                                                double *__restrict__ t1)
-{
-     using X = typename std::conditional<SPLIT, float4, D4>::type;
-     using S = typename std::conditional<SPLIT, float, double>::type;
-     __shared__ X xs[32][9];
-     __shared__ S ss[32][9];
-     const int q = blockIdx.z, p = q / I.nifo, d = q % I.nifo;
-     if (blockIdx.x == 0 && blockIdx.y == 0 && d == 0) sky_sums(I.partial, I.nblk, I.dp, I.nifo, p, I.ab);
-     {
-          const int c = threadIdx.x % 32, r = threadIdx.x / 32;
-          const int i = N2 * (blockIdx.y * 8 + r) + blockIdx.x * 32 + c;
-          if (i < I.N) {
-               const double sh = I.shft[(size_t)q * I.Nal + i];
-               double2 a, b;
-               splint_at(I, q, i, sh, shft0(I.sp[p], I.detssb + (size_t)d * 3 * I.N), I.dp[d].sig2, a, b);
-               X v;
-               v.x = a.x;
-               v.y = b.x;
-               v.z = a.y;
-               v.w = b.y;
-               xs[c][r] = v;
-               const double di = (double)i, e = __dmul_rn((double)(2 * i), sh);
-               ss[c][r] = SPLIT ? (S)(float)e : (S)__dadd_rn(__dmul_rn(di, di), e);
-          }
-     }
-     __syncthreads();
-     const int c = threadIdx.x / 8, r = threadIdx.x % 8;
-     const int n1 = blockIdx.y * 8 + r, n2 = blockIdx.x * 32 + c;
-     if (N2 * n1 + n2 < I.N) {
-          const size_t o = ((size_t)q * N2 + n2) * CL + n1;
-          const X v = xs[c][r];
-          if constexpr (SPLIT) {
-               xab[o] = v;
-               s2out[(((size_t)p * N2 + n2) * CL + n1) * I.nifo + d] = ss[c][r];
-          } else {
-               xre[o] = make_double2(v.x, v.y);
-               xim[o] = make_double2(v.z, v.w);
-               t1[o] = ss[c][r];
-          }
-     }
 }
 
 // ------------------------------------------------------------------ spindown stage
@@ -553,6 +310,7 @@ struct StoreFstat {
 }  // namespace tdf
 
 #include "tdf_split.cuh"
+#include "tdf_sky.cuh"
 
 namespace tdf {
 

@@ -212,6 +212,27 @@ struct StoreNatural {
      }
 };
 
+// The same with arrays 2q and 2q + 1 interleaved: element k of the pair q is
+// (re, re, im, im) at x[(q*N + k)*4].
+struct StorePairs {
+     double *x;
+     int N1;
+     int N;
+     int nkeep, klast;
+     template <int L>
+     __device__ __forceinline__ void store(const double2 (&v)[1][8], int b, int k1, int t) const {
+          double *dst = x + (size_t)(b >> 1) * N * 4 + (b & 1);
+#pragma unroll
+          for (int m = 0; m < 8; m++) {
+               const int k = k1 + N1 * (t + m * (L / 8));
+               if (k < nkeep || k == klast) {
+                    dst[(size_t)k * 4] = v[0][m].x;
+                    dst[(size_t)k * 4 + 2] = v[0][m].y;
+               }
+          }
+     }
+};
+
 // Column-pass prologue: plain load of x[N2*n1 + n2] from natural-order arrays
 // of stride N (arrays already zero-padded to N).
 template <typename T>
@@ -265,68 +286,6 @@ struct LoadShuffled {
 __global__ void k_interp_factor(double *fac, int n, double dw, double scale) {
      const int k = blockIdx.x * blockDim.x + threadIdx.x;
      if (k < n) fac[k] = scale * 6. / (4. + 2. * cospi(dw * k));
-}
-
-// The middle of the interpolation (FP64) when Ninterp = 2 nfft: the rows of
-// the forward transform and the columns of the inverse one in one kernel.
-// With nfft = N1*L (rows of L points) the inverse transform has N1 columns of
-// 2L points, and the outputs X[k1 + N1*k2] of forward row k1 are exactly the
-// inputs of inverse column k1: the spectrum never goes to memory (one kernel
-// and one write and read of every spectrum less).  Half of an inverse
-// column's inputs are the zero padding.
-// CTA: LINES rows k1, 2L threads; the forward rows use half of them.
-// grid (N1/LINES, arrays)
-template <int L>
-struct InterpMid {
-     static constexpr size_t line_bytes = sizeof(double2) * LINES * (size_t)LineGeom<double, 2 * L>::STRIDE;
-     static constexpr size_t tab_off = sizeof(double2) * 3 * L + line_bytes;   // four-step tables of the epilogue
-};
-
-template <int L>
-__global__ void __launch_bounds__(2 * L, 512 / L)
-k_interp_mid(const double2 *__restrict__ y, size_t stride, const double2 *__restrict__ tw1,
-             const double2 *__restrict__ tw2, const double *__restrict__ fac, int N1,
-             StoreFourstep<double, +1, 1> epi) {
-     extern __shared__ __align__(128) unsigned char smem_raw[];
-     double2 *t1 = reinterpret_cast<double2 *>(smem_raw), *t2 = t1 + L, *lines = t2 + 2 * L;
-     const int c = threadIdx.x % LINES, t = threadIdx.x / LINES;
-     const int k1 = blockIdx.x * LINES + c;
-     const bool fwd = t < L / 8;
-     double2 v[1][8];
-     if (fwd) {
-          const double2 *r = y + (size_t)blockIdx.y * stride + (size_t)k1 * L + t;
-#pragma unroll
-          for (int m = 0; m < 8; m++) v[0][m] = r[m * (L / 8)];
-     }
-     load_table<double>(t1, tw1, L);
-     load_table<double>(t2, tw2, 2 * L);
-     epi.template load_tables<2 * L>(smem_raw);
-     double2 *s[1] = {lines + c * LineGeom<double, 2 * L>::STRIDE};
-     __syncthreads();
-     line_fft<double, L, -1, 1>(v, s, t1, t, fwd);
-     if (fwd) {
-          const int nfft = N1 * L;
-#pragma unroll
-          for (int m = 0; m < 8; m++) {
-               const int k2 = t + m * (L / 8), k = k1 + N1 * k2;
-               s[0][pad8(k2)] = cscale(v[0][m], __ldg(&fac[k <= nfft / 2 ? k : nfft - k]));
-          }
-     }
-     __syncthreads();
-     // input n1 = t + m L/4 of the inverse column: bins k2 = n1 below nfft/2,
-     // k2 = n1 - L in the top quarter; bin nfft/2 itself (row 0) on the low side
-#pragma unroll
-     for (int m = 0; m < 8; m++) {
-          const int n1 = t + m * (L / 4);
-          v[0][m] = m < 2 ? s[0][pad8(n1)] : (m >= 6 ? s[0][pad8(n1 - L)] : make_double2(0., 0.));
-     }
-     if (k1 == 0 && t == 0) {
-          v[0][2] = v[0][6];
-          v[0][6] = make_double2(0., 0.);
-     }
-     __syncthreads();
-     line_fft<double, 2 * L, +1, 1>(v, s, t2, t);
-     epi.template store<2 * L>(v, blockIdx.y, k1, t, smem_raw);
 }
 
 }  // namespace tdf

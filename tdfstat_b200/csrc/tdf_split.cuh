@@ -3,7 +3,7 @@
 //   k_split_col /
 //   k_fp64_col    demodulation of a template's samples, the N1-point FFTs of
 //                 its columns and the four-step twiddle -> Y
-//   k_row<V>      the N2-point FFTs of the rows of Y and the F-statistic
+//   k_row         the N2-point FFTs of the rows of Y and the F-statistic
 //   k_spinpass    split form: both as one ordered launch of persistent CTAs
 //                 (opt-in)
 //
@@ -256,61 +256,70 @@ template <class V, int L, bool ROW> struct SplitLine {
      }
 };
 
-// the L/8 threads of one column, or the L/2 of a row block, wait for one another
+// the NT threads of a group (one column, one row block) wait for one another
 // (id: the group's number within the CTA)
-template <int L, bool ROW>
+template <int NT>
 __device__ __forceinline__ void group_sync(int id) {
-     constexpr int n = ROW ? L / 2 : L / 8;
-     if (n <= 32)
+     if (NT <= 32)
           __syncwarp();
      else
-          asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "n"(n > 32 ? n : 32) : "memory");
+          asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "n"(NT > 32 ? NT : 32) : "memory");
 }
+// threads of a group: L/8 per column, four times that per row block
+template <int L, bool ROW> constexpr int group_threads = ROW ? L / 2 : L / 8;
 
-// The passes from span NS on, the data and the pass's twiddles at hand.
-// s: the memory of the thread's first line, the k-th one's `next` bytes
-// further; read() is called when the thread has read the last exchange.
-template <int L, bool ROW, int NS, int T, class V, class F>
+// The passes from span NS on, the data and the pass's twiddles at hand, by a
+// group of NT threads.  s: the memory of the thread's first line, the k-th
+// one's `next` bytes further; read() is called when the thread has read the
+// last exchange; threads with active = false only keep the group's barriers.
+template <int L, bool ROW, int NS, int NT, int T, class V, class F>
 __device__ __forceinline__ void line_pass(PV<V> (&v)[T][8], unsigned char *s, int next, const V *__restrict__ ltw,
-                                          int t, int id, const PassTw<V, L, (NS > 1 ? NS : 8)> &tw, const F &read) {
+                                          int t, int id, const PassTw<V, L, (NS > 1 ? NS : 8)> &tw, const F &read,
+                                          bool active) {
      using G = SplitLine<V, L, ROW>;
      constexpr int R = pass_radix(L, NS);
-     if constexpr (NS > 1) ppass_twiddle<L, NS, T>(v, tw);
+     if (active) {
+          if constexpr (NS > 1) ppass_twiddle<L, NS, T>(v, tw);
 #pragma unroll
-     for (int k = 0; k < T; k++) ppass_dft<R>(v[k]);
+          for (int k = 0; k < T; k++) ppass_dft<R>(v[k]);
+     }
      if constexpr (NS * R < L) {
           // (R = 8 here) output r of butterfly t goes to (t/NS)*8 NS + t%NS + r NS
           constexpr int RN = pass_radix(L, NS * 8);
           PassTw<V, L, NS * 8> tn;
-          tn.load(ltw, t);
-          if constexpr (NS > 1) group_sync<L, ROW>(id);   // the previous exchange is read
+          if (active) tn.load(ltw, t);
+          if constexpr (NS > 1) group_sync<NT>(id);   // the previous exchange is read
           const int d = NS == 1 ? G::dist(8) * t : G::pos((t / NS) * NS * 8 + (t % NS));
+          if (active) {
 #pragma unroll
-          for (int k = 0; k < T; k++)
+               for (int k = 0; k < T; k++)
 #pragma unroll
-               for (int r = 0; r < 8; r++) G::put(s + k * next, d + (NS == 1 ? r : r * G::dist(NS)), v[k][r]);
-          group_sync<L, ROW>(id);
+                    for (int r = 0; r < 8; r++) G::put(s + k * next, d + (NS == 1 ? r : r * G::dist(NS)), v[k][r]);
+          }
+          group_sync<NT>(id);
+          if (active) {
 #pragma unroll
-          for (int k = 0; k < T; k++)
+               for (int k = 0; k < T; k++)
 #pragma unroll
-               for (int q = 0; q < 8 / RN; q++) {
-                    const int d1 = G::pos(t + q * (L / 8));
+                    for (int q = 0; q < 8 / RN; q++) {
+                         const int d1 = G::pos(t + q * (L / 8));
 #pragma unroll
-                    for (int r = 0; r < RN; r++)
-                         v[k][q + r * (8 / RN)] = G::get(s + k * next, d1 + r * G::dist(L / RN));
-               }
+                         for (int r = 0; r < RN; r++)
+                              v[k][q + r * (8 / RN)] = G::get(s + k * next, d1 + r * G::dist(L / RN));
+                    }
+          }
           if constexpr (NS * 8 * RN >= L) read();
-          line_pass<L, ROW, NS * 8, T>(v, s, next, ltw, t, id, tn, read);
+          line_pass<L, ROW, NS * 8, NT, T>(v, s, next, ltw, t, id, tn, read, active);
      }
 }
 
 // L-point forward transform of a thread's T lines: thread t holds
 // x[t + m L/8] on entry and X[t + m L/8] on exit.  The lines' shared memory
 // must be free on entry.
-template <int L, bool ROW, int T, class V, class F>
+template <int L, bool ROW, int T, int NT = group_threads<L, ROW>, class V, class F>
 __device__ __forceinline__ void split_fft(PV<V> (&v)[T][8], unsigned char *s, int next, const V *__restrict__ ltw,
-                                          int t, int id, const F &read) {
-     line_pass<L, ROW, 1, T>(v, s, next, ltw, t, id, PassTw<V, L, 8>(), read);
+                                          int t, int id, const F &read, bool active = true) {
+     line_pass<L, ROW, 1, NT, T>(v, s, next, ltw, t, id, PassTw<V, L, 8>(), read, active);
 }
 
 // ------------------------------------------------------------------ column pass
@@ -807,7 +816,8 @@ constexpr unsigned ERR_NEED_FULL_F = 4u;   // a batch needs the full F spectra (
 //     threshold; only the end bins c = 0 and RUN-1 of every run go to the
 //     edge ring E[((b*NJ + j)*L + k2)*2 + (c > 0)] (j = CTA index) for the
 //     neighbours of the other CTAs' end-bin candidates.
-template <class V> struct RowArgs {
+template <class W> struct RowArgs {
+     using V = W;
      using R1 = decltype(V::x);
      const V *y;
      const V *ltw;
@@ -931,7 +941,7 @@ __device__ __forceinline__ void split_row_block(const SplitRow &a, int b, int bl
           v[0][m] = unpack4(shared ? p[0] : __ldcg(p));
           v[1][m] = unpack4(shared ? p[1 - 2 * odd] : __ldcg(p + 1 - 2 * odd));
      }
-     if (shared) group_sync<L, true>(id);   // the exchanges reuse the rows' memory
+     if (shared) group_sync<L / 2>(id);   // the exchanges reuse the rows' memory
      split_fft<L, true, 2>(v, lines + (2 * c + odd) * LB, LB * (1 - 2 * odd), a.ltw, t, id, read);
      split_fstat<L, N1, HALF>(v, a, b, blk * RUN + 2 * c, t);
 }
@@ -969,7 +979,7 @@ __device__ __forceinline__ void split_row_block(const Fp64Row &a, int b, int blk
           v[0][m].re = y[tid + m * (L / 8 * R)];
           v[0][m].im = y[L * R + tid + m * (L / 8 * R)];
      }
-     group_sync<L, true>(id);   // the exchanges reuse the rows' memory
+     group_sync<L / 2>(id);   // the exchanges reuse the rows' memory
      split_fft<L, true, 1>(v, lines + c * (SplitLine<double2, L, true>::STRIDE * sizeof(double2)), 0, a.ltw, t, id, read);
      fp64_fstat<L, N1, HALF>(v[0], a, b, blk * R + c, t);
 }
@@ -1003,8 +1013,9 @@ template <class V, int L> __host__ __device__ constexpr size_t split_row_smem() 
 // observed) precede the bulk copies it starts next
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-template <class V, int L, int N1, bool HALF>
-__global__ void __launch_bounds__(512, 1) k_row(const __grid_constant__ RowArgs<V> a) {
+template <class A, int L, int N1, bool HALF>
+__global__ void __launch_bounds__(512, 1) k_row(const __grid_constant__ A a) {
+     using V = typename A::V;
      extern __shared__ __align__(128) unsigned char smem_raw[];
      constexpr int GT = split_row_threads<L>(), G = split_row_groups<L>(), NB = split_row_bufs<L>();
      constexpr unsigned BYTES = SplitLine<V, L, true>::BYTES, COPY = 2 * sizeof(V) * L * run_of<V>;
@@ -1040,7 +1051,7 @@ __global__ void __launch_bounds__(512, 1) k_row(const __grid_constant__ RowArgs<
           const int item = (int)blockIdx.x + j * (int)gridDim.x;
           split_row_block<L, N1, HALF>(a, item / BPT, item % BPT, tid, g, reinterpret_cast<const V *>(buf), true, buf,
                                        [&] {
-                                            group_sync<L, true>(g);   // the group is done with the buffer
+                                            group_sync<L / 2>(g);   // the group is done with the buffer
                                             if (tid == 0 && j + NB < n) {
                                                  fence_proxy_async();
                                                  copy(j + NB);
@@ -1150,7 +1161,7 @@ k_spinpass(const __grid_constant__ SplitCol col, const __grid_constant__ SplitRo
                unsigned char *s = smem_raw + line * SplitLine<float2, L, false>::BYTES;
                // RUN columns, two in turn for each of the CTA's RUN/2 thread groups
                split_col_line<L, L, 2, 1>(col, b, blk * RUN + 2 * line, t, line, s);
-               group_sync<L, false>(line);
+               group_sync<L / 8>(line);
                split_col_line<L, L, 2, 1>(col, b, blk * RUN + 2 * line + 1, t, line, s);
                pend = b;
           } else {
