@@ -1217,7 +1217,7 @@ static int run_resolve(tdf_engine *e, int l, const TmplParam *dtp, int ntg) {
      if (blocks) {
           k_block_means<T><<<dim3(e->nblk_mu, ntg), 256, 0, st>>>(Ln.Fbuf.as<T>(), e->nF, e->nblk_mu, Ln.mubuf.as<T>());
           CUCHK(cudaGetLastError());
-          dim3 g((e->nF + 255) / 256, ntg);
+          dim3 g((e->nF + 2047) / 2048, ntg);
           if (split) k_threshold<T, false><<<g, 256, 0, st>>>(Ln.Fbuf.as<T>(), Ln.mubuf.as<T>(), A);
           else k_threshold<T, true><<<g, 256, 0, st>>>(Ln.Fbuf.as<T>(), Ln.mubuf.as<T>(), A);
           e->launches += 2;

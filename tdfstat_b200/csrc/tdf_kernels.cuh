@@ -15,6 +15,7 @@
 #pragma once
 
 #include <float.h>
+#include <math_constants.h>
 
 #include <type_traits>
 
@@ -321,8 +322,11 @@ __global__ void k_block_means(const T *__restrict__ F, int nF, int nblk, T *__re
 {
      const int j = blockIdx.x, b = blockIdx.y;
      const T *src = F + (size_t)b * nF + (size_t)j * 4096;
-     T s = 0;
-     for (int k = threadIdx.x; k < 4096; k += 256) s += src[k];
+     T v[16], s = 0;
+#pragma unroll
+     for (int k = 0; k < 16; k++) v[k] = src[threadIdx.x + 256 * k];   // all in flight
+#pragma unroll
+     for (int k = 0; k < 16; k++) s += v[k];
      __shared__ T red[256];
      red[threadIdx.x] = s;
      __syncthreads();
@@ -502,15 +506,30 @@ __global__ void __launch_bounds__(256) k_resolve_sparse(ThrArgs A, SparseArgs S)
      }
 }
 
-// Full scan of every bin (used with the blocks_avg normalisation).
-// grid (ceil((fr1-fr0+1)/256), ntmpl), 256 threads
+// Full scan of every bin (used with the blocks_avg normalisation).  A thread
+// looks at 8 bins of one block, so that a CTA has one mean; bins clearly below
+// the threshold are passed over by a product instead of the exact quotient
+// (one bin per thread and a division each took 29 us for 64 templates of
+// 127,000 bins, 12 us now).  grid (ceil(nF/2048), ntmpl), 256 threads
 template <typename T, bool FP64>
 __global__ void __launch_bounds__(256) k_threshold(const T *__restrict__ F, const T *__restrict__ mu, ThrArgs A)
 {
-     const int b = blockIdx.y;
-     const int i = A.fr0 + blockIdx.x * 256 + threadIdx.x;
-     if (i < A.fr0 + 1 || i >= A.fr1 - 1) return;
-     threshold_bin<T, FP64>(F, mu, A, b, i);
+     const int b = blockIdx.y, r0 = blockIdx.x * 2048 + threadIdx.x;
+     const T *Fb = F + (size_t)b * A.nF;
+     T lim = -CUDART_INF;
+     if (A.thr > 0.) {
+          const int j = (blockIdx.x * 2048) >> 12;
+          lim = (T)(A.thr * (1. - 1e-5) * (mu && j < A.nblk ? (double)mu[(size_t)b * A.nblk + j] : 1.));
+     }
+     T v[8];
+#pragma unroll
+     for (int k = 0; k < 8; k++) v[k] = r0 + 256 * k < A.nF ? Fb[r0 + 256 * k] : lim;
+#pragma unroll
+     for (int k = 0; k < 8; k++) {
+          const int i = A.fr0 + r0 + 256 * k;
+          if (i < A.fr0 + 1 || i >= A.fr1 - 1 || v[k] < lim) continue;
+          threshold_bin<T, FP64>(F, mu, A, b, i);
+     }
 }
 
 }  // namespace tdf
