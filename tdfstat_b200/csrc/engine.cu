@@ -234,7 +234,7 @@ static int launch_row_hc(int sms, const A &a, cudaStream_t st) {
      const size_t smem = split_row_smem<V, L>();
      if constexpr (std::is_same<A, CoefRow>::value) register_sky_kernel((const void *)kern);
      TRY(set_smem(kern, smem));
-     kern<<<std::min(sms, a.nt * (N1 / run_of<V>)), 512, smem, st>>>(a);
+     kern<<<std::min(sms, a.nt * (N1 / run_of<V>)), split_row_cta<V, L>(), smem, st>>>(a);
      CUCHK(cudaGetLastError());
      return TDF_OK;
 }

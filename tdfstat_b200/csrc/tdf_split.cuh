@@ -1001,9 +1001,13 @@ __device__ __forceinline__ void split_row_block(const Fp64Row &a, int b, int blk
 // *err), and every copy started is waited for.
 // (FP64: the same block and buffer bytes, four rows, one line per thread.)
 template <int L> __host__ __device__ constexpr int split_row_threads() { return L / 2; }   // of a group
-template <int L> __host__ __device__ constexpr int split_row_groups() { return 512 / split_row_threads<L>(); }
+// Half as many buffers again as 512 threads' groups fit the shared memory; with
+// short lines the split form gives one of the spare ones to a fifth group (96
+// registers): 2^17 points 0.561 -> 0.547 us per template, 2^16 0.341 -> 0.326.
+template <class V, int L> __host__ __device__ constexpr int split_row_cta() { return sizeof(V) == 8 && L == 256 ? 640 : 512; }
+template <class V, int L> __host__ __device__ constexpr int split_row_groups() { return split_row_cta<V, L>() / split_row_threads<L>(); }
 template <int L> __host__ __device__ constexpr int split_row_bufs() {
-     return L >= 1024 ? 1 : split_row_groups<L>() * 3 / 2;
+     return L >= 1024 ? 1 : 512 / split_row_threads<L>() * 3 / 2;
 }
 template <class V, int L> __host__ __device__ constexpr size_t split_row_smem() {
      return split_row_bufs<L>() * (SplitLine<V, L, true>::BYTES + sizeof(uint64_t) + sizeof(int));
@@ -1014,10 +1018,10 @@ template <class V, int L> __host__ __device__ constexpr size_t split_row_smem() 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
 template <class A, int L, int N1, bool HALF>
-__global__ void __launch_bounds__(512, 1) k_row(const __grid_constant__ A a) {
+__global__ void __launch_bounds__(split_row_cta<typename A::V, L>(), 1) k_row(const __grid_constant__ A a) {
      using V = typename A::V;
      extern __shared__ __align__(128) unsigned char smem_raw[];
-     constexpr int GT = split_row_threads<L>(), G = split_row_groups<L>(), NB = split_row_bufs<L>();
+     constexpr int GT = split_row_threads<L>(), G = split_row_groups<V, L>(), NB = split_row_bufs<L>();
      constexpr unsigned BYTES = SplitLine<V, L, true>::BYTES, COPY = 2 * sizeof(V) * L * run_of<V>;
      static_assert(COPY <= BYTES, "a row block must fit in its exchange buffer");
      constexpr int BPT = N1 / run_of<V>;   // blocks per template
@@ -1134,7 +1138,7 @@ __device__ __forceinline__ bool wait_count(const unsigned *p, unsigned target, i
 // (Y is written and read within the launch: the row blocks read it with
 // __ldcg, past L1.)
 template <int L, bool HALF>
-__global__ void __launch_bounds__(split_row_threads<L>(), split_row_groups<L>())
+__global__ void __launch_bounds__(split_row_threads<L>(), 512 / split_row_threads<L>())
 k_spinpass(const __grid_constant__ SplitCol col, const __grid_constant__ SplitRow row_, const __grid_constant__ SpinOrder o) {
      extern __shared__ __align__(128) unsigned char smem_raw[];
      __shared__ unsigned s_tk[2];
