@@ -183,7 +183,7 @@ static int launch_row(int L, dim3 grid, const Src &src, const Epi &epi, const cx
 template <int L>
 static int launch_sky_col_L(int Q, const SkyCol &a, cudaStream_t st) {
      auto kern = k_sky_col<L>;
-     const size_t smem = fp64_col_lines<L>() * SplitLine<double2, L, false>::BYTES;
+     const size_t smem = fp64_col_lines<L>() / run_of<double2> * SplitLine<double2, L, true>::BYTES;
      register_sky_kernel((const void *)kern);
      TRY(set_smem(kern, smem));
      kern<<<dim3(a.N2 / fp64_col_lines<L>(), Q), fp64_col_threads<L>(), smem, st>>>(a);

@@ -89,14 +89,20 @@ __device__ __forceinline__ void store_col64(D2 (&v)[8], double2 *y, const double
      }
 }
 
+// The lanes of a warp are four columns at eight rows: the samples come in
+// natural order, so a load touches eight rows' lines of 128 bytes.  With the 32
+// rows of one column per warp it touched 32 (L1 49% busy on them, the load
+// queue full): 75 -> 65 us per sky point of 2^18 samples for the whole stage,
+// 31.2 -> 28.5 for 2^17, 15.0 -> 13.9 for 2^16 (two detectors, batches).
 // grid (N2 / fp64_col_lines<L>(), Q)
 template <int L>
 __global__ void __launch_bounds__(fp64_col_threads<L>(), 512 / fp64_col_threads<L>())
 k_sky_col(const __grid_constant__ SkyCol a) {
      extern __shared__ __align__(128) unsigned char smem_raw[];
-     using G = SplitLine<double2, L, false>;
-     const int line = threadIdx.x / (L / 8), t = threadIdx.x % (L / 8);
-     const int n2 = blockIdx.x * fp64_col_lines<L>() + line, q = blockIdx.y, d = q % a.nifo;
+     using G = SplitLine<double2, L, true>;
+     constexpr int R = run_of<double2>;
+     const int grp = threadIdx.x / (L / 2), c = threadIdx.x % R, t = threadIdx.x % (L / 2) / R;
+     const int n2 = blockIdx.x * fp64_col_lines<L>() + grp * R + c, q = blockIdx.y, d = q % a.nifo;
      const SkyParam S = a.sp[q / a.nifo];
      const DetParam &D = a.dp[d];
      D2 v[1][8];
@@ -136,7 +142,7 @@ k_sky_col(const __grid_constant__ SkyCol a) {
           p[0] = s2;
           p[1] = t2;
      }
-     split_fft<L, false, 1>(v, smem_raw + line * G::BYTES, 0, a.ltw, t, line, [] {});
+     split_fft<L, true, 1>(v, smem_raw + grp * G::BYTES + c * (G::STRIDE * sizeof(double2)), 0, a.ltw, t, grp, [] {});
      store_col64<L>(v[0], a.y + (size_t)q * (2 * L * a.N2), a.w0, a.ws, a.N2, n2, t);
 }
 
