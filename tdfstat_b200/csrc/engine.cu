@@ -1122,7 +1122,7 @@ static bool spin_fused(const tdf_engine *e, int N1, int N2) {
 }
 
 template <typename T>
-static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt) {
+static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt, bool select) {
      cudaStream_t st = lane_stream(e, l);
      tdf_engine::Lane &Ln = e->ln[l];
      const FFTTables<T> *tb;
@@ -1142,7 +1142,7 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
                              e->N, e->CL, (e->N + t.N2 - 1) / t.N2, e->nifo, nt};
           SplitRow row{Ln.Ybuf.as<float2>(), t.ltw2.template as<float2>(), Ln.Fbuf.as<float>() + (size_t)boff * e->nF,
                        ctp, e->aabb[e->cur].as<AaBb>(), e->nF, e->opts.fr[0], e->opts.fr[1], e->opts.thr,
-                       blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff, nullptr, nullptr, nt, errw};
+                       blocks || !select ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff, nullptr, nullptr, nt, errw};
           if (e->sparse_now) {
                row.cand = nullptr;
                row.E = Ln.Ebuf.as<float>();
@@ -1176,7 +1176,7 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
           tev = e->timing ? timing_begin(e, st) : (size_t)-1;
           const Fp64Row row{Ln.Ybuf.as<double2>(), t.ltw2.template as<double2>(),
                             Ln.Fbuf.as<double>() + (size_t)boff * e->nF, ctp, e->aabb[e->cur].as<AaBb>(), e->nF,
-                            e->opts.fr[0], e->opts.fr[1], e->opts.thr, blocks ? nullptr : Ln.cand.as<uint2>(), tcnt + G,
+                            e->opts.fr[0], e->opts.fr[1], e->opts.thr, blocks || !select ? nullptr : Ln.cand.as<uint2>(), tcnt + G,
                             e->cand_cap, boff, nullptr, nullptr, nt, errw};
           TRY(launch_rows(t.N1, t.N2, e->sms, row, st));
      }
@@ -1188,14 +1188,16 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt)
 // Trigger selection for the ntg templates of a resolve group (starting at
 // dtp; their F spectra fill the F ring in order): the candidate bins the row
 // passes collected, or, with blocks_avg, block means and a scan of every bin.
+// select = false: the block means only.
 template <typename T>
-static int run_resolve(tdf_engine *e, int l, const TmplParam *dtp, int ntg) {
+static int run_resolve(tdf_engine *e, int l, const TmplParam *dtp, int ntg, bool select) {
      cudaStream_t st = lane_stream(e, l);
      tdf_engine::Lane &Ln = e->ln[l];
      const bool split = std::is_same<T, float>::value;
      const unsigned G = (unsigned)group_templates(e);
      unsigned *tcnt = Ln.tcnt;
      const bool blocks = e->opts.blocks_avg && e->nblk_mu > 0;
+     if (!select && !blocks) return TDF_OK;
      unsigned long long *cnt = e->counters(e->cur);
      ThrArgs A;
      A.nF = e->nF;
@@ -1217,10 +1219,17 @@ static int run_resolve(tdf_engine *e, int l, const TmplParam *dtp, int ntg) {
      if (blocks) {
           k_block_means<T><<<dim3(e->nblk_mu, ntg), 256, 0, st>>>(Ln.Fbuf.as<T>(), e->nF, e->nblk_mu, Ln.mubuf.as<T>());
           CUCHK(cudaGetLastError());
+          e->launches++;
+     }
+     if (!select) {
+          if (e->timing) timing_end(e, tev, KT_THR, ntg, st);
+          return TDF_OK;
+     }
+     if (blocks) {
           dim3 g((e->nF + 2047) / 2048, ntg);
           if (split) k_threshold<T, false><<<g, 256, 0, st>>>(Ln.Fbuf.as<T>(), Ln.mubuf.as<T>(), A);
           else k_threshold<T, true><<<g, 256, 0, st>>>(Ln.Fbuf.as<T>(), Ln.mubuf.as<T>(), A);
-          e->launches += 2;
+          e->launches++;
      } else if (split && e->sparse_now) {
           SparseArgs S{Ln.Ebuf.as<float>(), Ln.cand.as<uint4>(), tcnt + G, e->cand_cap, e->t_f32.N1, e->t_f32.N2};
           k_resolve_sparse<<<64, 256, 0, st>>>(A, S);
@@ -1241,7 +1250,9 @@ static int run_resolve(tdf_engine *e, int l, const TmplParam *dtp, int ntg) {
 // chunks, group k on lane k % nlanes.  Lanes 1.. start after everything
 // queued on the engine stream so far (sky stage, template upload) and the
 // engine stream waits for them at the end, so callers see one ordered stream.
-static int run_templates(tdf_engine *e, const TmplParam *dtp, int nt) {
+// select = false leaves the F spectra (and block means) without looking for
+// triggers, for callers that read the spectrum itself.
+static int run_templates(tdf_engine *e, const TmplParam *dtp, int nt, bool select = true) {
      const int G = group_templates(e);
      const int ngroups = (nt + G - 1) / G;
      // per-kernel event timing measures kernels one after another: one lane
@@ -1256,11 +1267,11 @@ static int run_templates(tdf_engine *e, const TmplParam *dtp, int nt) {
           const int ntg = std::min(G, nt - g0);
           for (int ci = 0; ci * e->Tc < ntg; ci++) {
                const int n = std::min(e->Tc, ntg - ci * e->Tc);
-               if (e->form == TDF_FORM_SPLIT) TRY(run_chunk<float>(e, l, dtp + g0, ci, n));
-               else TRY(run_chunk<double>(e, l, dtp + g0, ci, n));
+               if (e->form == TDF_FORM_SPLIT) TRY(run_chunk<float>(e, l, dtp + g0, ci, n, select));
+               else TRY(run_chunk<double>(e, l, dtp + g0, ci, n, select));
           }
-          if (e->form == TDF_FORM_SPLIT) TRY(run_resolve<float>(e, l, dtp + g0, ntg));
-          else TRY(run_resolve<double>(e, l, dtp + g0, ntg));
+          if (e->form == TDF_FORM_SPLIT) TRY(run_resolve<float>(e, l, dtp + g0, ntg, select));
+          else TRY(run_resolve<double>(e, l, dtp + g0, ntg, select));
      }
      for (int l = 1; l < lanes; l++) {
           CUCHK(cudaEventRecord(e->join_ev[l], e->lane_own[l]));
@@ -2369,7 +2380,7 @@ int tdf_fstat_spectrum(tdf_engine *e, int32_t pm, float mm, float nn, float ss, 
      CUCHK(cudaMemsetAsync(e->zeroed.p, 0, e->zeroed.bytes, e->stream));
      CUCHK(cudaStreamWaitEvent(e->stream, e->sky_done[0], 0));
      e->sparse_now = false;   // the spectrum itself is the output: the full F store
-     TRY(run_templates(e, e->tparam.as<TmplParam>(), 1));
+     TRY(run_templates(e, e->tparam.as<TmplParam>(), 1, false));
      CUCHK(cudaMemcpyAsync(e->h_cnt, e->counters(0), 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->stream));
      const int n = e->nF;
      const bool split = e->form == TDF_FORM_SPLIT;
