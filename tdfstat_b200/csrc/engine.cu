@@ -538,7 +538,8 @@ struct tdf_engine {
      // (k_spinpass), a template's rows fuse_lag templates behind its
      // columns (TDF_FUSE_LAG=n).  Off by default: its spectra stay in L2,
      // but each row block's wait and the publishing fences sit on the CTA's
-     // critical path, and it measured ~10% slower than the two launches.
+     // critical path: 2.96 us per template of 2^18 points and two detectors
+     // against 2.37 for the two launches.
      bool fused = false;
      int fuse_lag = 3;
      // split form: the row pass keeps F on the chip and hands over only the
@@ -2719,7 +2720,7 @@ extern "C" int tdf_fstat_operands_static(const void *d_xab, const float *d_s2, i
      StoreFourstep<float, -1, 2> epi{Y, hi, lo, N2, nfftf};
      TRY((launch_col<float, -1, 2>(N1, dim3(N2 / LINES, 1), pro, epi, line1, st)));
      RowsY<float, 2> src{Y, nfftf, N2};
-     StoreFstat<float> epi2{d_F, tp, ab, fr1 - fr0 + 1, fr0, fr1, N1, 0.0, nullptr, nullptr, 0u, 0};
+     StoreFstat epi2{d_F, tp, ab, fr1 - fr0 + 1, fr0, fr1, N1};
      TRY((launch_row<float, -1, 2>(N2, dim3(N1 / LINES, 1), src, epi2, line2, st)));
      return TDF_OK;
 }

@@ -1,6 +1,6 @@
 // tdf_bulk.cuh -- asynchronous copies global -> shared memory for sm_100a:
 // bulk copies (cp.async.bulk, no multicast) completing on mbarrier
-// transaction counts, bounded waits on those barriers, and per-thread copies.
+// transaction counts, and bounded waits on those barriers.
 #pragma once
 
 #include <stdint.h>
@@ -56,20 +56,6 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned b
              smem_addr(dst)),
          "l"((uint64_t)src), "r"(bytes), "r"(smem_addr(bar))
          : "memory");
-}
-
-// Per-thread asynchronous copies global -> shared memory of 16 or 8 bytes
-// (both addresses aligned to the size), waited for with cp_async_wait_all();
-// a thread's copies are all in flight at once and hold no registers.
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"((uint64_t)src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"((uint64_t)src) : "memory");
-}
-// the calling thread's copies have landed (other threads' need a barrier)
-__device__ __forceinline__ void cp_async_wait_all() {
-     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 }  // namespace tdf

@@ -206,39 +206,33 @@ __device__ __forceinline__ void pass_load(cx<T> (&v)[8], const cx<T> *s, int t) 
 
 // Full L-point transform of NA lines that share a thread: v[a] in/out as in
 // the register convention above; s[a] = the line's shared memory; tw = line
-// twiddle table (shared).  All threads of the CTA must call it (barriers);
-// those that hold no butterfly of the line pass active = false.
+// twiddle table (shared).  All threads of the CTA must call it (barriers).
 template <typename T, int L, int SIGN, int NA>
-__device__ __forceinline__ void line_fft(cx<T> (&v)[NA][8], cx<T> *const (&s)[NA], const cx<T> *tw, int t,
-                                         bool active = true) {
+__device__ __forceinline__ void line_fft(cx<T> (&v)[NA][8], cx<T> *const (&s)[NA], const cx<T> *tw, int t) {
      using G = LineGeom<T, L>;
      int NS = 1;
 #pragma unroll
      for (int p = 0; p < G::P8; p++) {
           const bool last = (p == G::P8 - 1) && (G::RL == 1);
-          if (active) {
-               if (p > 0) pass_twiddle<T, L, 8, SIGN, NA>(v, tw, t, NS);
+          if (p > 0) pass_twiddle<T, L, 8, SIGN, NA>(v, tw, t, NS);
 #pragma unroll
-               for (int a = 0; a < NA; a++) {
-                    pass_dft<8, SIGN>(v[a]);
-                    if (!last) pass_store<T, L, 8>(v[a], s[a], t, NS);
-               }
+          for (int a = 0; a < NA; a++) {
+               pass_dft<8, SIGN>(v[a]);
+               if (!last) pass_store<T, L, 8>(v[a], s[a], t, NS);
           }
           if (!last) {
                __syncthreads();
                constexpr int RN = 8;   // next pass radix (8, or the last radix)
-               if (active) {
 #pragma unroll
-                    for (int a = 0; a < NA; a++) {
-                         if (p + 1 < G::P8) pass_load<T, L, RN>(v[a], s[a], t);
-                         else pass_load<T, L, (G::RL > 1 ? G::RL : 8)>(v[a], s[a], t);
-                    }
+               for (int a = 0; a < NA; a++) {
+                    if (p + 1 < G::P8) pass_load<T, L, RN>(v[a], s[a], t);
+                    else pass_load<T, L, (G::RL > 1 ? G::RL : 8)>(v[a], s[a], t);
                }
                __syncthreads();
           }
           NS *= 8;
      }
-     if (G::RL > 1 && active) {
+     if (G::RL > 1) {
           constexpr int RR = G::RL > 1 ? G::RL : 2;
           pass_twiddle<T, L, RR, SIGN, NA>(v, tw, t, NS);
 #pragma unroll
@@ -252,16 +246,8 @@ __device__ __forceinline__ void load_table(cx<T> *dst, const cx<T> *__restrict__
      for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
-// Four-step twiddle W_N^m (forward sign), m < N <= 2^20, from two tables:
-// hi[m >> 10] * lo[m & 1023].
-template <typename T>
-__device__ __forceinline__ cx<T> fourstep_twiddle(const cx<T> *__restrict__ hi, const cx<T> *__restrict__ lo, int m) {
-     cx<T> a = __ldg(&hi[m >> 10]);
-     cx<T> b = __ldg(&lo[m & 1023]);
-     return cmul(a, b);
-}
-
-// the same from copies of the tables in shared memory
+// Four-step twiddle W_N^m (forward sign), m < N <= 2^20, from two tables in
+// shared memory: hi[m >> 10] * lo[m & 1023].
 template <typename T>
 __device__ __forceinline__ cx<T> fourstep_twiddle_smem(const cx<T> *hi, const cx<T> *lo, int m) {
      return cmul(hi[m >> 10], lo[m & 1023]);

@@ -266,44 +266,20 @@ struct DemodSplit {
      }
 };
 
-template <typename T> __device__ __forceinline__ T aa_of(const AaBb &ab);
-template <> __device__ __forceinline__ float aa_of<float>(const AaBb &ab) { return ab.aaf; }
-template <> __device__ __forceinline__ double aa_of<double>(const AaBb &ab) { return ab.aa; }
-template <typename T> __device__ __forceinline__ T bb_of(const AaBb &ab);
-template <> __device__ __forceinline__ float bb_of<float>(const AaBb &ab) { return ab.bbf; }
-template <> __device__ __forceinline__ double bb_of<double>(const AaBb &ab) { return ab.bb; }
-
-// Row-pass epilogue of the spindown FFT: F[k] over [fr0, fr1].  With a
-// candidate list (cand != nullptr) it also appends every bin of the MAX_ALG 3
-// loop range [fr0+1, fr1-2] whose F passes the threshold test, so that the
-// local-maximum rule only has to look at those bins afterwards.
-template <typename T>
+// Row-pass epilogue of the allocation-free entry point: F[k] over [fr0, fr1].
 struct StoreFstat {
-     T *F;
+     float *F;
      const TmplParam *tp;
      const AaBb *ab;
      int nF, fr0, fr1, N1;
-     double thr;
-     uint2 *cand;
-     unsigned *cand_cnt;
-     unsigned cand_cap;
-     int boff;        // index of this chunk's first template within its resolve group
      template <int L>
-     __device__ __forceinline__ void store(const cx<T> (&v)[2][8], int b, int k1, int t) const {
+     __device__ __forceinline__ void store(const float2 (&v)[2][8], int b, int k1, int t) const {
           const AaBb s = ab[tp[b].slot];
-          const T aa = aa_of<T>(s), bb = bb_of<T>(s);
-          T *dst = F + (size_t)b * nF - fr0;
+          float *dst = F + (size_t)b * nF - fr0;
 #pragma unroll
           for (int m = 0; m < 8; m++) {
                const int k = k1 + N1 * (t + m * (L / 8));
-               if (k >= fr0 && k <= fr1) {
-                    const T f = cnorm(v[0][m]) / aa + cnorm(v[1][m]) / bb;
-                    dst[k] = f;
-                    if (cand && !(f < thr) && k >= fr0 + 1 && k < fr1 - 1) {
-                         const unsigned c = atomicAdd(cand_cnt, 1u);
-                         if (c < cand_cap) cand[c] = make_uint2((unsigned)(b + boff), (unsigned)k);
-                    }
-               }
+               if (k >= fr0 && k <= fr1) dst[k] = cnorm(v[0][m]) / s.aaf + cnorm(v[1][m]) / s.bbf;
           }
      }
 };

@@ -157,14 +157,6 @@ __host__ __device__ constexpr int pass_powers(int R) { return R == 8 ? 3 : (R ==
 __host__ __device__ constexpr int ltw_offset(int L, int NS) {
      return NS <= 8 ? 0 : ltw_offset(L, NS / 8) + pass_powers(pass_radix(L, NS / 8)) * (NS / 8);
 }
-__host__ __device__ constexpr int ltw_entries(int L) {
-     int n = 0, NS = 8;
-     while (NS < L) {
-          n += pass_powers(pass_radix(L, NS)) * NS;
-          NS *= 8;
-     }
-     return n;
-}
 
 // A pass's twiddles W^jm, W^2jm, W^4jm of the butterflies a thread owns
 // (loaded ahead of the exchange that precedes the pass).
