@@ -353,7 +353,8 @@ def run_tdf(args, rank, world, local_rank):
                         "frac": round(achieved / peak, 4), "traffic": None,
                         "kernel": ("k_spinpass (demodulation + both FFT passes + F, one ordered launch)"
                                    if col_n and not ktimes.get("rowpass_launches")
-                                   else "k_colpass (demodulation + first FFT pass)"),
+                                   else "%s (demodulation + first FFT pass)"
+                                   % ("k_split_col" if args.form == "split" else "k_fp64_col")),
                         "peak_kind": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind,
                         "algorithmic_bytes_per_template": bt,
                         "kernel_ms": {k: round(v, 3) for k, v in ktimes.items() if k.endswith("_ms")},
