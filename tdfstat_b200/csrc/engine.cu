@@ -2240,6 +2240,10 @@ int tdf_search_segments_device(tdf_engine *e, int32_t nseg, const int32_t *slots
                const uint64_t f[] = {(uint64_t)B.slot, (uint64_t)B.nb, (uint64_t)B.nt, (uint64_t)B.sky_off,
                                      (uint64_t)B.tp_off};
                key = fnv1a(key, f, sizeof(f));
+               // the sky stage takes the segment's oms by value: an upload may
+               // have brought another
+               const double oms = e->sdv[B.slot].seg.oms;
+               key = fnv1a(key, &oms, sizeof(oms));
           }
           const uintptr_t cfg[] = {(uintptr_t)e->Tc, (uintptr_t)e->Gt, (uintptr_t)e->nlanes, (uintptr_t)e->sparse_now,
                                    (uintptr_t)e->plan_sky.p, (uintptr_t)e->plan_tp.p, (uintptr_t)e->plan_pts.p,

@@ -87,3 +87,31 @@ def test_segment_slot_upload_replaces_data(three_jobs):
     eng.upload_segment(s1, jobs[2].segment())
     assert eng.search_segments_device([s1], [len(pm)], pm, mm, nn) == want
     eng.close()
+
+
+def test_replayed_call_follows_an_upload_with_another_band(three_jobs):
+    """tdf_engine_upload_segment() and tdf_engine_upload() may bring a segment
+    of another reference frequency (oms = 2 pi fpo dt).  With the same points
+    the call keeps its shape, so a graph captured before the upload must not be
+    replayed with the old oms: every later call counts as a fresh engine does."""
+    from tdfstat_b200.engine import Engine
+    job = three_jobs["split"][0]
+    opts = job.search_opts()
+    opts.thr = 8.0   # a few hundred noise triggers, so that the counts tell the bands apart
+    pm, mm, nn = (np.asarray(v)[:1] for v in job.sky_points())
+    segs, want = [], []
+    for scale in (1.0, 1.25):   # 100 and 125 Hz: the point stays inside the sky
+        seg = job.segment()
+        seg.oms *= scale
+        e1 = Engine(seg, opts, form="split")
+        want.append(e1.search_device(pm, mm, nn))
+        e1.close()
+        segs.append(seg)
+    assert want[0][0] == want[1][0] > 0 and want[0][1] != want[1][1]
+    eng = Engine(segs[0], opts, form="split")
+    for upload in (lambda s: eng.upload_segment(0, s), eng.upload):
+        for k in (0, 1, 0):
+            upload(segs[k])
+            for rep in range(3):   # plain launches, capture, replay
+                assert eng.search_segments_device([0], [1], pm, mm, nn) == want[k], (k, rep)
+    eng.close()
