@@ -1729,7 +1729,13 @@ static int run_plan(tdf_engine *e, const std::vector<PlanBatch> &pb, uint64_t ke
           const int64_t l0 = e->launches;
           const int st = enqueue_plan(e, pb);
           cudaGraph_t graph = nullptr;
-          const cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
+          cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
+          // the capture left its record in the slots' events, and a wait
+          // outside of it (the next search's sky stage) is refused on such one
+          for (int s = 0; s < 2; s++) {
+               const cudaError_t re = cudaEventRecord(e->spin_done[s], e->stream);
+               if (ce == cudaSuccess) ce = re;
+          }
           if (st != TDF_OK || ce != cudaSuccess) {
                if (graph) cudaGraphDestroy(graph);
                e->launches = l0;

@@ -115,3 +115,26 @@ def test_replayed_call_follows_an_upload_with_another_band(three_jobs):
             for rep in range(3):   # plain launches, capture, replay
                 assert eng.search_segments_device([0], [1], pm, mm, nn) == want[k], (k, rep)
     eng.close()
+
+
+def test_other_calls_after_a_captured_one(three_jobs):
+    """A search and a spectrum right after the call was captured (its second
+    time) and replayed give what a fresh engine gives."""
+    from tdfstat_b200.engine import Engine
+    job = three_jobs["split"][0]
+    pm, mm, nn = job.sky_points()
+    ss = float(job.range.spndr[0])
+    e1 = Engine(job.segment(), job.search_opts(), form="split", max_sky_batch=1)
+    want = e1.search_device(pm, mm, nn)
+    F = e1.fstat(int(pm[0]), float(mm[0]), float(nn[0]), ss)
+    e1.close()
+    for times in (2, 3):
+        eng = Engine(job.segment(), job.search_opts(), form="split", max_sky_batch=1)
+        for _ in range(times):
+            assert eng.search_segments_device([0], [len(pm)], pm, mm, nn) == want
+        np.testing.assert_array_equal(eng.fstat(int(pm[0]), float(mm[0]), float(nn[0]), ss), F)
+        assert eng.search_device(pm, mm, nn) == want
+        for _ in range(times):
+            assert eng.search_segments_device([0], [len(pm)], pm, mm, nn) == want
+        assert eng.search_device(pm, mm, nn) == want
+        eng.close()
