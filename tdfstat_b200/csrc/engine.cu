@@ -37,6 +37,9 @@ static int set_error(int code, const char *fmt, ...) {
      vsnprintf(buf, sizeof(buf), fmt, ap);
      va_end(ap);
      g_last_error = buf;
+     // a CUDA error that is reported is done with: the runtime would hand it to
+     // the next launch check of this thread as well
+     if (code == TDF_ERR_CUDA || code == TDF_ERR_OUT_OF_MEMORY) cudaGetLastError();
      return code;
 }
 

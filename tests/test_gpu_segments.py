@@ -138,3 +138,23 @@ def test_other_calls_after_a_captured_one(three_jobs):
             assert eng.search_segments_device([0], [len(pm)], pm, mm, nn) == want
         assert eng.search_device(pm, mm, nn) == want
         eng.close()
+
+
+def test_engine_after_a_failed_one(three_jobs):
+    """An engine whose buffers do not fit the device is refused with
+    TDF_ERR_OUT_OF_MEMORY, and the next one is not touched by that error."""
+    from tdfstat_b200 import _abi
+    from tdfstat_b200.engine import Engine, TdfError
+    job = three_jobs["split"][0]
+    pm, mm, nn = job.sky_points()
+    want = None
+    for _ in range(2):
+        eng = Engine(job.segment(), job.search_opts(), form="split")
+        got = eng.search_device(pm, mm, nn)
+        eng.close()
+        assert want is None or got == want
+        want = got
+        with pytest.raises(TdfError) as ei:   # petabytes: the first allocation is refused
+            Engine(job.segment(), job.search_opts(), form="split", max_sky_batch=10 ** 6)
+        assert ei.value.status == _abi.TDF_ERR_OUT_OF_MEMORY
+    assert want[0] > 0
