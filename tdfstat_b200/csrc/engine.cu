@@ -545,6 +545,10 @@ struct tdf_engine {
      // against 2.37 for the two launches.
      bool fused = false;
      int fuse_lag = 3;
+     // probes after which a row pass gives up waiting for a block's copy, in
+     // the sky and in the spindown stage (TDF_SKY_WAIT_PROBES=n,
+     // TDF_ROW_WAIT_PROBES=n; 0 gives up at once, to test what follows)
+     int sky_probes = 1 << 20, row_probes = 1 << 20;
      // split form: the row pass keeps F on the chip and hands over only the
      // candidates and the edge bins of its runs (TDF_FULL_F=1: full F ring);
      // blocks_avg, and a batch that needs more of the spectrum, use the full
@@ -961,7 +965,7 @@ static int run_sky_stage(tdf_engine *e, int npts, const SkyParam *dsky = nullptr
                            ti.base.as<double2>(), ti.step.as<double2>(), e->fac.as<double>(), t.N1};
           TRY(launch_sky_mid(t.N2, Q, mid, st));
           const CoefRow row{e->B1.as<double2>(), ti.ltw2.as<double2>(), e->B0.as<D2>(), ws, e->n2N + 2, e->Ninterp - 1, Q,
-                            reinterpret_cast<unsigned *>(e->counters(sl) + 1)};
+                            reinterpret_cast<unsigned *>(e->counters(sl) + 1), e->sky_probes};
           TRY(launch_rows(ti.N1, ti.N2, e->sms, row, st));
           coef = &e->B0;
           e->launches += 3;
@@ -1146,7 +1150,7 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt,
                              e->N, e->CL, (e->N + t.N2 - 1) / t.N2, e->nifo, nt};
           SplitRow row{Ln.Ybuf.as<float2>(), t.ltw2.template as<float2>(), Ln.Fbuf.as<float>() + (size_t)boff * e->nF,
                        ctp, e->aabb[e->cur].as<AaBb>(), e->nF, e->opts.fr[0], e->opts.fr[1], e->opts.thr,
-                       blocks || !select ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff, nullptr, nullptr, nt, errw};
+                       blocks || !select ? nullptr : Ln.cand.as<uint2>(), tcnt + G, e->cand_cap, boff, nullptr, nullptr, nt, errw, e->row_probes};
           if (e->sparse_now) {
                row.cand = nullptr;
                row.E = Ln.Ebuf.as<float>();
@@ -1181,7 +1185,7 @@ static int run_chunk(tdf_engine *e, int l, const TmplParam *dtp, int ci, int nt,
           const Fp64Row row{Ln.Ybuf.as<double2>(), t.ltw2.template as<double2>(),
                             Ln.Fbuf.as<double>() + (size_t)boff * e->nF, ctp, e->aabb[e->cur].as<AaBb>(), e->nF,
                             e->opts.fr[0], e->opts.fr[1], e->opts.thr, blocks || !select ? nullptr : Ln.cand.as<uint2>(), tcnt + G,
-                            e->cand_cap, boff, nullptr, nullptr, nt, errw};
+                            e->cand_cap, boff, nullptr, nullptr, nt, errw, e->row_probes};
           TRY(launch_rows(t.N1, t.N2, e->sms, row, st));
      }
      if (e->timing) timing_end(e, tev, KT_ROW, nt, st);
@@ -1380,7 +1384,7 @@ static int run_templates_batch(tdf_engine *e, int nt) {
 // the error of a kernel error word whose bounded waits gave up, else TDF_OK
 static int wait_error(unsigned errf) {
      if (errf & ERR_STAGE_TIMEOUT)
-          return set_error(TDF_ERR_CUDA, "spindown stage: an asynchronous copy did not complete within its wait limit");
+          return set_error(TDF_ERR_CUDA, "row pass: an asynchronous copy did not complete within its wait limit");
      if (errf & ERR_ORDER_TIMEOUT)
           return set_error(TDF_ERR_CUDA, "spindown stage: a row block's wait for its column blocks gave up");
      return TDF_OK;
@@ -1393,9 +1397,9 @@ static int finish_slot(tdf_engine *e, int slot, bool collect, int64_t *ntrig_tot
      if (e->timing) timing_collect(e);
      const unsigned long long nfound = e->h_cnt[2 * slot];
      const unsigned errf = (unsigned)(e->h_cnt[2 * slot + 1] & 0xffffffffu);
+     TRY(wait_error(errf));   // before what wrong values may have led to
      if (errf & ERR_OVERFLOW)
           return set_error(TDF_ERR_TRIGGER_OVERFLOW, "Too many triggers! buffer_size=%d [triggers]", e->opts.bufsize / 2);
-     TRY(wait_error(errf));
      if (errf & ERR_NEED_FULL_F) {
           *need_full = true;
           return TDF_OK;
@@ -1926,6 +1930,11 @@ int tdf_engine_create(const tdf_segment *seg, const tdf_search_opts *opts, int f
      if (fp && fp[0] == '1') e->fused = true;
      const char *fl = getenv("TDF_FUSE_LAG");
      if (fl && atoi(fl) > 0) e->fuse_lag = atoi(fl);
+     for (auto &w : {std::make_pair("TDF_SKY_WAIT_PROBES", &e->sky_probes),
+                     std::make_pair("TDF_ROW_WAIT_PROBES", &e->row_probes)}) {
+          const char *v = getenv(w.first);
+          if (v && v[0] >= '0' && v[0] <= '9') *w.second = std::min(atoi(v), 1 << 20);
+     }
      const char *gt = getenv("TDF_GROUP_TEMPLATES");
      if (gt && atoi(gt) > 0) e->Gt = std::min(atoi(gt), (int)tdf_engine::kGtMax);
      autotune_cache_lookup(e);
@@ -2263,9 +2272,9 @@ int tdf_search_segments_device(tdf_engine *e, int32_t nseg, const int32_t *slots
           CUCHK(cudaStreamSynchronize(e->stream));
           if (check_plan) TRY(plan_check(e, hp, hp_seg, ntm));
           const unsigned errf = (unsigned)((e->h_cnt[1] | e->h_cnt[3]) & 0xffffffffu);
+          TRY(wait_error(errf));
           if (errf & ERR_OVERFLOW)
                return set_error(TDF_ERR_TRIGGER_OVERFLOW, "Too many triggers! buffer_size=%d [triggers]", e->opts.bufsize / 2);
-          TRY(wait_error(errf));
           if ((errf & ERR_NEED_FULL_F) && e->sparse_now) {
                e->sparse_now = false;   // once more with the full F store
                continue;

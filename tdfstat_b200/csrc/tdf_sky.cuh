@@ -220,6 +220,7 @@ struct CoefRow {
      int nkeep, klast;
      int nt;          // pairs
      unsigned *err;
+     int probes;      // limit of the waits for a row block
 };
 
 template <int L, int N1, bool HALF, class F>

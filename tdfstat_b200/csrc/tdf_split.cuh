@@ -826,6 +826,7 @@ template <class W> struct RowArgs {
      uint4 *scand;    // sparse form: candidate records
      int nt;          // templates of the launch
      unsigned *err;
+     int probes;      // limit of the waits for a row block
 };
 using SplitRow = RowArgs<float2>;
 using Fp64Row = RowArgs<double2>;
@@ -989,8 +990,11 @@ __device__ __forceinline__ void split_row_block(const Fp64Row &a, int b, int blk
 // starts the copy of block j + NB into that buffer and notes it in issued[]
 // (a group that got ahead of the buffer's previous user must not take that
 // user's barrier phase for its own).  A block's copy depends on the block NB
-// before it only, so every wait ends; all are bounded (ERR_STAGE_TIMEOUT in
-// *err), and every copy started is waited for.
+// before it only, so every wait ends; all are bounded.  A thread whose wait
+// gave up reports ERR_STAGE_TIMEOUT in *err and neither waits nor starts a copy
+// again: it only keeps its group's barriers, and the groups whose blocks are
+// then never copied give up in turn.  Before the CTA leaves, every copy that was
+// started is waited for.
 // (FP64: the same block and buffer bytes, four rows, one line per thread.)
 template <int L> __host__ __device__ constexpr int split_row_threads() { return L / 2; }   // of a group
 // Half as many buffers again as 512 threads' groups fit the shared memory; with
@@ -1040,21 +1044,26 @@ __global__ void __launch_bounds__(split_row_cta<typename A::V, L>(), 1) k_row(co
      bool ok = true;
      for (int j = g; j < n; j += G) {
           unsigned char *buf = smem_raw + (j % NB) * BYTES;
-          int probes = 1 << 22;
-          while (issued[j % NB] != j && --probes > 0) {}
-          __threadfence_block();
-          ok &= probes > 0 && mbar_wait(&full[j % NB], (unsigned)(j / NB) & 1u);
+          if (ok) {
+               int probes = 4 * a.probes;
+               while (issued[j % NB] != j && --probes > 0) {}
+               __threadfence_block();
+               ok = probes > 0 && mbar_wait(&full[j % NB], (unsigned)(j / NB) & 1u, a.probes);
+          }
           const int item = (int)blockIdx.x + j * (int)gridDim.x;
           split_row_block<L, N1, HALF>(a, item / BPT, item % BPT, tid, g, reinterpret_cast<const V *>(buf), true, buf,
                                        [&] {
                                             group_sync<L / 2>(g);   // the group is done with the buffer
-                                            if (tid == 0 && j + NB < n) {
+                                            if (tid == 0 && ok && j + NB < n) {
                                                  fence_proxy_async();
                                                  copy(j + NB);
                                             }
                                        });
      }
      if (!ok) atomicOr(a.err, ERR_STAGE_TIMEOUT);
+     if (__syncthreads_or(!ok) && threadIdx.x == 0)
+          for (int i = 0; i < NB; i++)
+               if (issued[i] >= 0) mbar_wait(&full[i], (unsigned)(issued[i] / NB) & 1u);
 }
 
 // ------------------------------------------------------------------ fused pass order
