@@ -1419,7 +1419,9 @@ static int finish_slot(tdf_engine *e, int slot, bool collect, int64_t *ntrig_tot
                CUCHK(cudaMemcpy(e->h_trig.data() + o + ahead, e->trig[slot].as<Trig>() + ahead,
                                 (nfound - ahead) * sizeof(Trig), cudaMemcpyDeviceToHost));
      }
-     CUCHK(cudaMemsetAsync(e->counters(slot), 0, 2 * sizeof(unsigned long long), e->stream));
+     // on the sky stream: the slot's next sky stage, the first to write to them,
+     // comes after it
+     CUCHK(cudaMemsetAsync(e->counters(slot), 0, 2 * sizeof(unsigned long long), sky_stream_of(e)));
      return TDF_OK;
 }
 
@@ -1461,7 +1463,8 @@ static int search_core(tdf_engine *e, int npts, const int32_t *pm, const float *
           *ntrig_total = 0;
           CUCHK(cudaStreamSynchronize(e->sky_stream));
           CUCHK(cudaStreamSynchronize(e->stream));
-          CUCHK(cudaMemsetAsync(e->zeroed.p, 0, e->zeroed.bytes, e->stream));
+          // the sky stages report errors there too, and the engine stream follows them
+          CUCHK(cudaMemsetAsync(e->zeroed.p, 0, e->zeroed.bytes, sky_stream_of(e)));
           int pending[2] = {0, 0};
           bool over = false, need_full = false;
           size_t b = 0;
@@ -2398,9 +2401,9 @@ int tdf_fstat_spectrum(tdf_engine *e, int32_t pm, float mm, float nn, float ss, 
      q.sgnl0 = T.sgnl0;
      q.slot = 0;
      q.id = 0;
+     CUCHK(cudaMemsetAsync(e->zeroed.p, 0, e->zeroed.bytes, sky_stream_of(e)));   // see search_core()
      TRY(run_sky_stage(e, 1));
      CUCHK(cudaMemcpyAsync(e->tparam.p, e->h_tp[0], sizeof(TmplParam), cudaMemcpyHostToDevice, e->stream));
-     CUCHK(cudaMemsetAsync(e->zeroed.p, 0, e->zeroed.bytes, e->stream));
      CUCHK(cudaStreamWaitEvent(e->stream, e->sky_done[0], 0));
      e->sparse_now = false;   // the spectrum itself is the output: the full F store
      TRY(run_templates(e, e->tparam.as<TmplParam>(), 1, false));

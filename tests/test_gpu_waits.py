@@ -101,3 +101,12 @@ def test_row_pass_that_gives_up_stops_copying_and_reports(monkeypatch, form, nam
     The call reports it, the groups start no copy whose buffer is still being
     filled, and the copies in flight are waited for before the CTA leaves."""
     _gives_up(monkeypatch, name, form, kinds)
+
+
+@pytest.mark.parametrize("overlap", ["1", "0"])
+@pytest.mark.parametrize("form", ["split", "fp64"])
+def test_sky_stage_that_gives_up_is_reported(monkeypatch, form, overlap):
+    """The sky stage reports from its own stream into a word that each batch
+    starts at zero: the clearing comes before the stage, for a spectrum, a
+    call's first batches and the batches that follow in the same slot."""
+    _gives_up(monkeypatch, "TDF_SKY_WAIT_PROBES", form, ("spectrum", "search"), (("TDF_SKY_OVERLAP", overlap),))
