@@ -1,0 +1,81 @@
+"""The scalar arithmetic of the spindown kernels (tdf_split.cuh), evaluated on
+the host: the functions are the kernels' own, compiled by nvcc for the host,
+and consist of IEEE operations that give the same bits there (no contraction).
+They are compared with the x87 extended precision of numpy.longdouble."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from tdfstat_b200 import build as B
+
+L = np.longdouble
+TWO_PI = L("6.283185307179586476925286766559005768")
+
+SOURCE = r"""
+#include <math.h>
+#include <string.h>
+#include "tdf_kernels.cuh"
+using namespace tdf;
+extern "C" void spin_phase(double het1, double spnd, int N, long n, const int *i, float *plain, float *big) {
+     SpinPhase p;
+     const bool past = p.init(het1, spnd, N);
+     for (long k = 0; k < n; k++) {
+          plain[k] = past ? NAN : p.at<false>((double)i[k]);
+          big[k] = p.at<true>((double)i[k]);
+     }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("spin_math")
+    src, out = os.path.join(d, "spin_math.cu"), os.path.join(d, "spin_math.so")
+    with open(src, "w") as f:
+        f.write(SOURCE)
+    r = subprocess.run([B.nvcc(), "-std=c++17", "-O2", *B.ARCH, "-Xcompiler", "-fPIC", "-shared",
+                        "-I" + os.path.join(B.REPO, "include"), "-I" + B.CSRC, "-o", out, src],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return C.CDLL(out)
+
+
+def _p(a, t):
+    return a.ctypes.data_as(C.POINTER(t))
+
+
+# N, spindown phase at the last sample in turns (2^18 turns: the limit of the plain branch)
+@pytest.mark.parametrize("N,turns", [(5385, 0.3), (86164, 900.0), (258492, -9000.0), (516985, 2.0 ** 18 * 0.99),
+                                     (258492, 2.0 ** 18 * 40)])
+def test_split_phase_is_rounded_to_fp32_once(lib, N, turns):
+    """The phase in radians is off by the FP32 rounding of a value up to pi
+    (half of 2^-22), by the fixed-point fraction (2^-33 turns), and by the FP64
+    roundings of h, w and q: 2.5 * 2^-53 of the turns."""
+    lib.spin_phase.argtypes = [C.c_double, C.c_double, C.c_int, C.c_long] + [C.c_void_p] * 3
+    rng = np.random.default_rng(N)
+    i = np.unique(np.concatenate([[0, 1, N - 1], rng.integers(0, N, 6000)])).astype(np.int32)
+    het1 = rng.uniform(0, 2 * np.pi / 2 ** 18)
+    spnd = turns * 2 * np.pi / float(N) ** 2
+    plain, big = np.zeros(len(i), np.float32), np.zeros(len(i), np.float32)
+    lib.spin_phase(het1, spnd, N, len(i), i.ctypes.data, plain.ctypes.data, big.ctypes.data)
+    t = (L(het1) * i + L(spnd) * i.astype(L) ** 2) / TWO_PI
+    f = t - np.rint(t)
+    for got in (plain, big):
+        if np.isnan(got).all():
+            assert abs(turns) > 2 ** 18
+            continue
+        d = (got.astype(L) / TWO_PI - f)
+        d -= np.rint(d)   # fractions near half a turn may carry either sign
+        d = np.abs(d * TWO_PI)
+        tol = 2.0 ** -23 + 2 * np.pi * (2.0 ** -33 + (abs(turns) + 1) * 2.5 * 2.0 ** -53)
+        assert np.max(d) <= tol, (float(np.max(d)), tol)
+        # a value rounded once, evenly spread over its interval: the rms error over
+        # [-pi, pi] is the root mean square of the half ulps over sqrt(3)
+        x = np.linspace(0.001, np.pi, 10000).astype(np.float32)
+        once = np.sqrt(np.mean((np.spacing(x) / 2) ** 2) / 3)
+        rest = 2 * np.pi * (2.0 ** -33 + (abs(turns) + 1) * 2.5 * 2.0 ** -53)
+        if abs(turns) > 100:
+            assert float(np.sqrt(np.mean(d * d))) <= 1.05 * once + rest
