@@ -982,18 +982,36 @@ __device__ __forceinline__ void split_row_block(const SplitRow &a, int b, int bl
      split_fstat<L, N1, HALF>(v, a, b, blk * RUN + 2 * c, t);
 }
 
+// F = A/aa + B/bb of the FP64 form (A = |Fa|^2, B = |Fb|^2) with 1/aa and 1/bb
+// in two doubles each, whose lower parts' terms are added first: two roundings
+// of F's size, where the two quotients and their sum make three.  Row pass at
+// 2^18 points 2.35 us per template, with divisions 2.51 (2.28 with single
+// reciprocals, which round once more than the divisions).
+struct FstatSums {
+     double aa, bb, ah, al, bh, bl;
+     __host__ __device__ __forceinline__ FstatSums(double a, double b) : aa(a), bb(b), ah(1. / a), bh(1. / b) {
+          al = fma(-ah, aa, 1.) * ah;
+          bl = fma(-bh, bb, 1.) * bh;
+     }
+     __host__ __device__ __forceinline__ double f(double A, double B) const {
+          const double v = fma(A, ah, fma(B, bh, fma(A, al, B * bl)));
+          // sums that are zero, values that are not finite
+          return fabs(v) <= DBL_MAX ? v : A / aa + B / bb;
+     }
+};
+
 // F of row k1 in the FP64 form, the full store (see RowArgs), HALF as above
 template <int L, int N1, bool HALF>
 __device__ __forceinline__ void fp64_fstat(const D2 (&v)[8], const Fp64Row &a, int b, int k1, int t) {
-     const AaBb sums = a.ab[a.tp[b].slot];
-     const double ia = 1. / sums.aa, ib = 1. / sums.bb;
+     const AaBb ab = a.ab[a.tp[b].slot];
+     const FstatSums sums(ab.aa, ab.bb);
      double *dst = a.F + (size_t)b * a.nF - a.fr0;
 #pragma unroll
      for (int m = 0; m < (HALF ? 4 : 8); m++) {
           const int k = k1 + N1 * (t + m * (L / 8));
-          const double2 q = pfma(v[m].re, v[m].re, pmul(v[m].im, v[m].im));
-          const double f = fma(q.x, ia, __dmul_rn(q.y, ib));
           if (k >= a.fr0 && k <= a.fr1) {
+               const double2 q = pfma(v[m].re, v[m].re, pmul(v[m].im, v[m].im));
+               const double f = sums.f(q.x, q.y);
                dst[k] = f;
                if (a.cand && !(f < a.thr) && k >= a.fr0 + 1 && k < a.fr1 - 1) {
                     const unsigned c = atomicAdd(a.cand_cnt, 1u);

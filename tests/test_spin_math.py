@@ -27,6 +27,9 @@ extern "C" void spin_phase(double het1, double spnd, int N, long n, const int *i
           big[k] = p.at<true>((double)i[k]);
      }
 }
+extern "C" void fp64_fstat(long n, const double *A, const double *B, const double *aa, const double *bb, double *F) {
+     for (long k = 0; k < n; k++) F[k] = FstatSums(aa[k], bb[k]).f(A[k], B[k]);
+}
 """
 
 
@@ -79,3 +82,26 @@ def test_split_phase_is_rounded_to_fp32_once(lib, N, turns):
         rest = 2 * np.pi * (2.0 ** -33 + (abs(turns) + 1) * 2.5 * 2.0 ** -53)
         if abs(turns) > 100:
             assert float(np.sqrt(np.mean(d * d))) <= 1.05 * once + rest
+
+
+def test_fp64_fstat_rounds_no_more_than_the_quotients(lib):
+    """A/aa + B/bb as the FP64 rows form it: two roundings, each of at most
+    half an ulp of F (the quotients and their sum make three); values that are
+    not finite as the quotients give them."""
+    lib.fp64_fstat.argtypes = [C.c_long] + [C.c_void_p] * 5
+    rng = np.random.default_rng(7)
+    n = 200000
+    A, B, aa, bb = (np.exp(rng.uniform(-20, 20, n)) for _ in range(4))
+    F = np.zeros(n)
+    lib.fp64_fstat(n, *(v.ctypes.data for v in (A, B, aa, bb, F)))
+    want = A.astype(L) / aa + B.astype(L) / bb
+    ulps = np.abs(F.astype(L) - want) / np.spacing(want.astype(np.float64))
+    # the lower parts' terms are 2^-53 of F and rounded to 2^-53 of that; extended precision has 2^-64
+    assert np.max(ulps) <= 1.0 + 2.0 ** -9, float(np.max(ulps))
+    odd = np.array([[0., 0., 0., 0.], [1., 1., 0., 2.], [np.inf, 1., 4., 3.], [1., np.inf, 3., 4.],
+                    [np.nan, 1., 3., 3.], [0., 0., 5., 7.], [1e308, 1e308, 1e-3, 1.], [1., 1., np.inf, 2.]])
+    A, B, aa, bb = (np.ascontiguousarray(odd[:, k]) for k in range(4))
+    F = np.zeros(len(odd))
+    lib.fp64_fstat(len(odd), *(v.ctypes.data for v in (A, B, aa, bb, F)))
+    with np.errstate(all="ignore"):
+        np.testing.assert_array_equal(F, A / aa + B / bb)
