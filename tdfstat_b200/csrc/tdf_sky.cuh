@@ -432,14 +432,14 @@ __global__ void __launch_bounds__(256) k_splint(const __grid_constant__ SplintIn
           if (i < I.N) {
                // xDatm{a,b}[i] = splint(interpftpad*(i - (shft[i] - shft[0])))/sig2
                const double *e = I.detssb + (size_t)d * 3 * I.N;
-               const double sh = shft_at(I.sp[p], e + 3 * (size_t)i), is2 = 1. / I.dp[d].sig2;
+               const double sh = shft_at(I.sp[p], e + 3 * (size_t)i), sig2 = I.dp[d].sig2;
                const D2 y = splint_eval(I.C + (size_t)q * I.stride, I.n, I.np,
                                         I.interpftpad * (i - __dsub_rn(sh, shft_at(I.sp[p], e))));
                X v;
-               v.x = y.re.x * is2;
-               v.y = y.re.y * is2;
-               v.z = y.im.x * is2;
-               v.w = y.im.y * is2;
+               v.x = y.re.x / sig2;
+               v.y = y.re.y / sig2;
+               v.z = y.im.x / sig2;
+               v.w = y.im.y / sig2;
                xs[c][r] = v;
                const double di = (double)i, h = __dmul_rn((double)(2 * i), sh);
                ss[c][r] = SPLIT ? (S)(float)h : (S)__dadd_rn(__dmul_rn(di, di), h);
