@@ -27,6 +27,9 @@ extern "C" void spin_phase(double het1, double spnd, int N, long n, const int *i
           big[k] = p.at<true>((double)i[k]);
      }
 }
+extern "C" void spin_sincos(long n, const double *x, double *s, double *c) {
+     for (long k = 0; k < n; k++) sincos_spin(x[k], s[k], c[k]);
+}
 extern "C" void fp64_fstat(long n, const double *A, const double *B, const double *aa, const double *bb, double *F) {
      for (long k = 0; k < n; k++) F[k] = FstatSums(aa[k], bb[k]).f(A[k], B[k]);
 }
@@ -105,3 +108,26 @@ def test_fp64_fstat_rounds_no_more_than_the_quotients(lib):
     lib.fp64_fstat(len(odd), *(v.ctypes.data for v in (A, B, aa, bb, F)))
     with np.errstate(all="ignore"):
         np.testing.assert_array_equal(F, A / aa + B / bb)
+
+
+@pytest.mark.parametrize("phases", ["1", "100", "1e5", "1e9", "multiples 1e5", "multiples 1e9"])
+def test_fp64_sine_and_cosine(lib, phases):
+    """Absolute error of sincos_spin() up to 2^30 rad, near multiples of pi/2
+    as well: 2^-54 from each of the two reductions and the last multiply-add
+    (values below 1), 7e-17 at most from the series' roundings, together below
+    2^-52."""
+    lib.spin_sincos.argtypes = [C.c_long] + [C.c_void_p] * 3
+    rng = np.random.default_rng(11)
+    n = 200000
+    R = float(phases.split()[-1])
+    if phases.startswith("multiples"):
+        k = rng.integers(-int(R / 1.6), int(R / 1.6), n)
+        # an offset of up to 1e-3 of random size
+        x = (k * (TWO_PI / 4) + rng.choice([-1, 0, 1], n) * np.exp(rng.uniform(-40, -7, n))).astype(np.float64)
+    else:
+        x = rng.uniform(-R, R, n)
+    x = np.concatenate([x, [0.0, np.pi / 4, -np.pi / 4, np.pi / 2]])
+    s, c = np.zeros(len(x)), np.zeros(len(x))
+    lib.spin_sincos(len(x), x.ctypes.data, s.ctypes.data, c.ctypes.data)
+    for got, want in ((s, np.sin(x.astype(L))), (c, np.cos(x.astype(L)))):
+        assert np.max(np.abs(got.astype(L) - want)) <= 2.0 ** -52
