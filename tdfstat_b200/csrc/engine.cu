@@ -682,14 +682,31 @@ static int ensure_tparam(tdf_engine *e, size_t n) {
      if (n > e->h_tp_cap) {
           CUCHK(cudaStreamSynchronize(e->stream));
           size_t cap = std::max<size_t>(n, 4096);
+          e->h_tp_cap = 0;   // until all three buffers are there
           for (int s = 0; s < 2; s++) {
                if (e->h_tp[s]) cudaFreeHost(e->h_tp[s]);
                e->h_tp[s] = nullptr;
                CUCHK(cudaMallocHost((void **)&e->h_tp[s], cap * sizeof(TmplParam)));
           }
-          e->h_tp_cap = cap;
           TRY(e->tparam.alloc(cap * sizeof(TmplParam)));
+          e->h_tp_cap = cap;
      }
+     return TDF_OK;
+}
+
+// trigger buffers of cap records in place of those there are; without room for
+// both there are none (trig_cap = 0: the kernels then only count)
+static int alloc_triggers(tdf_engine *e, unsigned long long cap) {
+     e->trig_cap = 0;
+     for (DevBuf &b : e->trig) b.release();
+     for (DevBuf &b : e->trig) {
+          const int st = b.alloc(cap * sizeof(Trig));
+          if (st != TDF_OK) {
+               for (DevBuf &c : e->trig) c.release();
+               return st;
+          }
+     }
+     e->trig_cap = cap;
      return TDF_OK;
 }
 
@@ -756,9 +773,8 @@ static int engine_alloc(tdf_engine *e) {
      TRY(e->linesd.alloc(std::max<size_t>(1, e->lines.size()) * sizeof(double)));
      if (!e->lines.empty())
           CUCHK(cudaMemcpy(e->linesd.p, e->lines.data(), e->lines.size() * sizeof(double), cudaMemcpyHostToDevice));
-     e->trig_cap = 1ull << 21;
+     TRY(alloc_triggers(e, 1ull << 21));
      for (int s = 0; s < 2; s++) {
-          TRY(e->trig[s].alloc(e->trig_cap * sizeof(Trig)));
           CUCHK(cudaEventCreateWithFlags(&e->done[s], cudaEventDisableTiming));
      }
      {
@@ -1511,7 +1527,7 @@ static int search_core(tdf_engine *e, int npts, const int32_t *pm, const float *
                CUCHK(cudaEventRecord(e->spin_done[slot], e->stream));
                CUCHK(cudaMemcpyAsync(e->h_cnt + 2 * slot, e->counters(slot), 2 * sizeof(unsigned long long),
                                      cudaMemcpyDeviceToHost, e->stream));
-               if (collect)
+               if (collect && e->trig_cap >= tdf_engine::kTrigAhead)
                     CUCHK(cudaMemcpyAsync(e->h_trig0[slot], e->trig[slot].p, tdf_engine::kTrigAhead * sizeof(Trig),
                                           cudaMemcpyDeviceToHost, e->stream));
                CUCHK(cudaEventRecord(e->done[slot], e->stream));
@@ -1536,11 +1552,12 @@ static int search_core(tdf_engine *e, int npts, const int32_t *pm, const float *
           if (!over) break;
           if (++grown > 3) return set_error(TDF_ERR_CAPACITY, "trigger buffer could not be sized");
           // a batch found more triggers than the buffer holds: grow and rerun
-          unsigned long long need = std::max(e->h_cnt[0], e->h_cnt[2]);
-          e->trig_cap = std::max<unsigned long long>(need + (need >> 2), e->trig_cap * 2);
-          for (int s = 0; s < 2; s++) {
-               e->trig[s].release();
-               TRY(e->trig[s].alloc(e->trig_cap * sizeof(Trig)));
+          const unsigned long long need = std::max(e->h_cnt[0], e->h_cnt[2]), old = e->trig_cap;
+          const int st = alloc_triggers(e, std::max<unsigned long long>(need + (need >> 2), old * 2));
+          if (st != TDF_OK) {
+               const std::string why = g_last_error;
+               alloc_triggers(e, old);   // the engine stays usable
+               return set_error(st, "%s", why.c_str());
           }
      }
      return TDF_OK;
