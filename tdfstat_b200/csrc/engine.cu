@@ -822,6 +822,7 @@ static void engine_free(tdf_engine *e) {
           L.mubuf.release();
           L.cand.release();
           L.Ebuf.release();
+          L.ctl.release();
      }
      e->t_nfft.release();
      e->t_ninterp.release();

@@ -51,3 +51,26 @@ def test_trigger_buffers_that_cannot_grow():
     assert many[0] == 4 * 401 and many[1] > 2 ** 21
     assert eng.search_device(*(v[:1] for v in pts)) == few
     eng.close()
+
+
+def test_engines_give_back_their_memory():
+    """Creating, using and closing engines takes no device memory for good: a
+    buffer of the smallest kind (512 bytes) left behind per lane keeps about 20 KB
+    of the device's memory from being given back, 6 MB after 300 engines."""
+    import torch
+    job = _job(16.0, 1, 2880, 1.0, 14.5)
+    seg, opts = job.segment(), job.search_opts()
+    pm, mm, nn = job.sky_points()
+
+    def rounds(n):
+        for k in range(n):
+            eng = Engine(seg, opts, form=("split", "fp64")[k % 2], max_sky_batch=1)
+            if k % 100 < 2:
+                eng.search_device(pm, mm, nn)
+            eng.close()
+
+    torch.cuda.init()
+    rounds(8)
+    free = torch.cuda.mem_get_info()[0]
+    rounds(300)
+    assert torch.cuda.mem_get_info()[0] >= free
