@@ -298,8 +298,8 @@ struct DevBuf {
 template <typename T>
 struct FFTTables {
      int N = 0, N1 = 0, N2 = 0;
-     DevBuf line1, line2, hi, lo;
-     DevBuf base, step, ltw1, ltw2;   // spindown passes (build_split)
+     DevBuf line1, line2, hi, lo;     // general passes (build_general)
+     DevBuf base, step, ltw1, ltw2;   // spindown passes and interpolation by two (build_split)
      int build(int n) {
           N = n;
           int l = ilog2i(n);
@@ -307,12 +307,16 @@ struct FFTTables {
           N2 = n / N1;
           if (N1 < 64 || N2 < 64 || N1 > 1024 || N2 > 1024)
                return set_error(TDF_ERR_UNSUPPORTED, "FFT length %d outside 2^12..2^20", n);
+          return TDF_OK;
+     }
+     // tables of tdf_passes.cuh: the two lines' twiddles, the four-step ones in two factors
+     int build_general() {
           TRY(fill(line1, N1, N1));
           TRY(fill(line2, N2, N2));
-          int nhi = std::max(1, n / 1024);
+          int nhi = std::max(1, N / 1024);
           std::vector<cx<T>> h(nhi), o(1024);
-          for (int j = 0; j < nhi; j++) h[j] = tw((long)j * 1024, n);
-          for (int j = 0; j < 1024; j++) o[j] = tw(j, n);
+          for (int j = 0; j < nhi; j++) h[j] = tw((long)j * 1024, N);
+          for (int j = 0; j < 1024; j++) o[j] = tw(j, N);
           TRY(hi.alloc(nhi * sizeof(cx<T>)));
           TRY(lo.alloc(1024 * sizeof(cx<T>)));
           CUCHK(cudaMemcpy(hi.p, h.data(), nhi * sizeof(cx<T>), cudaMemcpyHostToDevice));
@@ -791,10 +795,7 @@ static int engine_alloc(tdf_engine *e) {
      TRY(ensure_tparam(e, 1));
      TRY(e->t_nfft.build(e->nfft));
      TRY(e->t_ninterp.build(e->Ninterp));
-     if (interp_fused(e)) {
-          TRY(e->t_nfft.build_split());
-          TRY(e->t_ninterp.build_split());
-     }
+     for (FFTTables<double> *t : {&e->t_nfft, &e->t_ninterp}) TRY(interp_fused(e) ? t->build_split() : t->build_general());
      return TDF_OK;
 }
 
