@@ -84,3 +84,27 @@ def test_fp64_form_refuses_transforms_above_2_18(jobs):
     with pytest.raises(TdfError) as ei:
         Engine.from_job(j64, form="fp64")
     assert ei.value.status == _abi.TDF_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("fftpad", [1, 2])
+def test_two_templates_per_thread_at_the_largest_sizes(jobs, fftpad):
+    """Five spindowns of 2^19 or 2^20 points fill the GPU with two templates
+    per thread (the last one alone); chunks of one template take one per
+    thread.  Records are equal bit for bit."""
+    j32, _ = jobs(fftpad)
+    opts = j32.search_opts()
+    opts.spndr[1] += 2.0
+    opts.thr = 9.0
+    pm, mm, nn = (v[:1] for v in j32.sky_points())
+    eng = Engine(j32.segment(), opts, form="split")
+    ref = None
+    for tc in (96, 5, 4, 1):
+        eng.templates_per_chunk = tc
+        r = eng.search(pm, mm, nn)
+        got = (r.hdr, r.lens, r.pairs_flat)
+        assert len(r) == 5 and r.ntrig > 100
+        if ref is None:
+            ref = got
+        for a, b in zip(got, ref):
+            np.testing.assert_array_equal(a, b)
+    eng.close()
