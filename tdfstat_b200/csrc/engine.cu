@@ -1985,6 +1985,9 @@ int tdf_engine_create(const tdf_segment *seg, const tdf_search_opts *opts, int f
      if (st == TDF_OK) st = upload_inputs(e, seg);
      if (st == TDF_OK) {
           ce = cudaStreamSynchronize(e->stream);
+          // tables and cleared buffers went through the default stream, which the
+          // engine's streams do not wait for
+          if (ce == cudaSuccess) ce = cudaStreamSynchronize(cudaStreamLegacy);
           if (ce != cudaSuccess) st = set_error(TDF_ERR_CUDA, "upload: %s", cudaGetErrorString(ce));
      }
      if (st != TDF_OK) {
