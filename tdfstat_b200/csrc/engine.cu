@@ -2274,6 +2274,7 @@ int tdf_search_segments_device(tdf_engine *e, int32_t nseg, const int32_t *slots
      *nrec = ntm;
      *ntrig = 0;
      if (pb.empty()) return TDF_OK;
+     e->signal_valid = false;   // a replayed call does not pass run_sky_stage()
      CUCHK(cudaStreamSynchronize(e->sky_stream));
      CUCHK(cudaStreamSynchronize(e->stream));
      TRY(e->plan_sky.alloc(std::max<size_t>(e->plan_sky.bytes, hs.size() * sizeof(SkyParam))));

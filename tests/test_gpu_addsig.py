@@ -129,3 +129,22 @@ def test_write_signal_matches_reference(tmp_path):
         with pytest.raises(TdfError):
             eng.signal(0, job.sett.N)
         eng.close()
+
+
+def test_no_signal_is_held_after_a_replayed_call(golden):
+    """The injected signal lies in the sky stage's work memory: a whole-call
+    over resident segments ends it like a search does, also when the call is
+    replayed as a graph."""
+    from tdfstat_b200.engine import TdfError
+    g = golden("g4_addsig")
+    job = g.job32
+    pm, mm, nn = job.sky_points()
+    eng = Engine.from_job(job, form="split")
+    for _ in range(4):   # plain launches, capture, replays
+        eng.add_signal(job.signal)
+        assert np.any(eng.signal(0, job.sett.N))
+        eng.search_segments_device([0], [len(pm)], pm, mm, nn)
+        with pytest.raises(TdfError) as ei:
+            eng.signal(0, job.sett.N)
+        assert ei.value.status == _abi.TDF_ERR_INVALID
+    eng.close()
