@@ -104,11 +104,11 @@ static int set_smem(K kern, size_t smem) {
      return TDF_OK;
 }
 
-// Kernels of the sky stage (the FP64 interpolation passes run with one
-// array, NA = 1; the spindown passes with two).  A captured graph holding
-// both gets the sky stage's kernel nodes at the low stream priority and the
-// others at the high one, as the two streams have them when launched
-// directly (set_graph_priorities).
+// Kernels of the sky stage (k_sky_col, k_sky_mid, k_row<CoefRow>, k_splint;
+// for other interpolation factors k_sky_prep and the general passes with one
+// array, NA = 1).  A captured graph that holds them and the spindown stage's
+// gets their nodes at the low stream priority and the others at the high one,
+// as the two streams have them when launched directly (set_graph_priorities).
 static std::mutex g_sky_mu;
 static std::vector<const void *> g_sky_kernels;
 
@@ -1567,11 +1567,12 @@ static int search_core(tdf_engine *e, int npts, const int32_t *pm, const float *
 
 // ------------------------------------------------------------------ autotuning
 //
-// The templates per chunk (Tc) set how many CTAs a column/row pass launches
-// (32*Tc and 64*Tc for nfftf = 2^17) against the SM count, and how much of
-// L2 the intermediate spectra take.  tdf_engine_autotune() times candidates
-// on the caller's points; with TDF_AUTOTUNE_CACHE=<file> the choice is kept
-// per (form, N, nfftf, nifo, SM count, sky batch) and reused by later
+// The templates per chunk (Tc) set how many CTAs a column pass launches (32
+// per template of 2^17 points, or of two templates that share a thread), how
+// many row blocks each of the row pass's persistent CTAs takes, and how much of
+// L2 the intermediate spectra take.  tdf_engine_autotune() times candidates on
+// the caller's points; with TDF_AUTOTUNE_CACHE=<file> the choice is kept per
+// (form, N, nfftf, nifo, SM count, sky batch, F store) and reused by later
 // engines.
 
 static int sm_count(int dev) {

@@ -8,8 +8,9 @@
 //   k_rowpass<T, L, SIGN, NA, Src, Epi>: CTA = LINES rows k1 of an
 //     N = N1*L transform, L threads; the first-pass inputs are loaded from
 //     the rows straight into registers, Epi::store consumes X[k1 + N1*k2].
-// They run the FP64 transforms (sky stage, FP64 form) and the allocation-free
-// FP32 entry point; the split form's spindown passes are in tdf_split.cuh.
+// They run the sky stage's transforms for interpolation factors other than two
+// and the allocation-free FP32 entry point; the spindown passes of both forms
+// are in tdf_split.cuh, the interpolation by two in tdf_sky.cuh.
 #pragma once
 
 #include <type_traits>

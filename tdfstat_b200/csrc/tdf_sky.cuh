@@ -14,9 +14,9 @@
 //
 // The two arrays (a, b) of a point and detector are transformed as one pair,
 // with the thread groups, exchanges and block layouts of the FP64 spindown
-// passes (tdf_split.cuh): per point of six days and two detectors in batches
-// of eight 86 us with separate arrays, CTA-wide barriers and the modulation in
-// a kernel of its own.
+// passes (tdf_split.cuh): 66 us per point of six days and two detectors in
+// batches of eight (86 with separate arrays, CTA-wide barriers and the
+// modulation in a kernel of its own).
 // The inverse transform runs as a forward one on values whose real and
 // imaginary parts are swapped.
 //
@@ -92,7 +92,7 @@ __device__ __forceinline__ void store_col64(D2 (&v)[8], double2 *y, const double
 // The lanes of a warp are four columns at eight rows: the samples come in
 // natural order, so a load touches eight rows' lines of 128 bytes.  With the 32
 // rows of one column per warp it touched 32 (L1 49% busy on them, the load
-// queue full): 75 -> 65 us per sky point of 2^18 samples for the whole stage,
+// queue full): 75 -> 66 us per sky point of 2^18 samples for the whole stage,
 // 31.2 -> 28.5 for 2^17, 15.0 -> 13.9 for 2^16 (two detectors, batches).
 // grid (N2 / fp64_col_lines<L>(), Q)
 template <int L>

@@ -18,14 +18,11 @@
 // but in half the issue slots, which the passes' loads, shared-memory
 // exchanges and address arithmetic share.
 //
-// Work per thread group.  Both passes run at 32 warps per SM and used to
-// alternate between all warps computing and all warps waiting (44-53% of
-// issue slots used, 3 of 16 cycles per instruction lost to eligible warps
-// that were not selected: the CTA-wide barriers keep its warps in phase).
-// A column is now transformed by L/8 threads of its own, with a barrier of
-// just those threads (none across a warp for L <= 256), so the columns of an
-// SM drift apart and one column's loads overlap another's butterflies.  That
-// needs a column's data to be contiguous:
+// Work per thread group.  A column is transformed by L/8 threads of its own,
+// with a barrier of just those threads (none across a warp for L <= 256):
+// CTA-wide barriers keep all warps in phase, computing together and waiting
+// together, while columns of their own drift apart and one column's loads
+// overlap another's butterflies.  That needs a column's data to be contiguous:
 //   operands  xab[(slot*nifo + d)*N2 + n2][n1] float4 (a.re, b.re, a.im, b.im)
 //             s2[slot*N2 + n2][n1][d]           (rows of CL >= N/N2 entries)
 //   Y         [template][k1/RUN][n2][k1%RUN]  float4, likewise (re, im)
@@ -1041,10 +1038,10 @@ __device__ __forceinline__ void split_row_block(const Fp64Row &a, int b, int blk
 }
 
 // The row pass: one persistent CTA per SM.  A row block (RUN rows, one
-// contiguous 128 L bytes of Y) took as long to load as to transform, and CTAs
-// that start together load together and compute together: 2^18 points ran at
-// 1.35-1.47 us per template where loading alone took 0.68 (DRAM rate) and
-// transforming alone 0.78.  Here the blocks come in by bulk copies into
+// contiguous 128 L bytes of Y) takes about as long to load as to transform
+// (2^18 points: 0.68 and 0.78 us per template alone), and CTAs that start
+// together do the one and then the other (1.35-1.47 us against 1.05 as
+// follows).  The blocks come in by bulk copies into
 // split_row_bufs() buffers while the split_row_groups() thread groups of the
 // CTA transform earlier ones in place, 16 warps of up to 128 registers (two
 // lines per thread share the pass twiddles).
